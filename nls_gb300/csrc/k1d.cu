@@ -1,12 +1,11 @@
 // k1d.cu -- 1-D (axially symmetric, radial) RK4 kernels for sm_103a.
 //
-// rk4_1d_resident: the whole grid of one solve lives in shared memory of one CTA or of a thread
-// block cluster (distributed shared memory) for every step of the launch.  Each RK4 stage
+// rk4_1d_resident (complex128, one CTA) and rk4_1d_cluster_tb (a thread-block cluster): the whole
+// grid of one solve lives in shared memory for every step of the launch.  Each RK4 stage
 // (nls/nls.f90:726-729) reads the previous stage's values from shared memory, evaluates the
 // radial Laplacian (make_laplacian, nls/nls.f90:132-295) and the pointwise terms of
-// `hamiltonian` (nls/nls.f90:621-650), and writes the next stage input; CTAs of a cluster push
-// their K edge values into their neighbours' halo slots and meet at one cluster barrier per
-// stage.  HBM is touched once per launch (load and store of the state).
+// `hamiltonian` (nls/nls.f90:621-650), and writes the next stage input.  HBM is touched once per
+// launch (load and store of the state).
 //
 // rk4_1d_stage: one RK4 stage over an arbitrary-size grid from global memory, the general path
 // for grids too large to stay resident.
@@ -73,194 +72,91 @@ __device__ __forceinline__ typename C2<T>::type lap1d(const typename C2<T>::type
   return lu;
 }
 
-template <typename T, int K, int NPT>
-__global__ void __launch_bounds__(512) rk4_1d_resident(const Inst1D* __restrict__ insts, int cl,
-                                                       int seg_cap) {
-  typedef typename C2<T>::type C;
+// What a complex128 node needs for every stage of a launch: its operator row (w2 + w1 / (p h) as in
+// the band matrix, or the near-axis row), and its pump also as a float pair.  FP64
+// instructions bound these kernels (f64_node.cuh).
+template <int K>
+struct Node64 {
+  double row[2 * K + 1];
+  double P;
+  F2 p;
+  bool p_ok;
+};
+template <int K>
+__device__ __forceinline__ Node64<K> node64(const Stencil1D& op, int p, const double* P, bool in) {
+  Node64<K> d;
+  d.P = in ? P[p] : 0.0;
+  d.p = f2_split(d.P);
+  d.p_ok = f64_in_range(d.P);
+#pragma unroll
+  for (int i = 0; i < 2 * K + 1; ++i)
+    d.row[i] = !in ? 0.0 : (p >= K ? dadd(op.w1[i] / ((double)p * op.h), op.w2[i]) : op.near[p][i]);
+  return d;
+}
+// Slope at the node whose value is in[li] (neighbours in[li - K] .. in[li + K]).
+template <int K>
+__device__ __forceinline__ double2 slope64(const double2* in, int li, const Node64<K>& d, const F64Consts& c) {
+  double vx[2 * K + 1], vy[2 * K + 1];
+#pragma unroll
+  for (int i = 0; i < 2 * K + 1; ++i) {
+    const double2 v = in[li + i - K];
+    vx[i] = v.x;
+    vy[i] = v.y;
+  }
+  double2 q;
+  f64_slope_1d<K>(vx, vy, d.row, d.p, d.P, d.p_ok, c, q.x, q.y);
+  return q;
+}
+
+template <int K, int NPT>
+__global__ void __launch_bounds__(512) rk4_1d_resident(const Inst1D* __restrict__ insts, int seg_cap) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  const int inst = blockIdx.x / cl;
-  const int rank = blockIdx.x % cl;
-  const Inst1D& I = insts[inst];
+  const Inst1D& I = insts[blockIdx.x];
   const int n = I.n;
-  const int seg = (n + cl - 1) / cl;
-  const int p0 = rank * seg;
-  const int len = max(0, min(seg, n - p0));
   const int NT = blockDim.x;
   const int tid = threadIdx.x;
   const int L = seg_cap + 2 * K;
-  C* buf[2] = {reinterpret_cast<C*>(smem_raw), reinterpret_cast<C*>(smem_raw) + L};
-
-  cg::cluster_group cluster = cg::this_cluster();
-  C* left_buf[2] = {nullptr, nullptr};
-  C* right_buf[2] = {nullptr, nullptr};
-  if (cl > 1) {
-    if (rank > 0) {
-      left_buf[0] = cluster.map_shared_rank(buf[0], rank - 1);
-      left_buf[1] = cluster.map_shared_rank(buf[1], rank - 1);
-    }
-    if (rank < cl - 1) {
-      right_buf[0] = cluster.map_shared_rank(buf[0], rank + 1);
-      right_buf[1] = cluster.map_shared_rank(buf[1], rank + 1);
-    }
-  }
-
-  for (int i = tid; i < 2 * L; i += NT) buf[0][i] = mk<T>(0, 0);
-  if (cl > 1) cluster.sync(); else __syncthreads();
-
-  const Params<T>& prm = ParamsOf<T>::get(I);
-  const Phys<T> ph = phys_of<T>(prm);
-  const RK<T> rk = rk_of<T>(prm);
-  const Weights1D<T, K> w = load_w<T, K>(I.op);
-  const T h = (T)I.op.h;
-  const C* __restrict__ Ug = reinterpret_cast<const C*>(I.u);
-  const T* __restrict__ Pg = reinterpret_cast<const T*>(I.P);
-
-  C u[NPT], acc[NPT];
-  T P[NPT], ir[NPT];
-  // Double precision: each node's full operator row (w2 + w1 / (p h), as in the band matrix, or
-  // the near-axis row), built once per launch, so a stage evaluates one (2K+1)-term dot product
-  // per node instead of separate D2 and D1 sums (FP64 runs at a small fraction of FP32 on GB300).
-  constexpr bool ROWS = sizeof(T) == 8;
-  T wrow[ROWS ? NPT : 1][2 * K + 1];
+  double2* const buf0 = reinterpret_cast<double2*>(smem_raw);
+  double2* const buf1 = buf0 + L;
+  for (int i = tid; i < 2 * L; i += NT) buf0[i] = make_double2(0.0, 0.0);
+  __syncthreads();
+  const F64Consts c = I.f64;
+  double2* __restrict__ Ug = reinterpret_cast<double2*>(I.u);
+  double2 u[NPT], acc[NPT];
+  Node64<K> nd[NPT];
 #pragma unroll
   for (int j = 0; j < NPT; ++j) {
-    const int li = tid + j * NT;
-    u[j] = mk<T>(0, 0);
-    acc[j] = mk<T>(0, 0);
-    P[j] = 0;
-    ir[j] = 0;
-    if (ROWS) {
-#pragma unroll
-      for (int i = 0; i < 2 * K + 1; ++i) wrow[ROWS ? j : 0][i] = 0;
-    }
-    if (li < len) {
-      const int p = p0 + li;
-      u[j] = Ug[p];
-      P[j] = Pg[p];
-      ir[j] = p >= K ? (T)1 / ((T)p * h) : (T)0;
-      if (ROWS) {
-#pragma unroll
-        for (int i = 0; i < 2 * K + 1; ++i)
-          wrow[ROWS ? j : 0][i] = p >= K ? w.w1[i] / ((T)p * h) + w.w2[i] : ParamsOf<T>::near(I.op, p, i);
-      }
-      buf[0][K + li] = u[j];
-      if (left_buf[0] && li < K) left_buf[0][seg + K + li] = u[j];
-      if (right_buf[0] && li >= seg - K) right_buf[0][li - (seg - K)] = u[j];
-    }
+    const int p = tid + j * NT;
+    const bool in = p < n;
+    u[j] = in ? Ug[p] : make_double2(0.0, 0.0);
+    acc[j] = make_double2(0.0, 0.0);
+    nd[j] = node64<K>(I.op, p, reinterpret_cast<const double*>(I.P), in);
+    if (in) buf0[K + p] = u[j];
   }
-  if (cl > 1) cluster.sync(); else __syncthreads();
-
-  // the pump enters as c12 * P (the reference evaluates coeffs(12) * pumping first)
-#pragma unroll
-  for (int j = 0; j < NPT; ++j) P[j] = ph.c12 * P[j];
-  // Nodes are processed in batches of CB: a batch's shared-memory loads are all issued before any
-  // of its stores and its arithmetic is written phase by phase across the batch, so the nodes'
-  // independent dependency chains overlap.
-  constexpr int CB0 = (sizeof(T) == 8 || K == 3) ? 2 : 4;
-  constexpr int CB = NPT < CB0 ? NPT : CB0;
+  __syncthreads();
   const int64_t steps = I.steps;
   for (int64_t step = 0; step < steps; ++step) {
 #pragma unroll 1
     for (int s = 1; s <= 4; ++s) {
-      const C* in = buf[(s & 1) ? 0 : 1];
-      const int ob = (s & 1) ? 1 : 0;
-      C* out = buf[ob];
-      const T coef = s == 3 ? rk.dt : rk.half_dt;
-      const T wk = (s == 2 || s == 3) ? (T)2 : (T)1;
+      const double2* in = (s & 1) ? buf0 : buf1;
+      double2* out = (s & 1) ? buf1 : buf0;
 #pragma unroll
-      for (int j0 = 0; j0 < NPT; j0 += CB) {
-        C v[CB][2 * K + 1];
-#pragma unroll
-        for (int i = 0; i < CB; ++i) {
-          const int li = tid + (j0 + i) * NT;
-          const int c = K + (li < len ? li : 0);
-#pragma unroll
-          for (int d = -K; d <= K; ++d) v[i][d + K] = in[c + d];
-        }
-        C lu[CB];
-#pragma unroll
-        for (int i = 0; i < CB; ++i) {
-          const int p = p0 + tid + (j0 + i) * NT;
-          if (ROWS) {
-            T lx = 0, ly = 0;
-#pragma unroll
-            for (int d = 0; d < 2 * K + 1; ++d) {
-              lx += wrow[ROWS ? j0 + i : 0][d] * v[i][d].x;
-              ly += wrow[ROWS ? j0 + i : 0][d] * v[i][d].y;
-            }
-            lu[i].x = lx;
-            lu[i].y = ly;
-          } else if (p >= K) {
-            T d2x = 0, d2y = 0, d1x = 0, d1y = 0;
-#pragma unroll
-            for (int d = -K; d <= K; ++d) {
-              d2x += w.w2[d + K] * v[i][d + K].x;
-              d2y += w.w2[d + K] * v[i][d + K].y;
-              if (d != 0) {
-                d1x += w.w1[d + K] * v[i][d + K].x;
-                d1y += w.w1[d + K] * v[i][d + K].y;
-              }
-            }
-            lu[i].x = d2x + ir[j0 + i] * d1x;
-            lu[i].y = d2y + ir[j0 + i] * d1y;
-          } else {
-            T lx = 0, ly = 0;
-#pragma unroll
-            for (int d = -K; d <= K; ++d) {
-              const T a = ParamsOf<T>::near(I.op, p, d + K);
-              lx += a * v[i][d + K].x;
-              ly += a * v[i][d + K].y;
-            }
-            lu[i].x = lx;
-            lu[i].y = ly;
-          }
-        }
-        T sq[CB], r[CB];
-#pragma unroll
-        for (int i = 0; i < CB; ++i) sq[i] = v[i][K].x * v[i][K].x + v[i][K].y * v[i][K].y;
-#pragma unroll
-        for (int i = 0; i < CB; ++i) r[i] = rdiv(P[j0 + i], ph.c13 + ph.c14 * sq[i]);
-#pragma unroll
-        for (int i = 0; i < CB; ++i) {
-          const int j = j0 + i;
-          const int li = tid + j * NT;
-          const T a = ph.c3 * r[i] - ph.c4;
-          const T b = ph.c5 * sq[i] + ph.c6 * r[i];
-          C k;
-          k.x = a * v[i][K].x + b * v[i][K].y - lu[i].y;
-          k.y = a * v[i][K].y - b * v[i][K].x + lu[i].x;
-          if (s == 1) acc[j] = k;
-          else {
-            acc[j].x += wk * k.x;
-            acc[j].y += wk * k.y;
-          }
-          C t;
-          if (s < 4) {
-            t.x = u[j].x + coef * k.x;
-            t.y = u[j].y + coef * k.y;
-          } else {
-            u[j].x = u[j].x + rk.dt6 * acc[j].x;
-            u[j].y = u[j].y + rk.dt6 * acc[j].y;
-            t = u[j];
-          }
-          if (li < len) {
-            out[K + li] = t;
-            if (left_buf[ob] && li < K) left_buf[ob][seg + K + li] = t;
-            if (right_buf[ob] && li >= seg - K) right_buf[ob][li - (seg - K)] = t;
-          }
+      for (int j = 0; j < NPT; ++j) {
+        const int p = tid + j * NT;
+        if (p < n) {
+          const double2 t = f64_stage(s, u[j], acc[j], slope64<K>(in, K + p, nd[j], c), c);
+          if (s == 4) u[j] = t;
+          out[K + p] = t;
         }
       }
-      if (cl > 1) cluster.sync(); else __syncthreads();
+      __syncthreads();
     }
   }
-
-  C* __restrict__ Uo = reinterpret_cast<C*>(I.u);
 #pragma unroll
   for (int j = 0; j < NPT; ++j) {
-    const int li = tid + j * NT;
-    if (li < len) Uo[p0 + li] = u[j];
+    const int p = tid + j * NT;
+    if (p < n) Ug[p] = u[j];
   }
-  if (cl > 1) cluster.sync();
 }
 
 // Cluster form with temporal blocking: each CTA also evaluates a halo of H = 4K nodes on both
@@ -303,20 +199,19 @@ __global__ void __launch_bounds__(512) rk4_1d_cluster_tb(const Inst1D* __restric
   for (int i = tid; i < 4 * W; i += NT) base[i] = mk<T>(0, 0);
   __syncthreads();
 
-  const Params<T>& prm = ParamsOf<T>::get(I);
-  const Phys<T> ph = phys_of<T>(prm);
-  const RK<T> rk = rk_of<T>(prm);
-  const Weights1D<T, K> w = load_w<T, K>(I.op);
+  constexpr bool F64 = sizeof(T) == 8;
+  const Phys<float> ph = phys_of<float>(I.pf);
+  const RK<float> rk = rk_of<float>(I.pf);
+  const Weights1D<float, K> w = load_w<float, K>(I.op);
+  const F64Consts c64 = I.f64;
   const T h = (T)I.op.h;
   const C* __restrict__ Ug = reinterpret_cast<const C*>(I.u);
   const T* __restrict__ Pg = reinterpret_cast<const T*>(I.P);
 
   // owned local indices li = tid + j*NT - H, j < NPT, covering [-H, seg + H)
   C u[NPT], acc[NPT];
-  T pc[NPT], ir[NPT];
-  // double precision: each node's full operator row, built once per launch (see rk4_1d_resident)
-  constexpr bool ROWS = sizeof(T) == 8;
-  T wrow[ROWS ? NPT : 1][2 * K + 1];
+  T pc[F64 ? 1 : NPT], ir[F64 ? 1 : NPT];
+  Node64<K> nd[F64 ? NPT : 1];
   unsigned indom = 0;
 #pragma unroll
   for (int j = 0; j < NPT; ++j) {
@@ -325,31 +220,21 @@ __global__ void __launch_bounds__(512) rk4_1d_cluster_tb(const Inst1D* __restric
     const bool in = li < seg + H && p >= 0 && p < n;
     indom |= (unsigned)in << j;
     u[j] = in ? Ug[p] : mk<T>(0, 0);
-    pc[j] = in ? ph.c12 * Pg[p] : (T)0;
-    ir[j] = (in && p >= K) ? (T)1 / ((T)p * h) : (T)0;
-    if (ROWS) {
-#pragma unroll
-      for (int i = 0; i < 2 * K + 1; ++i)
-        wrow[ROWS ? j : 0][i] = !in ? (T)0 : (p >= K ? w.w1[i] / ((T)p * h) + w.w2[i] : ParamsOf<T>::near(I.op, p, i));
+    if constexpr (F64) {
+      nd[j] = node64<K>(I.op, p, Pg, in);
+    } else {
+      pc[j] = in ? ph.c12 * Pg[p] : (T)0;
+      ir[j] = (in && p >= K) ? (T)1 / ((T)p * h) : (T)0;
     }
     acc[j] = mk<T>(0, 0);
     if (in) A[0][li] = u[j];
   }
   __syncthreads();
 
-  auto lap = [&](const C* in, int li, int p, T irv, int j) -> C {
+  // slope of the complex64 form
+  auto slope = [&](const C* in, int li, int p, T irv, T pcv) -> C {
     C lu;
-    if (ROWS) {
-      T lx = 0, ly = 0;
-#pragma unroll
-      for (int d = -K; d <= K; ++d) {
-        const C v = in[li + d];
-        lx += wrow[ROWS ? j : 0][d + K] * v.x;
-        ly += wrow[ROWS ? j : 0][d + K] * v.y;
-      }
-      lu.x = lx;
-      lu.y = ly;
-    } else if (p >= K) {
+    if (p >= K) {
       T d2x = 0, d2y = 0, d1x = 0, d1y = 0;
 #pragma unroll
       for (int d = -K; d <= K; ++d) {
@@ -374,13 +259,11 @@ __global__ void __launch_bounds__(512) rk4_1d_cluster_tb(const Inst1D* __restric
       lu.x = lx;
       lu.y = ly;
     }
-    return lu;
-  };
-  auto kval = [&](C v, T pcv, C lu) -> C {
+    const C v = in[li];
     const T sq = v.x * v.x + v.y * v.y;
-    const T r = rdiv(pcv, ph.c13 + ph.c14 * sq);
-    const T a = ph.c3 * r - ph.c4;
-    const T b = ph.c5 * sq + ph.c6 * r;
+    const T r = rdiv(pcv, (T)ph.c13 + (T)ph.c14 * sq);
+    const T a = (T)ph.c3 * r - (T)ph.c4;
+    const T b = (T)ph.c5 * sq + (T)ph.c6 * r;
     C k;
     k.x = a * v.x + b * v.y - lu.y;
     k.y = a * v.y - b * v.x + lu.x;
@@ -410,17 +293,22 @@ __global__ void __launch_bounds__(512) rk4_1d_cluster_tb(const Inst1D* __restric
       for (int j = 0; j < NPT; ++j) {
         const int li = tid + j * NT - H;
         if (((indom >> j) & 1u) && li >= lo && li < hi) {
-          const int p = p0 + li;
-          const C k = kval(in[li], pc[j], lap(in, li, p, ir[j], j));
-          if (s == 1) acc[j] = k;
-          else {
-            acc[j].x += wk * k.x;
-            acc[j].y += wk * k.y;
+          C un;
+          if constexpr (F64) {
+            un = f64_stage(s, u[j], acc[j], slope64<K>(in, li, nd[j], c64), c64);
+          } else {
+            const C k = slope(in, li, p0 + li, ir[j], pc[j]);
+            if (s == 1) acc[j] = k;
+            else {
+              acc[j].x += wk * k.x;
+              acc[j].y += wk * k.y;
+            }
+            un = s < 4 ? mk<T>(u[j].x + coef * k.x, u[j].y + coef * k.y)
+                       : mk<T>(u[j].x + rk.dt6 * acc[j].x, u[j].y + rk.dt6 * acc[j].y);
           }
           if (s < 4) {
-            out[li] = mk<T>(u[j].x + coef * k.x, u[j].y + coef * k.y);
+            out[li] = un;
           } else {
-            const C un = mk<T>(u[j].x + rk.dt6 * acc[j].x, u[j].y + rk.dt6 * acc[j].y);
             u[j] = un;
             Anext[li] = un;
             if (leftA[0] && li < H) leftA[par ^ 1][seg + li] = un;
@@ -488,6 +376,32 @@ __global__ void __launch_bounds__(256) rk4_1d_stage(int n, int s, const void* __
   }
 }
 
+// The same in double precision (f64_node.cuh; acc holds the slopes' sum).
+template <int K>
+__global__ void __launch_bounds__(256) rk4_1d_stage_f64(int n, int s, const double2* __restrict__ src,
+                                                        double2* __restrict__ U, const double* __restrict__ P,
+                                                        double2* __restrict__ acc, double2* __restrict__ dst,
+                                                        F64Consts c, Stencil1D op) {
+  const int p = blockIdx.x * blockDim.x + threadIdx.x;
+  if (p >= n) return;
+  double2 v[2 * K + 1];
+#pragma unroll
+  for (int d = -K; d <= K; ++d) {
+    const int q = p + d;
+    v[d + K] = (q >= 0 && q < n) ? src[q] : make_double2(0.0, 0.0);
+  }
+  const Node64<K> nd = node64<K>(op, p, P, true);
+  const double2 u = U[p];
+  double2 a = s == 1 ? make_double2(0.0, 0.0) : acc[p];
+  const double2 t = f64_stage(s, u, a, slope64<K>(v, K, nd, c), c);
+  if (s < 4) {
+    acc[p] = a;
+    dst[p] = t;
+  } else {
+    U[p] = t;
+  }
+}
+
 // v = H(u) for the diagnostics (chemical potential).
 template <typename T, int K>
 __global__ void __launch_bounds__(256) rhs_1d(int n, const void* __restrict__ u_, const void* __restrict__ P_,
@@ -514,20 +428,34 @@ __global__ void __launch_bounds__(256) rhs_1d(int n, const void* __restrict__ u_
 template <typename T, int K, int NPT>
 static cudaError_t launch_res(const Inst1D* d_insts, int count, int cl, int seg_cap, int nt,
                               cudaStream_t stream, bool prepare_only) {
-  // one CTA: per-stage CTA barriers; a cluster: the temporally blocked form (one cluster
-  // barrier per step)
-  auto kern = cl > 1 ? rk4_1d_cluster_tb<T, K, NPT> : rk4_1d_resident<T, K, NPT>;
+  // one CTA: per-stage CTA barriers (complex64 takes the register kernel instead); a cluster: the
+  // temporally blocked form (one cluster barrier per step)
   const size_t smem = cl > 1 ? (size_t)4 * (seg_cap + 8 * K) * sizeof(typename C2<T>::type)
                              : (size_t)2 * (seg_cap + 2 * K) * sizeof(typename C2<T>::type);
+  if (cl == 1) {
+    if constexpr (sizeof(T) == 8) {
+      static size_t configured = 0;
+      if (smem > configured) {
+        cudaError_t e = cudaFuncSetAttribute(rk4_1d_resident<K, NPT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                             (int)smem);
+        if (e != cudaSuccess) return e;
+        configured = smem;
+      }
+      if (prepare_only) return cudaSuccess;
+      rk4_1d_resident<K, NPT><<<count, nt, smem, stream>>>(d_insts, seg_cap);
+      return cudaGetLastError();
+    }
+    return cudaErrorInvalidValue;
+  }
+  auto kern = rk4_1d_cluster_tb<T, K, NPT>;
   // Attributes are raised once, monotonically, so launches inside a stream capture never need
   // to change them (prepare_1d_resident runs before any capture).
-  static size_t configured_smem[2] = {0, 0};
+  static size_t configured_smem = 0;
   static bool non_portable = false;
-  const int ki = cl > 1 ? 1 : 0;
-  if (smem > configured_smem[ki]) {
+  if (smem > configured_smem) {
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
-    configured_smem[ki] = smem;
+    configured_smem = smem;
   }
   if (cl > 8 && !non_portable) {
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
@@ -566,7 +494,7 @@ static cudaError_t launch_res_npt(const Inst1D* d, int count, int cl, int seg_ca
     case 2: return launch_res<T, K, 2>(d, count, cl, seg_cap, nt, s, prepare_only);
     case 4: return launch_res<T, K, 4>(d, count, cl, seg_cap, nt, s, prepare_only);
     case 8:
-      if (sizeof(T) == 4) return launch_res<T, K, 8>(d, count, cl, seg_cap, nt, s, prepare_only);
+      if constexpr (sizeof(T) == 4) return launch_res<T, K, 8>(d, count, cl, seg_cap, nt, s, prepare_only);
       return cudaErrorInvalidValue;
     default: return cudaErrorInvalidValue;
   }
@@ -725,9 +653,14 @@ cudaError_t launch_1d_stage(int dtype, int n, int s, const void* src, void* u, c
                             cudaStream_t st) {
   const int K = op.K;
   if (dtype == NLS_C128) {
-    if (K == 1) stage_1d_t<double, 1>(n, s, src, u, P, acc, dst, dt, ph, op, st);
-    else if (K == 2) stage_1d_t<double, 2>(n, s, src, u, P, acc, dst, dt, ph, op, st);
-    else if (K == 3) stage_1d_t<double, 3>(n, s, src, u, P, acc, dst, dt, ph, op, st);
+    const F64Consts c = make_f64(ph, dt);
+    auto go = [&](auto kern) {
+      kern<<<(n + 255) / 256, 256, 0, st>>>(n, s, (const double2*)src, (double2*)u, (const double*)P, (double2*)acc,
+                                            (double2*)dst, c, op);
+    };
+    if (K == 1) go(rk4_1d_stage_f64<1>);
+    else if (K == 2) go(rk4_1d_stage_f64<2>);
+    else if (K == 3) go(rk4_1d_stage_f64<3>);
     else return cudaErrorInvalidValue;
   } else {
     if (K == 1) stage_1d_t<float, 1>(n, s, src, u, P, acc, dst, dt, ph, op, st);

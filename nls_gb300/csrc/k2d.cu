@@ -21,6 +21,7 @@
 #include <tuple>
 #include <functional>
 #include <queue>
+#include <type_traits>
 #include <utility>
 #include <vector>
 
@@ -35,16 +36,10 @@ __device__ __forceinline__ typename C2<T>::type cadd4(typename C2<T>::type a, ty
   return mk<T>((a.x + b.x) + (c.x + d.x), (a.y + b.y) + (c.y + d.y));
 }
 
-// Complex pair arithmetic: Blackwell's packed FP32x2 pipe (FADD2/FMUL2/FFMA2) for complex64,
-// plain FP64 for complex128.
+// Complex pair arithmetic on Blackwell's packed FP32x2 pipe (FADD2/FMUL2/FFMA2).
 __device__ __forceinline__ float2 padd(float2 a, float2 b) { return __fadd2_rn(a, b); }
 __device__ __forceinline__ float2 pfma(float s, float2 b, float2 c) { return __ffma2_rn(make_float2(s, s), b, c); }
 __device__ __forceinline__ float2 pmul(float s, float2 b) { return __fmul2_rn(make_float2(s, s), b); }
-__device__ __forceinline__ double2 padd(double2 a, double2 b) { return make_double2(a.x + b.x, a.y + b.y); }
-__device__ __forceinline__ double2 pfma(double s, double2 b, double2 c) {
-  return make_double2(__fma_rn(s, b.x, c.x), __fma_rn(s, b.y, c.y));
-}
-__device__ __forceinline__ double2 pmul(double s, double2 b) { return make_double2(s * b.x, s * b.y); }
 
 // Fused multiply-add in the working precision (single-precision arguments must not be promoted
 // to the FP64 pipe, which runs at a small fraction of the FP32 rate on GB300).
@@ -97,8 +92,8 @@ template <typename T, int K, int RX, int NJ, int S, int CJ>
 __device__ __forceinline__ void tile_stage(const typename C2<T>::type* __restrict__ in,
                                            typename C2<T>::type* __restrict__ out, int x, int y0,
                                            typename C2<T>::type (&u)[NJ], typename C2<T>::type (&acc)[NJ],
-                                           const T (&pc)[NJ], unsigned dom, const Phys<T>& ph,
-                                           const RK<T>& rk, T wc, T w1, T w2) {
+                                           const T (&pc)[NJ], unsigned dom, const Phys<T> ph,
+                                           const RK<T> rk, T wc, T w1, T w2) {
   typedef typename C2<T>::type C;
   static_assert(NJ % CJ == 0, "row batches");
 #pragma unroll
@@ -152,6 +147,30 @@ __device__ __forceinline__ void tile_stage(const typename C2<T>::type* __restric
         u[j] = pfma(rk.dt6, acc[j], u[j]);
       }
     }
+  }
+}
+
+// The same stage in double precision (f64_node.cuh; one row at a time: the FP64 pipe bounds it).
+template <int K, int RX, int NJ, int S>
+__device__ __forceinline__ void tile_stage_f64(const double2* __restrict__ in, double2* __restrict__ out, int x,
+                                               int y0, double2 (&u)[NJ], double2 (&acc)[NJ], const double (&P)[NJ],
+                                               unsigned dom, const F64Consts& c) {
+#pragma unroll
+  for (int j = 0; j < NJ; ++j) {
+    const int at = (y0 + j) * RX + x;
+    const double2 v = in[at];
+    double vx[4 * K], vy[4 * K];
+#pragma unroll
+    for (int d = 1; d <= K; ++d) {
+      const double2 n0 = in[at - d], n1 = in[at + d], n2 = in[at - d * RX], n3 = in[at + d * RX];
+      vx[4 * d - 4] = n0.x; vx[4 * d - 3] = n1.x; vx[4 * d - 2] = n2.x; vx[4 * d - 1] = n3.x;
+      vy[4 * d - 4] = n0.y; vy[4 * d - 3] = n1.y; vy[4 * d - 2] = n2.y; vy[4 * d - 1] = n3.y;
+    }
+    double2 q;
+    f64_slope_2d<K>(v.x, v.y, vx, vy, f2_split(P[j]), f64_in_range(P[j]), &P[j], c, q.x, q.y);
+    const double2 t = f64_stage(S, u[j], acc[j], q, c);
+    if (S == 4) u[j] = t;
+    else if (dom & (1u << j)) out[at] = t;
   }
 }
 
@@ -283,11 +302,9 @@ rk4_2d_fused(const Inst2D* __restrict__ insts, const TileItem* __restrict__ item
     const int gx = txi * G::TX - H + x;
     const int gy0 = tyi * G::TY - H + y0;
     const bool xin = gx >= 0 && gx < n;
-    const Params<T>& prm = ParamsOf<T>::get(I);
-    const Phys<T> ph = phys_of<T>(prm);
-    const RK<T> rk = rk_of<T>(prm);
-    const T wc = prm.wc, w1 = prm.w1, w2 = prm.w2;
-    const T c12 = prm.c12;
+    // single precision: c12 is folded into the pump here; double: into f64's constants
+    const Params<float>& prm = I.pf;
+    const T c12 = sizeof(T) == 4 ? (T)prm.c12 : (T)1;
 
     C u[NJ], acc[NJ];
     T pc[NJ];
@@ -331,13 +348,21 @@ rk4_2d_fused(const Inst2D* __restrict__ insts, const TileItem* __restrict__ item
     __syncthreads();
     // the staging buffer is free again: fetch the next tile while this one is computed
     if (TMA && threadIdx.x == 0 && nxt < n_items) issue(nxt);
-    tile_stage<T, K, RX, NJ, 1, G::CJ>(buf0, buf1, x, y0, u, acc, pc, dom, ph, rk, wc, w1, w2);
+    auto stage = [&](auto Sc, const C* in, C* out) {
+      constexpr int S = decltype(Sc)::value;
+      if constexpr (sizeof(T) == 8)
+        tile_stage_f64<K, RX, NJ, S>(in, out, x, y0, u, acc, pc, dom, I.f64);
+      else
+        tile_stage<T, K, RX, NJ, S, G::CJ>(in, out, x, y0, u, acc, pc, dom, phys_of<float>(prm), rk_of<float>(prm),
+                                           prm.wc, prm.w1, prm.w2);
+    };
+    stage(std::integral_constant<int, 1>{}, buf0, buf1);
     __syncthreads();
-    tile_stage<T, K, RX, NJ, 2, G::CJ>(buf1, buf0, x, y0, u, acc, pc, dom, ph, rk, wc, w1, w2);
+    stage(std::integral_constant<int, 2>{}, buf1, buf0);
     __syncthreads();
-    tile_stage<T, K, RX, NJ, 3, G::CJ>(buf0, buf1, x, y0, u, acc, pc, dom, ph, rk, wc, w1, w2);
+    stage(std::integral_constant<int, 3>{}, buf0, buf1);
     __syncthreads();
-    tile_stage<T, K, RX, NJ, 4, G::CJ>(buf1, nullptr, x, y0, u, acc, pc, dom, ph, rk, wc, w1, w2);
+    stage(std::integral_constant<int, 4>{}, buf1, nullptr);
 #pragma unroll
     for (int j = 0; j < NJ; ++j)
       if (store & (1u << j)) dst[(size_t)(gy0 + j) * n + gx] = u[j];
@@ -395,6 +420,48 @@ __global__ void __launch_bounds__(256) rk4_2d_stage(int n, int s, const void* __
     a.x += k.x;
     a.y += k.y;
     U[q] = mk<T>(u.x + rk.dt6 * a.x, u.y + rk.dt6 * a.y);
+  }
+}
+
+// The same in double precision (f64_node.cuh).  Bounded by the FP64
+// pipe: 8.5 FP64 instructions a node-stage (32 and two conversions before the float pairs and the
+// fixed-point neighbour sum).
+template <int K>
+__global__ void __launch_bounds__(256) rk4_2d_stage_f64(int n, int s, const double2* __restrict__ src,
+                                                        double2* __restrict__ U, const double* __restrict__ P,
+                                                        double2* __restrict__ acc, double2* __restrict__ dst,
+                                                        F64Consts c) {
+  pdl_wait();
+  pdl_trigger();
+  const int x = blockIdx.x * 32 + (threadIdx.x & 31);
+  const int y = blockIdx.y * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  if (x >= n || y >= n) return;
+  const size_t q = (size_t)y * n + x;
+  double vx[4 * K], vy[4 * K];
+  auto get = [&](int i, int xx, int yy) {
+    const bool in = xx >= 0 && xx < n && yy >= 0 && yy < n;
+    const double2 v = in ? src[(size_t)yy * n + xx] : make_double2(0.0, 0.0);
+    vx[i] = v.x;
+    vy[i] = v.y;
+  };
+#pragma unroll
+  for (int d = 1; d <= K; ++d) {
+    get(4 * d - 4, x - d, y);
+    get(4 * d - 3, x + d, y);
+    get(4 * d - 2, x, y - d);
+    get(4 * d - 1, x, y + d);
+  }
+  const double2 v = src[q], u = U[q];
+  double2 k;
+  const double p = P[q];
+  f64_slope_2d<K>(v.x, v.y, vx, vy, f2_split(p), f64_in_range(p), &p, c, k.x, k.y);
+  double2 a = s == 1 ? make_double2(0.0, 0.0) : acc[q];
+  const double2 t = f64_stage(s, u, a, k, c);
+  if (s < 4) {
+    acc[q] = a;
+    dst[q] = t;
+  } else {
+    U[q] = t;
   }
 }
 
@@ -973,9 +1040,13 @@ cudaError_t launch_2d_stage(int dtype, int n, int s, const void* src, void* u, c
   constexpr int RY = NLSG_STAGE2D_ROWS;
   const dim3 grid((n + 31) / 32, (n + RY - 1) / RY);
   if (dtype == NLS_C128) {
-    const Params<double> p = make_params<double>(ph, dt, op.center, op.w[0], op.w[1]);
-    if (op.K == 1) return launch_pdl(rk4_2d_stage<double, 1>, grid, dim3(32 * RY), 0, st, n, s, src, u, P, acc, dst, p);
-    if (op.K == 2) return launch_pdl(rk4_2d_stage<double, 2>, grid, dim3(32 * RY), 0, st, n, s, src, u, P, acc, dst, p);
+    const F64Consts c = make_f64(ph, dt, op);
+    auto go = [&](auto kern) {
+      return launch_pdl(kern, grid, dim3(32 * RY), 0, st, n, s, (const double2*)src, (double2*)u, (const double*)P,
+                        (double2*)acc, (double2*)dst, c);
+    };
+    if (op.K == 1) return go(rk4_2d_stage_f64<1>);
+    if (op.K == 2) return go(rk4_2d_stage_f64<2>);
     return cudaErrorInvalidValue;
   }
   const Params<float> p = make_params<float>(ph, dt, op.center, op.w[0], op.w[1]);

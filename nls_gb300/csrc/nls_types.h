@@ -3,6 +3,9 @@
 
 #include <stdint.h>
 
+#include <cmath>
+#include <cstring>
+
 #ifdef __CUDACC__
 #define NLSG_HD __host__ __device__
 #else
@@ -24,6 +27,22 @@ struct Params {
   T c3, c4, c5, c6, c12, c13, c14;   // coefficient slots 3-6 and 12-14
   T half_dt, dt, dt6;                // dt/2, dt, dt/6
   T wc, w1, w2;                      // 2-D cross-stencil weights (centre, distance 1, distance 2)
+};
+
+// Constants of the complex128 right-hand side as float pairs and doubles (f64_node.cuh), in the
+// order c13, c14, c3 c12, c4, c5, c6 c12, the step weights dt/2, dt, dt/6, and the 2-D stencil: its
+// centre weight and the unit (the outermost weight) of its whole-number neighbour weights, the
+// latter as a mantissa with bit 63 set and an exponent.
+struct F64Consts {
+  float h[6], l[6];
+  double d[6];
+  double half_dt, dt, dt6;
+  double centre, unit;
+  uint64_t unit_m;
+  int unit_e;
+  float lim;          // |A|, |B| below which the pairs' error is below the state's last place
+  int fast;           // every constant is zero or well inside the range of single precision
+  int pad;
 };
 
 // 1-D radial operator L = D2 + diag(1/r_p) D1 on r_p = p h (make_laplacian, nls/nls.f90:132-295).
@@ -59,7 +78,7 @@ struct Inst1D {
   PhysD ph;
   Stencil1D op;
   Params<float> pf;   // step constants (set_params)
-  Params<double> pd;
+  F64Consts f64;
 };
 
 // 16-byte aligned and sized, so a kernel can fetch a descriptor into shared memory with one bulk
@@ -76,8 +95,40 @@ struct alignas(16) Inst2D {
   Stencil2D op;
   const void* tmap;   // 3 CUtensorMap (u[0], u[1], P) in global memory for the TMA path, or null
   Params<float> pf;   // step constants (set_params)
-  Params<double> pd;
+  F64Consts f64;
 };
+
+inline F64Consts make_f64(const PhysD& ph, double dt, double centre = 0.0, double unit = 0.0) {
+  F64Consts c;
+  std::memset(&c, 0, sizeof(c));
+  const double v[6] = {ph.c13, ph.c14, ph.c3 * ph.c12, ph.c4, ph.c5, ph.c6 * ph.c12};
+  c.fast = 1;
+  for (int i = 0; i < 6; ++i) {
+    c.d[i] = v[i];
+    c.h[i] = (float)v[i];
+    c.l[i] = (float)(v[i] - (double)c.h[i]);
+    const double m = std::fabs(v[i]);
+    if (!(m == 0.0 || (m >= 0x1p-40 && m <= 0x1p20))) c.fast = 0;   // also refuses NaN
+  }
+  c.half_dt = dt * 0.5;
+  c.dt = dt;
+  c.dt6 = dt / 6.0;
+  // the pairs are good to 2^-44 or better of A and B, which enter the state as dt/2 A u and dt/2 B u
+  const double lim = 0x1p-8 / std::fabs(c.half_dt);
+  c.lim = lim < 0x1p60 ? (float)lim : 0x1p60f;
+  c.centre = centre;
+  // unit = unit_m / 2^63 * 2^(unit_e - 1023); 0 outside the normal range (the plain products then)
+  uint64_t bits;
+  std::memcpy(&bits, &unit, 8);
+  c.unit_e = (int)(bits >> 52);
+  if (c.unit_e < 200 || c.unit_e > 1800) c.unit_e = 0;
+  c.unit_m = (bits << 11) | (1ull << 63);
+  c.unit = unit;
+  return c;
+}
+inline F64Consts make_f64(const PhysD& ph, double dt, const Stencil2D& op) {
+  return make_f64(ph, dt, op.center, op.K == 1 ? op.w[0] : -op.w[1]);
+}
 
 template <typename T>
 inline Params<T> make_params(const PhysD& ph, double dt, double wc, double w1, double w2) {
@@ -92,12 +143,12 @@ inline Params<T> make_params(const PhysD& ph, double dt, double wc, double w1, d
 // Fill the precomputed constants of a 2-D instance from its ph, dt and op.
 inline void set_params(Inst2D& I) {
   I.pf = make_params<float>(I.ph, I.dt, I.op.center, I.op.w[0], I.op.w[1]);
-  I.pd = make_params<double>(I.ph, I.dt, I.op.center, I.op.w[0], I.op.w[1]);
+  I.f64 = make_f64(I.ph, I.dt, I.op);
 }
 
 inline void set_params(Inst1D& I) {
   I.pf = make_params<float>(I.ph, I.dt, 0.0, 0.0, 0.0);
-  I.pd = make_params<double>(I.ph, I.dt, 0.0, 0.0, 0.0);
+  I.f64 = make_f64(I.ph, I.dt);
 }
 
 template <typename T> struct ParamsOf;
@@ -109,8 +160,6 @@ template <> struct ParamsOf<float> {
   static NLSG_HD float near(const Stencil1D& s, int p, int i) { return s.nearf[p][i]; }
 };
 template <> struct ParamsOf<double> {
-  static NLSG_HD const Params<double>& get(const Inst2D& I) { return I.pd; }
-  static NLSG_HD const Params<double>& get(const Inst1D& I) { return I.pd; }
   static NLSG_HD double w2(const Stencil1D& s, int i) { return s.w2[i]; }
   static NLSG_HD double w1(const Stencil1D& s, int i) { return s.w1[i]; }
   static NLSG_HD double near(const Stencil1D& s, int p, int i) { return s.near[p][i]; }
