@@ -514,7 +514,7 @@ static cudaError_t launch_reg1d(const Inst1D* d, int count, int seg_cap, cudaStr
   if (npt > 8 || npt < K) return cudaErrorInvalidValue;
   int nt = (seg_cap + npt - 1) / npt;
   nt = ((nt + 31) / 32) * 32;
-  const size_t smem = (size_t)2 * (nt / 32) * 2 * K * sizeof(float2);
+  const size_t smem = reg1d_exchange_bytes(K, nt / 32);
   if (prepare_only) return cudaSuccess;
   switch (npt) {
     case 1: if (K <= 1) { rk4_1d_reg<(K <= 1 ? K : 1), 1><<<count, nt, smem, s>>>(d); return cudaGetLastError(); }
@@ -541,7 +541,7 @@ static cudaError_t launch_reg1d_cl(const Inst1D* d, int count, int cl, int seg_c
   npt = std::min(npt, 8);
   int nt = (nodes + npt - 1) / npt;
   nt = ((nt + 31) / 32) * 32;
-  const size_t smem = ((size_t)2 * (nt / 32) * 2 * K + (size_t)2 * 2 * 4 * K) * sizeof(float2);
+  const size_t smem = reg1d_exchange_bytes(K, nt / 32) + (size_t)2 * 2 * 4 * K * sizeof(float2);
   auto launch = [&](auto kern) -> cudaError_t {
     static bool non_portable = false;
     if (cl > 8 && !non_portable) {

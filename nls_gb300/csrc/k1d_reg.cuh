@@ -40,36 +40,37 @@ __device__ __forceinline__ Reg1DConst<K> reg1d_const(const Inst1D& I) {
 
 // One RK4 stage S over the thread's NPT nodes.  t holds the stage input (re, im per node); on
 // return it holds the next stage's input (S < 4), or u the new state (S = 4).  L / R: the K nodes
-// before the thread's first and after its last node.  Nodes at or beyond n stay zero.
-template <int K, int NPT, int S>
-__device__ __forceinline__ void reg1d_stage(float2 (&t)[NPT], float2 (&acc)[NPT], float2 (&u)[NPT],
-                                            const float (&pc)[NPT], const float (&ir)[NPT],
-                                            const float2 (&L)[K], const float2 (&R)[K], int p0, int n,
-                                            const Reg1DConst<K>& c) {
+// before the thread's first and after its last node.  Nodes at or beyond n stay zero.  NEAR: the
+// warp holds the nodes at the axis (a warp-uniform choice; within it every lane evaluates both
+// forms of its first K nodes and thread 0 takes the near-axis rows).
+template <int K, int NPT, int S, bool NEAR>
+__device__ __forceinline__ void reg1d_stage_form(float2 (&t)[NPT], float2 (&acc)[NPT], float2 (&u)[NPT],
+                                                 const float (&pc)[NPT], const float (&ir)[NPT],
+                                                 const float2 (&L)[K], const float2 (&R)[K], int p0, int n,
+                                                 const Reg1DConst<K>& c) {
   auto at = [&](int idx) -> float2 { return idx < 0 ? L[K + idx] : (idx >= NPT ? R[idx - NPT] : t[idx]); };
   float2 nt[NPT];
 #pragma unroll
   for (int i = 0; i < NPT; ++i) {
     const int p = p0 + i;
-    float2 lu;
-    if (i < K && p0 == 0) {
+    // D2 u + (1/r) D1 u, the centre tap of D1 being zero
+    float2 d2 = mul2(c.w2[K], at(i));
+    float2 d1 = mul2(c.w1[0], at(i - K));
+#pragma unroll
+    for (int d = 1; d <= K; ++d) {
+      d2 = fma2(c.w2[K - d], at(i - d), d2);
+      d2 = fma2(c.w2[K + d], at(i + d), d2);
+      if (d < K) d1 = fma2(c.w1[K - d], at(i - d), d1);
+      d1 = fma2(c.w1[K + d], at(i + d), d1);
+    }
+    float2 lu = fma2(f2(ir[i], ir[i]), d1, d2);
+    if (NEAR && i < K) {
       // near-axis rows (only thread 0 holds nodes p = i < K, as NPT >= K) carry the mirror folds
       // at r = 0; the weights of nodes before 0 are zero
-      lu = mul2(c.near[i < K ? i : 0][0], at(i - K));
+      float2 ln = mul2(c.near[i < K ? i : 0][0], at(i - K));
 #pragma unroll
-      for (int d = 1; d <= 2 * K; ++d) lu = fma2(c.near[i < K ? i : 0][d], at(i - K + d), lu);
-    } else {
-      // D2 u + (1/r) D1 u, the centre tap of D1 being zero
-      float2 d2 = mul2(c.w2[K], at(i));
-      float2 d1 = mul2(c.w1[0], at(i - K));
-#pragma unroll
-      for (int d = 1; d <= K; ++d) {
-        d2 = fma2(c.w2[K - d], at(i - d), d2);
-        d2 = fma2(c.w2[K + d], at(i + d), d2);
-        if (d < K) d1 = fma2(c.w1[K - d], at(i - d), d1);
-        d1 = fma2(c.w1[K + d], at(i + d), d1);
-      }
-      lu = fma2(f2(ir[i], ir[i]), d1, d2);
+      for (int d = 1; d <= 2 * K; ++d) ln = fma2(c.near[i < K ? i : 0][d], at(i - K + d), ln);
+      lu = f2(p0 == 0 ? ln.x : lu.x, p0 == 0 ? ln.y : lu.y);
     }
     // q = (a - i b) u + i L u, r = c12 P / (c13 + c14 |u|^2), a = c3 r - c4, b = c5 |u|^2 + c6 r
     const float2 v = t[i];
@@ -83,11 +84,11 @@ __device__ __forceinline__ void reg1d_stage(float2 (&t)[NPT], float2 (&acc)[NPT]
     else acc[i] = fma2(f2(2.f, 2.f), q, acc[i]);
     if (S < 4) {
       const float2 w = S == 3 ? fma2(f2(2.f, 2.f), q, u[i]) : add2(u[i], q);
-      nt[i] = p < n ? w : f2(0.f, 0.f);
+      nt[i] = f2(p < n ? w.x : 0.f, p < n ? w.y : 0.f);
     } else {
       // the state stays in registers across steps: nodes beyond the grid must stay zero
       const float2 w = fma2(f2(1.f / 3.f, 1.f / 3.f), acc[i], u[i]);
-      u[i] = p < n ? w : f2(0.f, 0.f);
+      u[i] = f2(p < n ? w.x : 0.f, p < n ? w.y : 0.f);
     }
   }
   if (S < 4) {
@@ -95,26 +96,58 @@ __device__ __forceinline__ void reg1d_stage(float2 (&t)[NPT], float2 (&acc)[NPT]
     for (int i = 0; i < NPT; ++i) t[i] = nt[i];
   }
 }
+template <int K, int NPT, int S>
+__device__ __forceinline__ void reg1d_stage(float2 (&t)[NPT], float2 (&acc)[NPT], float2 (&u)[NPT],
+                                            const float (&pc)[NPT], const float (&ir)[NPT],
+                                            const float2 (&L)[K], const float2 (&R)[K], int p0, bool near, int n,
+                                            const Reg1DConst<K>& c) {
+  if (near) reg1d_stage_form<K, NPT, S, true>(t, acc, u, pc, ir, L, R, p0, n, c);
+  else reg1d_stage_form<K, NPT, S, false>(t, acc, u, pc, ir, L, R, p0, n, c);
+}
+
+// Exchange of warp-end nodes within a CTA: [2 parities][nw + 2 warps][2 ends][K] values in shared
+// memory, the first and the last warp's entries (beyond the CTA) zero.  Returns bytes.
+__host__ __device__ inline size_t reg1d_exchange_bytes(int K, int nw) {
+  return (size_t)2 * (nw + 2) * 2 * K * sizeof(float2);
+}
+struct Reg1DEx {
+  float2 *mine, *nb;   // this lane's end of its warp (lanes 0 and 31), and the neighbour's end it reads
+  int parity;          // values between the two parities
+};
+template <int K>
+__device__ __forceinline__ Reg1DEx reg1d_exchange(float2* ex, int warp, int lane, int nw) {
+  for (int i = threadIdx.x; i < 2 * (nw + 2) * 2 * K; i += blockDim.x) ex[i] = f2(0.f, 0.f);
+  Reg1DEx e;
+  e.mine = ex + ((warp + 1) * 2 + (lane == 31 ? 1 : 0)) * K;
+  e.nb = lane == 31 ? ex + ((warp + 2) * 2 + 0) * K : ex + (warp * 2 + 1) * K;
+  e.parity = (nw + 2) * 2 * K;
+  __syncthreads();
+  return e;
+}
 
 // The K nodes before the thread's first node (L) and after its last (R): from the adjacent lanes
 // by shuffle, across a warp boundary from the neighbouring warp's published end nodes (stage
-// parity double-buffers them, so one CTA barrier per stage suffices), zero beyond the grid.
+// parity double-buffers them, so one CTA barrier per stage suffices), zero beyond the CTA.  Without
+// branches: every lane reads a neighbour's end and selects (branches cost a lone warp a quarter of a
+// stage: 8192 nodes on one warp per sub-partition ran at 930 cycles a stage, 250 of them resolving).
 template <int K, int NPT, int S>
-__device__ __forceinline__ void reg1d_halo(const float2 (&t)[NPT], float2 (&L)[K], float2 (&R)[K],
-                                           float2* __restrict__ ex, int warp, int lane, int nw) {
-  float2* e = ex + (S & 1) * (nw * 2 * K);
+__device__ __forceinline__ void reg1d_halo(const float2 (&t)[NPT], float2 (&L)[K], float2 (&R)[K], const Reg1DEx& e,
+                                           int lane) {
+  const int off = (S & 1) ? e.parity : 0;
+  const bool first = lane == 0, lastl = lane == 31;
+  if (first || lastl) {
 #pragma unroll
-  for (int k = 0; k < K; ++k) {
-    if (lane == 0) e[(warp * 2 + 0) * K + k] = t[k];
-    if (lane == 31) e[(warp * 2 + 1) * K + k] = t[NPT - K + k];
+    for (int k = 0; k < K; ++k)
+      e.mine[off + k] = f2(lastl ? t[NPT - K + k].x : t[k].x, lastl ? t[NPT - K + k].y : t[k].y);
   }
   __syncthreads();
 #pragma unroll
   for (int k = 0; k < K; ++k) {
-    L[k] = f2(__shfl_up_sync(0xffffffffu, t[NPT - K + k].x, 1), __shfl_up_sync(0xffffffffu, t[NPT - K + k].y, 1));
-    R[k] = f2(__shfl_down_sync(0xffffffffu, t[k].x, 1), __shfl_down_sync(0xffffffffu, t[k].y, 1));
-    if (lane == 0) L[k] = warp > 0 ? e[((warp - 1) * 2 + 1) * K + k] : f2(0.f, 0.f);
-    if (lane == 31) R[k] = warp < nw - 1 ? e[((warp + 1) * 2 + 0) * K + k] : f2(0.f, 0.f);
+    const float2 v = e.nb[off + k];
+    const float lx = __shfl_up_sync(0xffffffffu, t[NPT - K + k].x, 1), ly = __shfl_up_sync(0xffffffffu, t[NPT - K + k].y, 1);
+    const float rx = __shfl_down_sync(0xffffffffu, t[k].x, 1), ry = __shfl_down_sync(0xffffffffu, t[k].y, 1);
+    L[k] = f2(first ? v.x : lx, first ? v.y : ly);
+    R[k] = f2(lastl ? v.x : rx, lastl ? v.y : ry);
   }
 }
 
@@ -122,11 +155,12 @@ template <int K, int NPT>
 __global__ void __launch_bounds__(512) rk4_1d_reg(const Inst1D* __restrict__ insts) {
   static_assert(NPT >= K, "a thread's neighbours must lie within the adjacent lanes");
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  float2* ex = reinterpret_cast<float2*>(smem_raw);  // [2 parities][warps][2 ends][K]
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nw = blockDim.x >> 5;
   const Inst1D& I = insts[blockIdx.x];
   const int n = I.n;
   const int p0 = tid * NPT;
+  const bool near = warp == 0;
+  const Reg1DEx e = reg1d_exchange<K>(reinterpret_cast<float2*>(smem_raw), warp, lane, nw);
   const Reg1DConst<K> c = reg1d_const<K>(I);
   const float h = (float)I.op.h;
   const float c12 = I.pf.c12;
@@ -148,14 +182,14 @@ __global__ void __launch_bounds__(512) rk4_1d_reg(const Inst1D* __restrict__ ins
   for (int64_t step = 0; step < steps; ++step) {
 #pragma unroll
     for (int i = 0; i < NPT; ++i) t[i] = u[i];
-    reg1d_halo<K, NPT, 1>(t, L, R, ex, warp, lane, nw);
-    reg1d_stage<K, NPT, 1>(t, acc, u, pc, ir, L, R, p0, n, c);
-    reg1d_halo<K, NPT, 2>(t, L, R, ex, warp, lane, nw);
-    reg1d_stage<K, NPT, 2>(t, acc, u, pc, ir, L, R, p0, n, c);
-    reg1d_halo<K, NPT, 3>(t, L, R, ex, warp, lane, nw);
-    reg1d_stage<K, NPT, 3>(t, acc, u, pc, ir, L, R, p0, n, c);
-    reg1d_halo<K, NPT, 4>(t, L, R, ex, warp, lane, nw);
-    reg1d_stage<K, NPT, 4>(t, acc, u, pc, ir, L, R, p0, n, c);
+    reg1d_halo<K, NPT, 1>(t, L, R, e, lane);
+    reg1d_stage<K, NPT, 1>(t, acc, u, pc, ir, L, R, p0, near, n, c);
+    reg1d_halo<K, NPT, 2>(t, L, R, e, lane);
+    reg1d_stage<K, NPT, 2>(t, acc, u, pc, ir, L, R, p0, near, n, c);
+    reg1d_halo<K, NPT, 3>(t, L, R, e, lane);
+    reg1d_stage<K, NPT, 3>(t, acc, u, pc, ir, L, R, p0, near, n, c);
+    reg1d_halo<K, NPT, 4>(t, L, R, e, lane);
+    reg1d_stage<K, NPT, 4>(t, acc, u, pc, ir, L, R, p0, near, n, c);
   }
   float2* __restrict__ Uo = reinterpret_cast<float2*>(I.u);
 #pragma unroll
@@ -180,8 +214,8 @@ __global__ void __launch_bounds__(512) rk4_1d_reg_cl(const Inst1D* __restrict__ 
   constexpr int H = 4 * K;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nw = blockDim.x >> 5;
-  float2* ex = reinterpret_cast<float2*>(smem_raw);   // [2 parities][warps][2 ends][K]
-  float2* halo = ex + 2 * nw * 2 * K;                 // [2 parities][2 sides: left, right][H]
+  float2* ex = reinterpret_cast<float2*>(smem_raw);
+  float2* halo = ex + reg1d_exchange_bytes(K, nw) / sizeof(float2);   // [2 parities][2 sides: left, right][H]
   cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
   const int inst = blockIdx.x / cl, rank = blockIdx.x % cl;
   const Inst1D& I = insts[inst];
@@ -190,6 +224,8 @@ __global__ void __launch_bounds__(512) rk4_1d_reg_cl(const Inst1D* __restrict__ 
   const int q0 = min(n, rank * seg), q1 = min(n, q0 + seg);
   const int lo = max(0, q0 - H), hi = min(n, q1 + H);
   const int p0 = lo + tid * NPT;
+  const bool near = warp == 0 && lo == 0;
+  const Reg1DEx e = reg1d_exchange<K>(ex, warp, lane, nw);
   const Reg1DConst<K> c = reg1d_const<K>(I);
   const float h = (float)I.op.h;
   const float c12 = I.pf.c12;
@@ -226,14 +262,14 @@ __global__ void __launch_bounds__(512) rk4_1d_reg_cl(const Inst1D* __restrict__ 
     }
 #pragma unroll
     for (int i = 0; i < NPT; ++i) t[i] = u[i];
-    reg1d_halo<K, NPT, 1>(t, L, R, ex, warp, lane, nw);
-    reg1d_stage<K, NPT, 1>(t, acc, u, pc, ir, L, R, p0, hi, c);
-    reg1d_halo<K, NPT, 2>(t, L, R, ex, warp, lane, nw);
-    reg1d_stage<K, NPT, 2>(t, acc, u, pc, ir, L, R, p0, hi, c);
-    reg1d_halo<K, NPT, 3>(t, L, R, ex, warp, lane, nw);
-    reg1d_stage<K, NPT, 3>(t, acc, u, pc, ir, L, R, p0, hi, c);
-    reg1d_halo<K, NPT, 4>(t, L, R, ex, warp, lane, nw);
-    reg1d_stage<K, NPT, 4>(t, acc, u, pc, ir, L, R, p0, hi, c);
+    reg1d_halo<K, NPT, 1>(t, L, R, e, lane);
+    reg1d_stage<K, NPT, 1>(t, acc, u, pc, ir, L, R, p0, near, hi, c);
+    reg1d_halo<K, NPT, 2>(t, L, R, e, lane);
+    reg1d_stage<K, NPT, 2>(t, acc, u, pc, ir, L, R, p0, near, hi, c);
+    reg1d_halo<K, NPT, 3>(t, L, R, e, lane);
+    reg1d_stage<K, NPT, 3>(t, acc, u, pc, ir, L, R, p0, near, hi, c);
+    reg1d_halo<K, NPT, 4>(t, L, R, e, lane);
+    reg1d_stage<K, NPT, 4>(t, acc, u, pc, ir, L, R, p0, near, hi, c);
 #pragma unroll
     for (int i = 0; i < NPT; ++i) {
       const int p = p0 + i;
