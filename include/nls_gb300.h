@@ -262,6 +262,14 @@ int nls_test_set_stream_dep_extra(int device, unsigned extra_steps);
  * use. */
 int nls_test_set_stream_steps_per_launch(int mode);
 
+/* No counterpart in the reference.  Test control of the failure path of the bounded waits of the
+ * solves spread over the whole GPU: with extra > 0 every wait for another CTA's values on `device`
+ * asks for a tag that far ahead of the one published, so it gives up after its bound (about a
+ * second), sets the context's status word, and the synchronising call returns NLS_ERR_TIMEOUT; 0
+ * restores normal operation.  No fault is raised and the context stays usable.  Not for production
+ * use. */
+int nls_test_set_exchange_tag_extra(int device, unsigned extra);
+
 #ifdef __cplusplus
 }
 #endif

@@ -319,4 +319,61 @@ NLSG_HD inline void f64_slope_1d(const double (&vx)[2 * K + 1], const double (&v
   ky = dfma(A, vy[K], dfma(-bw, vx[K], lx));
 }
 
+#ifdef __CUDACC__
+// The same with two adjacent lanes a node, part 0 its real and part 1 its imaginary part: each lane
+// splits and squares its own part, the lanes exchange the squares, lane 0 forms A and lane 1 B.
+struct F64Lane {
+  F2 alpha, beta;   // lane 0: -c4 and c3 c12, lane 1: c5 and c6 c12
+  int part;
+};
+__device__ __forceinline__ F64Lane f64_lane(int part, const F64Consts& c) {
+  F64Lane l;
+  l.part = part;
+  l.alpha = part ? F2{c.h[4], c.l[4]} : F2{-c.h[3], -c.l[3]};
+  l.beta = part ? F2{c.h[5], c.l[5]} : F2{c.h[2], c.l[2]};
+  return l;
+}
+__device__ __forceinline__ float f64_other(float v) { return __shfl_xor_sync(0xffffffffu, v, 1); }
+__device__ __forceinline__ double f64_other(double v) { return __shfl_xor_sync(0xffffffffu, v, 1); }
+__device__ __forceinline__ bool f64_coeffs_lanes(double mine, F2 p, bool p_ok, const F64Lane& l, const F64Consts& c,
+                                                 double& A, double& B) {
+  const F2 x = f2_square(f2_split(mine));
+  const F2 o = F2{f64_other(x.h), f64_other(x.l)};
+  const F2 s = l.part ? f2_density(o, x) : f2_density(x, o);
+  bool ok;
+  const F2 r = f2_reservoir(p, s, c, ok);
+  const F2 v = f2_add(f2_mul(l.alpha, l.part ? s : F2{1.f, 0.f}), f2_mul(l.beta, r));
+  const float av = v.h < 0.f ? -v.h : v.h;
+  ok = ok && c.fast != 0 && p_ok && f64_in_range(mine) && av < c.lim;
+  const double val = f2_join(v), his = f64_other(val);
+  A = l.part ? his : val;
+  B = l.part ? val : his;
+  // every lane takes part in the exchange, whatever its own answer
+  const int other_ok = __shfl_xor_sync(0xffffffffu, (int)ok, 1);
+  return ok && other_ok != 0;
+}
+// This lane's part of the slope: v the node, other the other part's neighbours.
+template <int K>
+__device__ __forceinline__ double f64_slope_1d_lanes(double2 v, const double (&other)[2 * K + 1],
+                                                     const double (&row)[2 * K + 1], F2 p, double P, bool p_ok,
+                                                     const F64Lane& l, const F64Consts& c) {
+  const double mine = l.part ? v.y : v.x, his = l.part ? v.x : v.y;
+  double A, B;
+  const bool ok = f64_coeffs_lanes(mine, p, p_ok, l, c, A, B);
+  double s = dmul(row[0], other[0]);
+#pragma unroll
+  for (int d = 1; d <= 2 * K; ++d)
+    if (d != K) s = dfma(row[d], other[d], s);
+  if (!ok) f64_coeffs_plain(v.x, v.y, P, c, A, B);
+  const double m = dfma(dadd(B, -row[K]), his, -s);
+  return dfma(A, mine, l.part ? -m : m);
+}
+// This lane's part of f64_stage.
+__device__ __forceinline__ double f64_stage_lane(int s, double u, double& acc, double k, const F64Consts& c) {
+  if (s == 4) return dfma(c.dt6, dadd(acc, k), u);
+  acc = s == 1 ? k : dfma(2.0, k, acc);
+  return dfma(s == 3 ? c.dt : c.half_dt, k, u);
+}
+#endif
+
 }  // namespace nlsg

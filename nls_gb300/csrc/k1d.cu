@@ -7,12 +7,15 @@
 // `hamiltonian` (nls/nls.f90:621-650), and writes the next stage input.  HBM is touched once per
 // launch (load and store of the state).
 //
+// rk4_1d_wide, rk4_1d_wide_f64 (k1d_wide.cuh): a single solve spread over the whole GPU.
+//
 // rk4_1d_stage: one RK4 stage over an arbitrary-size grid from global memory, the general path
 // for grids too large to stay resident.
 #include <cooperative_groups.h>
 
 #include "kernels.h"
 #include "nls_common.cuh"
+#include "exchange.cuh"
 #include "k1d_reg.cuh"
 
 namespace cg = cooperative_groups;
@@ -107,6 +110,12 @@ __device__ __forceinline__ double2 slope64(const double2* in, int li, const Node
   f64_slope_1d<K>(vx, vy, d.row, d.p, d.P, d.p_ok, c, q.x, q.y);
   return q;
 }
+
+}  // namespace nlsg
+
+#include "k1d_wide.cuh"
+
+namespace nlsg {
 
 template <int K, int NPT>
 __global__ void __launch_bounds__(512) rk4_1d_resident(const Inst1D* __restrict__ insts, int seg_cap) {
@@ -616,6 +625,75 @@ static cudaError_t dispatch_res(int dtype, int K, const Inst1D* d_insts, int cou
     if (K == 3) return launch_res_npt<float, 3>(d_insts, count, cl, seg_cap, s, prepare_only);
   }
   return cudaErrorInvalidValue;
+}
+
+// ---- one grid over the whole GPU (k1d_wide.cuh)
+
+template <typename F>
+static auto wide_kernel(int dtype, int K, F&& f) {
+  if (dtype == NLS_C128) return K == 1 ? f(rk4_1d_wide_f64<1>) : (K == 2 ? f(rk4_1d_wide_f64<2>) : f(rk4_1d_wide_f64<3>));
+  return K == 1 ? f(rk4_1d_wide<1, 1>) : (K == 2 ? f(rk4_1d_wide<2, 2>) : f(rk4_1d_wide<3, 4>));
+}
+
+static size_t wide_smem(int dtype, int K, int threads) {
+  return dtype == NLS_C128 ? (size_t)2 * (threads / 2 + 2 * K) * sizeof(double2)
+                           : reg1d_exchange_bytes(K, threads / 32);
+}
+
+// Segment length, steps per exchange and CTA size: the cheapest by a model of a step in cycles, the
+// four stages (longer when an SM's sub-partitions hold several warps) plus the exchange over the S
+// steps between two.  Constants from the measured instruction rates: a complex128 stage of one warp
+// per sub-partition is about 900 cycles and bound by its FP64 pipe, so more warps add up; a
+// complex64 one is about 180 of latency, of which more warps fill a part.  Grids that fit one CTA,
+// or too large for all CTAs to be resident, stay on the kernels of one CTA or cluster.
+Wide1DPlan wide_1d_plan(int dtype, int K, int n, int sms) {
+  Wide1DPlan best;
+  const int per = dtype == NLS_C128 ? 0 : (K == 1 ? 1 : (K == 2 ? 2 : 4));   // nodes a thread
+  double best_cost = 1e300;
+  for (int threads = 128; threads <= (dtype == NLS_C128 ? 512 : 256); threads *= 2) {
+    const int region = per ? threads * per : threads / 2;
+    for (int S = 1; S <= 8; ++S) {
+      const int seg = region - 8 * K * S;
+      if (seg < 8) break;
+      const int grid = (n + seg - 1) / seg;
+      if (grid < 2) continue;
+      const int on_sm = (grid + sms - 1) / sms, warps = on_sm * threads / 128;
+      const double stage = per ? 180.0 + 60.0 * (warps - 1) : 900.0 * warps;
+      const double cost = 4.0 * stage + 900.0 / S;
+      if (cost >= best_cost) continue;
+      int occ = 0;
+      if (on_sm > 1 || threads > 128)
+        occ = wide_kernel(dtype, K, [&](auto kern) {
+          int nb = 0;
+          return cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, kern, threads, wide_smem(dtype, K, threads)) ==
+                         cudaSuccess ? nb : 0;
+        });
+      else
+        occ = 1;
+      if (on_sm > occ) continue;
+      best_cost = cost;
+      best.grid = grid;
+      best.threads = threads;
+      best.seg = seg;
+      best.S = S;
+    }
+  }
+  return best;
+}
+
+size_t wide_1d_slot_bytes(int dtype, int n) { return (size_t)2 * n * sizeof(uint4) * (dtype == NLS_C128 ? 2 : 1); }
+
+cudaError_t launch_1d_wide(int dtype, int K, const Inst1D& I, const Wide1DPlan& p, void* xbuf, uint32_t tag,
+                           int* wait_flag, cudaStream_t s) {
+  const Wide1D g{p.seg, p.S};
+  return wide_kernel(dtype, K, [&](auto kern) {
+    return launch_coop(kern, dim3(p.grid), dim3(p.threads), wide_smem(dtype, K, p.threads), s, I, g, (uint4*)xbuf, tag,
+                       wait_flag);
+  });
+}
+
+cudaError_t exchange_tag_extra_set_1d(unsigned extra) {
+  return cudaMemcpyToSymbol(g_exchange_tag_extra, &extra, sizeof(extra));
 }
 
 int resident_1d_seg_limit(int dtype) { return dtype == NLS_C128 ? 2048 : 4096; }

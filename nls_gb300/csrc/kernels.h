@@ -29,6 +29,17 @@ inline int shortest_segment(int n, int cl) {
   const int seg = (n + cl - 1) / cl;
   return n - (cl - 1) * seg;
 }
+// One grid over the whole GPU by a cooperative launch (k1d_wide.cuh).  grid = 0: not for this size.
+// A launch of steps steps makes ceil(steps / S) exchanges, tags tag, tag + 1, ...; xbuf: zeroed once
+// when allocated, wide_1d_slot_bytes or more.
+struct Wide1DPlan {
+  int grid = 0, threads = 0, seg = 0, S = 0;
+};
+Wide1DPlan wide_1d_plan(int dtype, int K, int n, int sms);
+size_t wide_1d_slot_bytes(int dtype, int n);
+cudaError_t launch_1d_wide(int dtype, int K, const Inst1D& I, const Wide1DPlan& p, void* xbuf, uint32_t tag,
+                           int* wait_flag, cudaStream_t s);
+cudaError_t exchange_tag_extra_set_1d(unsigned extra);
 cudaError_t launch_1d_stage(int dtype, int n, int s, const void* src, void* u, const void* P,
                             void* acc, void* dst, double dt, const PhysD& ph, const Stencil1D& op,
                             cudaStream_t st);

@@ -69,6 +69,8 @@ struct nls_ctx {
   DevBuf io;        // uploaded inputs of host-buffer calls
   DevBuf diag;      // diagnostics partials and results
   DevBuf diagv;     // H(u) scratch of the device chemical potential
+  DevBuf xbuf;      // tagged exchange slots of cooperative launches, zeroed when allocated
+  uint32_t xtag = 0;    // last tag used in xbuf
   double* h_diag = nullptr;  // pinned
   // Status word of the bounded tile waits of this context's launches (a device int set by a
   // fused 2-D kernel whose copy wait expired), and its pinned host mirror.
@@ -207,6 +209,23 @@ static cudaError_t replay(nls_ctx* ctx, int64_t reps, F&& body) {
 
 // ------------------------------------------------------------------ single solves
 
+// Exchange slots of at least `bytes` and the first of `count` tags no earlier launch on them used.
+static cudaError_t exchange_slots(nls_ctx* ctx, size_t bytes, int64_t count, uint32_t* first) {
+  const bool grow = bytes > ctx->xbuf.bytes;
+  cudaError_t e = ctx->xbuf.ensure(bytes);
+  if (e != cudaSuccess) return e;
+  if (grow || (int64_t)ctx->xtag + count >= (int64_t)0x7fffffff) {
+    if ((e = cudaMemsetAsync(ctx->xbuf.p, 0, ctx->xbuf.bytes, ctx->stream)) != cudaSuccess) return e;
+    ctx->xtag = 0;
+  }
+  *first = ctx->xtag + 1;
+  ctx->xtag += (uint32_t)count;
+  return cudaSuccess;
+}
+
+// RK4 steps per cooperative launch (bounds a launch to well under a second).
+static constexpr int64_t kCoopStepsPerLaunch = 16384;
+
 static int solve_1d_dev(nls_ctx* ctx, int dtype, const nls_problem* pr, int64_t iters,
                         const void* P, void* u) {
   Stencil1D op;
@@ -222,6 +241,20 @@ static int solve_1d_dev(nls_ctx* ctx, int dtype, const nls_problem* pr, int64_t 
     std::memset(&I, 0, sizeof(I));
     I.u = u; I.P = P; I.n = n; I.cl = cl; I.steps = iters; I.dt = pr->dt; I.ph = ph; I.op = op;
     set_params(I);
+    // A solve on its own: spread over the whole GPU, unless it fits one CTA or the kernel a batch
+    // would take computes with other roundings (complex64 on more than 8 CTAs).
+    const Wide1DPlan plan = pr->variant == -1 && (dtype == NLS_C128 || cl <= 8)
+                                ? wide_1d_plan(dtype, op.K, n, ctx->sm_count) : Wide1DPlan();
+    if (plan.grid) {
+      for (int64_t done = 0; done < iters; done += I.steps) {
+        I.steps = std::min(kCoopStepsPerLaunch, iters - done);
+        uint32_t tag;
+        CK(ctx, exchange_slots(ctx, wide_1d_slot_bytes(dtype, n), (I.steps + plan.S - 1) / plan.S, &tag));
+        CK(ctx, launch_1d_wide(dtype, op.K, I, plan, ctx->xbuf.p, tag, ctx->wait_flag, ctx->stream));
+        ctx->launches += 1;
+      }
+      return NLS_OK;
+    }
     CK(ctx, ctx->desc.ensure(sizeof(Inst1D)));
     CK(ctx, cudaMemcpyAsync(ctx->desc.p, &I, sizeof(I), cudaMemcpyHostToDevice, ctx->stream));
     const int seg = (n + cl - 1) / cl;
@@ -1055,6 +1088,7 @@ static void ctx_release(nls_ctx* ctx) {
   ctx->io.release();
   ctx->diag.release();
   ctx->diagv.release();
+  ctx->xbuf.release();
   if (ctx->h_diag) cudaFreeHost(ctx->h_diag);
   if (ctx->wait_flag) cudaFree(ctx->wait_flag);
   if (ctx->h_wait_flag) cudaFreeHost(ctx->h_wait_flag);
@@ -1278,6 +1312,11 @@ NLS_API int nls_test_set_stream_steps_per_launch(int mode) {
 NLS_API int nls_test_set_stream_dep_extra(int device, unsigned extra_steps) {
   if (cudaSetDevice(device) != cudaSuccess) return NLS_ERR_CUDA;
   return stream_dep_extra_set(extra_steps) == cudaSuccess ? NLS_OK : NLS_ERR_CUDA;
+}
+
+NLS_API int nls_test_set_exchange_tag_extra(int device, unsigned extra) {
+  if (cudaSetDevice(device) != cudaSuccess) return NLS_ERR_CUDA;
+  return exchange_tag_extra_set_1d(extra) == cudaSuccess ? NLS_OK : NLS_ERR_CUDA;
 }
 
 NLS_API int nls_batch_set(nls_batch* b, int index, const void* pumping, const void* u0) {
