@@ -254,6 +254,14 @@ NLSG_HD inline double cross_sum_plain(const double (&v)[4 * K], const F64Consts&
   return dmul(c.unit, s);
 }
 
+// A pump as a pair for the 2-D kernels; out of range: NaN, recognised by f2_pump_ok.
+NLSG_HD inline F2 f2_pump(double P) {
+  F2 p = f2_split(P);
+  if (!f64_in_range(P)) p.l = fbits(0x7fc00000u);
+  return p;
+}
+NLSG_HD inline bool f2_pump_ok(F2 p) { return p.l == p.l; }
+
 // Slope of the 2-D model at a node u with the stencil's centre weight folded into B:
 //   k_re = A u_re + (B - centre) u_im - S_im,   k_im = A u_im - (B - centre) u_re + S_re
 // where S is the neighbour part.  Every complex128 2-D kernel uses these functions, so their results
@@ -352,7 +360,23 @@ __device__ __forceinline__ bool f64_coeffs_lanes(double mine, F2 p, bool p_ok, c
   const int other_ok = __shfl_xor_sync(0xffffffffu, (int)ok, 1);
   return ok && other_ok != 0;
 }
-// This lane's part of the slope: v the node, other the other part's neighbours.
+// This lane's part of the slope: v the node, mine its own part, other the other part's neighbours.
+template <int K>
+__device__ __forceinline__ double f64_slope_2d_lanes(double2 v, const double (&other)[4 * K], F2 p, bool p_ok, const double* P,
+                                                     const F64Lane& l, const F64Consts& c) {
+  const double mine = l.part ? v.y : v.x, his = l.part ? v.x : v.y;
+  double A, B;
+  bool oks;
+  const bool ok = f64_coeffs_lanes(mine, p, p_ok, l, c, A, B);
+  double s = cross_sum_fixed<K>(other, c, oks);
+  if (!(ok && oks)) {
+    if (!ok) f64_coeffs_plain(v.x, v.y, *P, c, A, B);
+    if (!oks) s = cross_sum_plain<K>(other, c);
+  }
+  // k_re = A u_re + m, k_im = A u_im - m with m = (B - centre) times the other part minus S
+  const double m = dfma(dadd(B, -c.centre), his, -s);
+  return dfma(A, mine, l.part ? -m : m);
+}
 template <int K>
 __device__ __forceinline__ double f64_slope_1d_lanes(double2 v, const double (&other)[2 * K + 1],
                                                      const double (&row)[2 * K + 1], F2 p, double P, bool p_ok,

@@ -9,6 +9,8 @@
 // tile list may span many independent solves (batched and served forms), each with its own size,
 // coefficients and ping-pong buffers; the persistent grid strides over the list.
 //
+// rk4_2d_wide_f64 (k2d_wide.cuh): a single complex128 grid held on chip by all SMs.
+//
 // rk4_2d_stage: one RK4 stage from global memory (no halo recomputation), used where tiles would
 // be too small to amortise their halo (double precision on modest grids) and as the general path.
 #include <cuda.h>
@@ -222,6 +224,8 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity) {
 
 #include "k2d_reg.cuh"
 #include "k2d_stream.cuh"
+#include "exchange.cuh"
+#include "k2d_wide.cuh"
 
 namespace nlsg {
 
@@ -1026,6 +1030,61 @@ void stream_sort_items(std::vector<StripItem>& items) {
   std::stable_sort(items.begin(), items.end(), [](const StripItem& a, const StripItem& b) {
     return (a.y1 - a.y0) > (b.y1 - b.y0);
   });
+}
+
+// ---- one complex128 grid over the whole GPU (k2d_wide.cuh)
+
+static constexpr size_t kWideSmem = 227 * 1024;
+
+// The tiling with the shortest stage by a model in cycles fitted to measured stages (order 3): one
+// lane a node 3240 at one warp a CTA (40^2), 3830 at 4 (128^2), 4960 at 14 (256^2), 14 230 at 54
+// (512^2); two lanes a node 2900 at 1, 3120 at 8, 6600 at 28 warps (the same grids).  So two lanes
+// up to about 300 nodes a CTA, one beyond, and above 1800 nodes a CTA the stage kernels, whose
+// launches amortise there (600^2: 40.2 us a step against 41.1 here; 512^2: 30.3 against 27.8).
+Wide2DPlan wide_2d_plan(int K, int n, int sms) {
+  Wide2DPlan best;
+  double best_cost = 1e300;
+  for (int gx = 1; gx <= std::min(sms, n); ++gx)
+    for (int gy = 1; gx * gy <= sms && gy <= n; ++gy) {
+      const int w = (n + gx - 1) / gx, h = (n + gy - 1) / gy;
+      if (w * h > 1800 || wide_2d_smem(K, w, h) > kWideSmem) continue;
+      const int inner = w > 2 * K && h > 2 * K ? (w - 2 * K) * (h - 2 * K) : 0, ring = w * h - inner;
+      for (int lanes = 0; lanes < 2; ++lanes) {
+        const int per = lanes ? 16 : 32;
+        const int ew = (ring + per - 1) / per, iw = (inner + per - 1) / per, total = ew + iw;
+        const double cost = (lanes ? std::max(2800.0 + 40.0 * total, 236.0 * total)
+                                   : std::max(3100.0 + 140.0 * total, 263.0 * total)) +
+                            (gx * gy > 1 ? 100.0 : 0.0) + ring + 0.1 * gx * gy;
+        if (cost >= best_cost) continue;
+        best_cost = cost;
+        best.gx = gx;
+        best.gy = gy;
+        best.lanes = lanes != 0;
+        best.edge_warps = std::min(ew, lanes ? 12 : 8);
+        best.threads = 32 * (best.edge_warps + std::min(iw, (lanes ? 32 : 24) - best.edge_warps));
+        best.smem = wide_2d_smem(K, w, h);
+      }
+    }
+  return best;
+}
+
+size_t wide_2d_slot_bytes(int n) { return (size_t)2 * 2 * n * n * sizeof(uint4); }
+
+cudaError_t launch_2d_wide(int K, const Inst2D& I, const Wide2DPlan& p, void* xbuf, uint32_t tag, int* wait_flag,
+                           cudaStream_t s) {
+  const Wide2D g{p.gx, p.gy, p.edge_warps};
+  auto go = [&](auto kern) -> cudaError_t {
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kWideSmem);
+    if (e != cudaSuccess) return e;
+    return launch_coop(kern, dim3(p.gx * p.gy), dim3(p.threads), p.smem, s, I, g, (uint4*)xbuf, tag, wait_flag);
+  };
+  if (K == 1) return p.lanes ? go(rk4_2d_wide_f64<1, true>) : go(rk4_2d_wide_f64<1, false>);
+  if (K == 2) return p.lanes ? go(rk4_2d_wide_f64<2, true>) : go(rk4_2d_wide_f64<2, false>);
+  return cudaErrorInvalidValue;
+}
+
+cudaError_t exchange_tag_extra_set_2d(unsigned extra) {
+  return cudaMemcpyToSymbol(g_exchange_tag_extra, &extra, sizeof(extra));
 }
 
 // Rows of 32 nodes per CTA of the stage kernels.  Two (64-thread CTAs) spread a small grid evenly

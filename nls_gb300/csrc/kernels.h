@@ -142,6 +142,18 @@ void stream_sort_items(std::vector<StripItem>& items);
 // region (k itself included); range[k] = {first, count} into deps.
 void stream_deps(const std::vector<StripItem>& items, const std::vector<int>& ns, int K, std::vector<int2>& range,
                  std::vector<int>& deps);
+// One complex128 grid over the whole GPU by a cooperative launch (k2d_wide.cuh).  gx = 0: not for
+// this size.  A launch of steps steps uses 4 steps + 1 tags; xbuf as for launch_1d_wide.
+struct Wide2DPlan {
+  int gx = 0, gy = 0, edge_warps = 0, threads = 0;
+  bool lanes = false;
+  size_t smem = 0;
+};
+Wide2DPlan wide_2d_plan(int K, int n, int sms);
+size_t wide_2d_slot_bytes(int n);
+cudaError_t launch_2d_wide(int K, const Inst2D& I, const Wide2DPlan& p, void* xbuf, uint32_t tag, int* wait_flag,
+                           cudaStream_t s);
+cudaError_t exchange_tag_extra_set_2d(unsigned extra);
 cudaError_t launch_2d_stage(int dtype, int n, int s, const void* src, void* u, const void* P,
                             void* acc, void* dst, double dt, const PhysD& ph, const Stencil2D& op,
                             cudaStream_t st);

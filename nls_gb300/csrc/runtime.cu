@@ -429,6 +429,22 @@ static int solve_2d_dev(nls_ctx* ctx, int dtype, const nls_problem* pr, int64_t 
   const size_t N = (size_t)n * n;
   const size_t cb = align256(N * csize(dtype));
   if (shape == TILE_UNFUSED) {
+    // a complex128 solve on its own: held on chip by all SMs where it fits
+    const Wide2DPlan plan = pr->variant == -1 && dtype == NLS_C128 ? wide_2d_plan(op.K, n, ctx->sm_count) : Wide2DPlan();
+    if (plan.gx) {
+      Inst2D I;
+      std::memset(&I, 0, sizeof(I));
+      I.u[0] = u; I.P = P; I.n = n; I.dt = pr->dt; I.ph = ph; I.op = op;
+      set_params(I);
+      for (int64_t done = 0; done < iters; done += I.steps) {
+        I.steps = std::min(kCoopStepsPerLaunch, iters - done);
+        uint32_t tag;
+        CK(ctx, exchange_slots(ctx, wide_2d_slot_bytes(n), 4 * I.steps + 1, &tag));
+        CK(ctx, launch_2d_wide(op.K, I, plan, ctx->xbuf.p, tag, ctx->wait_flag, ctx->stream));
+        ctx->launches += 1;
+      }
+      return NLS_OK;
+    }
     CK(ctx, ctx->scratch.ensure(3 * cb));
     char* base = (char*)ctx->scratch.p;
     void *tA = base, *tB = base + cb, *acc = base + 2 * cb;
@@ -1316,7 +1332,7 @@ NLS_API int nls_test_set_stream_dep_extra(int device, unsigned extra_steps) {
 
 NLS_API int nls_test_set_exchange_tag_extra(int device, unsigned extra) {
   if (cudaSetDevice(device) != cudaSuccess) return NLS_ERR_CUDA;
-  return exchange_tag_extra_set_1d(extra) == cudaSuccess ? NLS_OK : NLS_ERR_CUDA;
+  return exchange_tag_extra_set_1d(extra) == cudaSuccess && exchange_tag_extra_set_2d(extra) == cudaSuccess ? NLS_OK : NLS_ERR_CUDA;
 }
 
 NLS_API int nls_batch_set(nls_batch* b, int index, const void* pumping, const void* u0) {
