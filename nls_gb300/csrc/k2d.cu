@@ -226,6 +226,7 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity) {
 #include "k2d_stream.cuh"
 #include "exchange.cuh"
 #include "k2d_wide.cuh"
+#include "k2d_wide_reg.cuh"
 
 namespace nlsg {
 
@@ -1081,6 +1082,55 @@ cudaError_t launch_2d_wide(int K, const Inst2D& I, const Wide2DPlan& p, void* xb
   if (K == 1) return p.lanes ? go(rk4_2d_wide_f64<1, true>) : go(rk4_2d_wide_f64<1, false>);
   if (K == 2) return p.lanes ? go(rk4_2d_wide_f64<2, true>) : go(rk4_2d_wide_f64<2, false>);
   return cudaErrorInvalidValue;
+}
+
+// ---- one complex64 grid over the whole GPU (k2d_wide_reg.cuh)
+
+// Calls f(kernel, config) for the region of shape `shape` (rows 16, 32, 64, 96).
+template <typename F>
+static cudaError_t wide_reg_shape(int K, int shape, F&& f) {
+#define NLSG_WIDE_REG(NW, NJ)                                                                    if (K == 1) return f(rk4_2d_wide_reg<1, NW, NJ>, WideRegCfg<1, NW, NJ>());                     if (K == 2) return f(rk4_2d_wide_reg<2, NW, NJ>, WideRegCfg<2, NW, NJ>());
+  switch (shape) {
+    case 0: if (K == 1) return f(rk4_2d_wide_reg<1, 8, 2>, WideRegCfg<1, 8, 2>()); break;
+    case 1: NLSG_WIDE_REG(8, 4) break;
+    case 2: NLSG_WIDE_REG(16, 4) break;
+    case 3: NLSG_WIDE_REG(12, 8) break;
+  }
+#undef NLSG_WIDE_REG
+  return cudaErrorInvalidValue;
+}
+
+// The lowest region whose tiles all fit: fewer rows a warp, shorter stages.  us a step, order 3, by
+// rows of the region (16 / 32 / 64): 128^2 2.05 / 2.59 / 3.65, 256^2 - / 2.58 / 3.74; streaming 9.3
+// and 9.4.  96 rows as 12 warps of 8 (6.40 at 777^2) rather than 8 of 12 (6.68).  Beyond one tile an
+// SM (840 a side at order 3, 720 at order 5) the streaming and tile kernels; the largest here against
+// those: 840^2 6.35 and 11.6, order 5 700^2 9.03 and 9.83.
+WideReg2DPlan wide_reg_2d_plan(int K, int n, int sms) {
+  WideReg2DPlan best;
+  for (int shape = K == 1 ? 0 : 1; shape <= 3 && !best.tiles; ++shape) {
+    wide_reg_shape(K, shape, [&](auto, auto cfg) {
+      typedef typename decltype(cfg)::G G;
+      const int tx = (n + G::TX - 1) / G::TX, ty = (n + G::TY - 1) / G::TY;
+      if (tx * ty > sms) return cudaSuccess;
+      best.shape = shape;
+      best.tiles_x = tx;
+      best.tiles = tx * ty;
+      return cudaSuccess;
+    });
+  }
+  return best;
+}
+
+size_t wide_reg_2d_slot_bytes(int n) { return (size_t)2 * n * n * sizeof(uint4); }
+
+cudaError_t launch_2d_wide_reg(int K, const Inst2D& I, const WideReg2DPlan& p, void* xbuf, uint32_t tag, int* wait_flag,
+                               cudaStream_t s) {
+  return wide_reg_shape(K, p.shape, [&](auto kern, auto cfg) -> cudaError_t {
+    typedef decltype(cfg) C;
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::SMEM);
+    if (e != cudaSuccess) return e;
+    return launch_coop(kern, dim3(p.tiles), dim3(C::G::NT), C::SMEM, s, I, (uint4*)xbuf, tag, wait_flag);
+  });
 }
 
 cudaError_t exchange_tag_extra_set_2d(unsigned extra) {

@@ -153,6 +153,15 @@ Wide2DPlan wide_2d_plan(int K, int n, int sms);
 size_t wide_2d_slot_bytes(int n);
 cudaError_t launch_2d_wide(int K, const Inst2D& I, const Wide2DPlan& p, void* xbuf, uint32_t tag, int* wait_flag,
                            cudaStream_t s);
+// One complex64 grid, one register tile a CTA.  tiles = 0: not for this size.  A launch of steps
+// steps uses as many tags; the instance's tiles_x is the plan's.
+struct WideReg2DPlan {
+  int shape = 0, tiles_x = 0, tiles = 0;
+};
+WideReg2DPlan wide_reg_2d_plan(int K, int n, int sms);
+size_t wide_reg_2d_slot_bytes(int n);
+cudaError_t launch_2d_wide_reg(int K, const Inst2D& I, const WideReg2DPlan& p, void* xbuf, uint32_t tag, int* wait_flag,
+                               cudaStream_t s);
 cudaError_t exchange_tag_extra_set_2d(unsigned extra);
 cudaError_t launch_2d_stage(int dtype, int n, int s, const void* src, void* u, const void* P,
                             void* acc, void* dst, double dt, const PhysD& ph, const Stencil2D& op,

@@ -464,6 +464,23 @@ static int solve_2d_dev(nls_ctx* ctx, int dtype, const nls_problem* pr, int64_t 
     ctx->launches += 4 * iters;
     return NLS_OK;
   }
+  // a complex64 solve on its own: one register tile per SM where that covers the grid
+  const WideReg2DPlan plan = pr->variant == -1 && dtype == NLS_C64 ? wide_reg_2d_plan(op.K, n, ctx->sm_count)
+                                                                   : WideReg2DPlan();
+  if (plan.tiles) {
+    Inst2D I;
+    std::memset(&I, 0, sizeof(I));
+    I.u[0] = u; I.P = P; I.n = n; I.tiles_x = plan.tiles_x; I.dt = pr->dt; I.ph = ph; I.op = op;
+    set_params(I);
+    for (int64_t done = 0; done < iters; done += I.steps) {
+      I.steps = std::min(kCoopStepsPerLaunch, iters - done);
+      uint32_t tag;
+      CK(ctx, exchange_slots(ctx, wide_reg_2d_slot_bytes(n), I.steps, &tag));
+      CK(ctx, launch_2d_wide_reg(op.K, I, plan, ctx->xbuf.p, tag, ctx->wait_flag, ctx->stream));
+      ctx->launches += 1;
+    }
+    return NLS_OK;
+  }
   if (shape == TILE_STREAM) return solve_2d_stream(ctx, pr, op, ph, iters, P, u);
   // fused: ping-pong between the caller's buffer and one scratch buffer
   const int tx = tile_out_x(shape, op.K), ty = tile_out_y(shape, op.K);
