@@ -470,32 +470,6 @@ __global__ void __launch_bounds__(256) rk4_2d_stage_f64(int n, int s, const doub
   }
 }
 
-template <typename T, int K>
-__global__ void __launch_bounds__(256) rhs_2d(int n, const void* __restrict__ u_, const void* __restrict__ P_,
-                                              void* __restrict__ v_, Params<T> prm) {
-  typedef typename C2<T>::type C;
-  const int x = blockIdx.x * 32 + (threadIdx.x & 31);
-  const int y = blockIdx.y * 8 + (threadIdx.x >> 5);
-  if (x >= n || y >= n) return;
-  const C* __restrict__ src = reinterpret_cast<const C*>(u_);
-  const T* __restrict__ P = reinterpret_cast<const T*>(P_);
-  const Phys<T> ph = phys_of<T>(prm);
-  auto at = [&](int xx, int yy) -> C {
-    return (xx >= 0 && xx < n && yy >= 0 && yy < n) ? src[(size_t)yy * n + xx] : mk<T>(0, 0);
-  };
-  const size_t q = (size_t)y * n + x;
-  const C v = src[q];
-  const C s1 = cadd4<T>(at(x - 1, y), at(x + 1, y), at(x, y - 1), at(x, y + 1));
-  const T wc = prm.wc, w1 = prm.w1, w2 = prm.w2;
-  C lu = mk<T>(wc * v.x + w1 * s1.x, wc * v.y + w1 * s1.y);
-  if (K == 2) {
-    const C s2 = cadd4<T>(at(x - 2, y), at(x + 2, y), at(x, y - 2), at(x, y + 2));
-    lu.x += w2 * s2.x;
-    lu.y += w2 * s2.y;
-  }
-  reinterpret_cast<C*>(v_)[q] = rhs<T>(v, P[q], lu, ph);
-}
-
 // ------------------------------------------------------------------ launchers
 
 // Shape table: region RX x RY computed by (RX/32) x NS warps.
@@ -1162,23 +1136,6 @@ cudaError_t launch_2d_stage(int dtype, int n, int s, const void* src, void* u, c
   if (op.K == 1) return launch_pdl(rk4_2d_stage<float, 1>, grid, dim3(32 * RY), 0, st, n, s, src, u, P, acc, dst, p);
   if (op.K == 2) return launch_pdl(rk4_2d_stage<float, 2>, grid, dim3(32 * RY), 0, st, n, s, src, u, P, acc, dst, p);
   return cudaErrorInvalidValue;
-}
-
-cudaError_t launch_rhs_2d(int dtype, int n, const void* u, const void* P, void* v, const PhysD& ph,
-                          const Stencil2D& op, cudaStream_t st) {
-  dim3 grid((n + 31) / 32, (n + 7) / 8);
-  if (dtype == NLS_C128) {
-    const Params<double> p = make_params<double>(ph, 0.0, op.center, op.w[0], op.w[1]);
-    if (op.K == 1) rhs_2d<double, 1><<<grid, 256, 0, st>>>(n, u, P, v, p);
-    else if (op.K == 2) rhs_2d<double, 2><<<grid, 256, 0, st>>>(n, u, P, v, p);
-    else return cudaErrorInvalidValue;
-  } else {
-    const Params<float> p = make_params<float>(ph, 0.0, op.center, op.w[0], op.w[1]);
-    if (op.K == 1) rhs_2d<float, 1><<<grid, 256, 0, st>>>(n, u, P, v, p);
-    else if (op.K == 2) rhs_2d<float, 2><<<grid, 256, 0, st>>>(n, u, P, v, p);
-    else return cudaErrorInvalidValue;
-  }
-  return cudaGetLastError();
 }
 
 }  // namespace nlsg

@@ -1,48 +1,129 @@
-// kdiag.cu -- FP64 diagnostics on the device: norms, chemical potential sums, error vs a
-// double-precision reference.  Two-pass reductions with a fixed block count and a fixed order,
-// so a result never depends on what else runs on the GPU.
+// kdiag.cu -- FP64 diagnostics on the device: norms, chemical potential sums, damping integral, error
+// vs a double-precision reference.  One launch each: blocks write partial sums, the last block to
+// finish adds them in a fixed order, so a result never depends on what else runs on the GPU.
+//
+// The FP64 pipe would bound these sums, not memory (a DFMA of a warp takes 19 cycles of its SM, a
+// conversion 16; 8 bytes a lane arrive in 12).  The complex64 forms therefore add up groups of 16
+// nodes in pairs of floats (f64_node.cuh) -- products of floats are exact as pairs, the group's sum
+// good to 2^-46 of the sum of its terms' sizes, independently from group to group -- and add the
+// groups in FP64.  Small grids and groups whose values the pairs cannot hold (non-finite, squares near the ends of
+// single precision) are added in FP64 node by node.
+#include <algorithm>
+
 #include "kernels.h"
 #include "nls_common.cuh"
 
 namespace nlsg {
 
-static constexpr int kDiagBlocks = 304;  // 2 x 152 SMs
+static constexpr int kDiagBlocks = 1216;  // 8 x 152 SMs
 static constexpr int kDiagThreads = 256;
 static constexpr int kDiagMaxNV = 4;
+static constexpr int kGroup = 16;         // nodes added up in float pairs
+// Grids from which the groups are added up in pairs: their errors, independent of one another, leave
+// 2^-46 / sqrt(groups), below 2^-52 of the sum of the terms' sizes; smaller grids cost FP64 nothing.
+static constexpr long long kPairsFrom = 65536;
 
-size_t diag_partials_bytes(long long) { return (size_t)kDiagBlocks * kDiagMaxNV * sizeof(double); }
+size_t diag_partials_bytes(long long) { return (size_t)kDiagBlocks * kDiagMaxNV * sizeof(double) + 256; }
 
 __device__ __forceinline__ double weight(int mode, long long i, double dx) {
   return mode == 1 ? (double)i * dx : 1.0;
 }
 
-template <typename T>
-__global__ void __launch_bounds__(kDiagThreads) k_norm(long long n, const void* __restrict__ u_, int mode,
-                                                       double dx, double* __restrict__ part) {
-  typedef typename C2<T>::type C;
-  __shared__ double sm[32 * 2];
-  const C* u = reinterpret_cast<const C*>(u_);
-  double v[2] = {0.0, 0.0};
-  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n;
-       i += (long long)gridDim.x * blockDim.x) {
-    const C a = u[i];
-    const double x = (double)a.x, y = (double)a.y;
-    v[0] += weight(mode, i, dx) * (x * x + y * y);
-    v[1] += (isfinite(x) && isfinite(y)) ? 0.0 : 1.0;
-  }
-  block_sum<2>(v, sm);
+// Block sums to part; the last block of the launch adds all blocks' and writes out.  The word after
+// the partials counts finished blocks; it starts at zero and is left at zero.
+template <int NV>
+__device__ __forceinline__ void diag_finish(double (&v)[NV], double* __restrict__ part, double* __restrict__ out) {
+  __shared__ double sm[32 * NV];
+  __shared__ bool last;
+  block_sum<NV>(v, sm);
+  unsigned* const ticket = reinterpret_cast<unsigned*>(part + kDiagBlocks * kDiagMaxNV);
   if (threadIdx.x == 0) {
-    part[blockIdx.x * 2 + 0] = v[0];
-    part[blockIdx.x * 2 + 1] = v[1];
+#pragma unroll
+    for (int k = 0; k < NV; ++k) part[blockIdx.x * NV + k] = v[k];
+    __threadfence();
+    last = atomicInc(ticket, gridDim.x - 1) == gridDim.x - 1;
   }
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+#pragma unroll
+  for (int k = 0; k < NV; ++k) v[k] = 0.0;
+  for (int b = threadIdx.x; b < (int)gridDim.x; b += blockDim.x)
+#pragma unroll
+    for (int k = 0; k < NV; ++k) v[k] += __ldcg(part + b * NV + k);
+  block_sum<NV>(v, sm);
+  if (threadIdx.x == 0)
+#pragma unroll
+    for (int k = 0; k < NV; ++k) out[k] = v[k];
 }
 
+// acc += t, the error of the high sum kept in the low one.
+__device__ __forceinline__ void pair_add(F2& acc, F2 t) {
+  const F2 s = f2_sum(acc.h, t.h);
+  acc.h = s.h;
+  acc.l = fadd(acc.l, fadd(s.l, t.l));
+}
+__device__ __forceinline__ F2 pair_prod(float a, float b) {
+  F2 r;
+  r.h = fmul(a, b);
+  r.l = ffma(a, b, -r.h);
+  return r;
+}
+// A group's sum of squares from which what single precision loses below 2^-100 is below a double's
+// last place, and no square overflowed (false for NaN).
+__device__ __forceinline__ bool pair_range(float sum_sq) { return sum_sq >= 0x1p-40f && sum_sq < 0x1p100f; }
+__device__ __forceinline__ double pair_value(F2 a) { return f2_join(f2_sum(a.h, a.l)); }
+
+__global__ void __launch_bounds__(kDiagThreads) k_norm_c64(long long n, const float2* __restrict__ u,
+                                                           double* __restrict__ part, double* __restrict__ out) {
+  double v[2] = {0.0, 0.0};
+  const long long stride = (long long)gridDim.x * blockDim.x;
+  for (long long i0 = (long long)blockIdx.x * blockDim.x + threadIdx.x; i0 < n; i0 += kGroup * stride) {
+    float2 a[kGroup];
+#pragma unroll
+    for (int k = 0; k < kGroup; ++k) a[k] = i0 + k * stride < n ? u[i0 + k * stride] : make_float2(0.f, 0.f);
+    F2 s = {0.f, 0.f};
+#pragma unroll
+    for (int k = 0; k < kGroup; ++k) {
+      pair_add(s, pair_prod(a[k].x, a[k].x));
+      pair_add(s, pair_prod(a[k].y, a[k].y));
+    }
+    if (n >= kPairsFrom && pair_range(s.h)) {
+      v[0] += pair_value(s);
+    } else {
+#pragma unroll 1
+      for (int k = 0; k < kGroup; ++k) {
+        if (i0 + k * stride >= n) break;
+        const float2 b = u[i0 + k * stride];
+        const double x = b.x, y = b.y;
+        v[0] += x * x + y * y;
+        v[1] += (isfinite(b.x) && isfinite(b.y)) ? 0.0 : 1.0;
+      }
+    }
+  }
+  diag_finish<2>(v, part, out);
+}
+
+__global__ void __launch_bounds__(kDiagThreads) k_norm_c128(long long n, const double2* __restrict__ u,
+                                                            double* __restrict__ part, double* __restrict__ out) {
+  double v[2] = {0.0, 0.0};
+  int bad = 0;
+  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
+    const double2 a = u[i];
+    v[0] = dfma(a.x, a.x, dfma(a.y, a.y, v[0]));
+    // exponent all ones: infinite or NaN
+    bad += ((dhi(a.x) & 0x7ff00000u) == 0x7ff00000u || (dhi(a.y) & 0x7ff00000u) == 0x7ff00000u) ? 1 : 0;
+  }
+  v[1] = (double)bad;
+  diag_finish<2>(v, part, out);
+}
+
+// Sums of conj(u) H(u) and |u|^2 over one array pair (the radial grids, weighted by r).
 template <typename T>
 __global__ void __launch_bounds__(kDiagThreads) k_mu(long long n, const void* __restrict__ u_,
                                                      const void* __restrict__ h_, int mode, double dx,
-                                                     double* __restrict__ part) {
+                                                     double* __restrict__ part, double* __restrict__ out) {
   typedef typename C2<T>::type C;
-  __shared__ double sm[32 * 3];
   const C* u = reinterpret_cast<const C*>(u_);
   const C* hv = reinterpret_cast<const C*>(h_);
   double v[3] = {0.0, 0.0, 0.0};
@@ -56,12 +137,108 @@ __global__ void __launch_bounds__(kDiagThreads) k_mu(long long n, const void* __
     v[1] += w * (ax * by - ay * bx);
     v[2] += w * (ax * ax + ay * ay);
   }
-  block_sum<3>(v, sm);
-  if (threadIdx.x == 0) {
-    part[blockIdx.x * 3 + 0] = v[0];
-    part[blockIdx.x * 3 + 1] = v[1];
-    part[blockIdx.x * 3 + 2] = v[2];
+  diag_finish<3>(v, part, out);
+}
+
+// The same on a square grid with H(u) (order 5) formed on the way: a warp walks kGroup rows of 32
+// columns with the five rows of its column in registers.  complex64: H in single precision as
+// before, the sums in float pairs; complex128: f64_slope_2d and FP64 sums.  Before, H was written
+// and read back by launches of their own and every term added in FP64.
+__global__ void __launch_bounds__(kDiagThreads) k_mu_2d_c64(int n, const float2* __restrict__ u,
+                                                            const float* __restrict__ P, Params<float> prm,
+                                                            double* __restrict__ part, double* __restrict__ out) {
+  double v[3] = {0.0, 0.0, 0.0};
+  const Phys<float> ph = phys_of<float>(prm);
+  const int lane = threadIdx.x & 31;
+  const int cols = (n + 31) / 32;
+  const long long tiles = (long long)cols * ((n + kGroup - 1) / kGroup);
+  const int warps = blockDim.x >> 5;
+  for (long long t = (long long)blockIdx.x * warps + (threadIdx.x >> 5); t < tiles; t += (long long)gridDim.x * warps) {
+    const int x = (int)(t % cols) * 32 + lane, y0 = (int)(t / cols) * kGroup;
+    if (x >= n) continue;
+    auto at = [&](int xx, int y) -> float2 {
+      return xx >= 0 && xx < n && y >= 0 && y < n ? u[(size_t)y * n + xx] : make_float2(0.f, 0.f);
+    };
+    auto slope = [&](float2 c, float2 s1, float2 s2, float p) -> float2 {
+      const float2 lu = f2(prm.wc * c.x + prm.w1 * s1.x + prm.w2 * s2.x, prm.wc * c.y + prm.w1 * s1.y + prm.w2 * s2.y);
+      return rhs<float>(c, p, lu, ph);
+    };
+    auto sum4 = [](float2 a, float2 b, float2 c, float2 d) -> float2 {
+      return f2((a.x + b.x) + (c.x + d.x), (a.y + b.y) + (c.y + d.y));
+    };
+    float2 w[5];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) w[k] = at(x, y0 - 2 + k);
+    F2 re = {0.f, 0.f}, im = {0.f, 0.f}, m = {0.f, 0.f};
+#pragma unroll
+    for (int j = 0; j < kGroup; ++j) {
+      const int y = y0 + j;
+      w[(j + 4) % 5] = at(x, y + 2);
+      const float2 c = w[(j + 2) % 5];
+      const float p = y < n ? P[(size_t)y * n + x] : 0.f;
+      const float2 h = slope(c, sum4(at(x - 1, y), at(x + 1, y), w[(j + 1) % 5], w[(j + 3) % 5]),
+                             sum4(at(x - 2, y), at(x + 2, y), w[j % 5], w[(j + 4) % 5]), p);
+      if (y < n) {
+        pair_add(re, pair_prod(c.x, h.x));
+        pair_add(re, pair_prod(c.y, h.y));
+        pair_add(im, pair_prod(c.x, h.y));
+        pair_add(im, pair_prod(-c.y, h.x));
+        pair_add(m, pair_prod(c.x, c.x));
+        pair_add(m, pair_prod(c.y, c.y));
+      }
+    }
+    if ((long long)n * n >= kPairsFrom && pair_range(m.h) && fabsf(re.h) < 0x1p100f && fabsf(im.h) < 0x1p100f) {
+      v[0] += pair_value(re);
+      v[1] += pair_value(im);
+      v[2] += pair_value(m);
+    } else {
+#pragma unroll 1
+      for (int y = y0; y < y0 + kGroup && y < n; ++y) {
+        const float2 c = at(x, y);
+        const float2 h = slope(c, sum4(at(x - 1, y), at(x + 1, y), at(x, y - 1), at(x, y + 1)),
+                               sum4(at(x - 2, y), at(x + 2, y), at(x, y - 2), at(x, y + 2)), P[(size_t)y * n + x]);
+        const double ax = c.x, ay = c.y, bx = h.x, by = h.y;
+        v[0] += ax * bx + ay * by;
+        v[1] += ax * by - ay * bx;
+        v[2] += ax * ax + ay * ay;
+      }
+    }
   }
+  diag_finish<3>(v, part, out);
+}
+
+__global__ void __launch_bounds__(kDiagThreads) k_mu_2d_c128(int n, const double2* __restrict__ u,
+                                                             const double* __restrict__ P, F64Consts c,
+                                                             double* __restrict__ part, double* __restrict__ out) {
+  double v[3] = {0.0, 0.0, 0.0};
+  const int cols = (n + 31) / 32, lane = threadIdx.x & 31, warps = blockDim.x >> 5;
+  const long long tiles = (long long)cols * n;
+  for (long long t = (long long)blockIdx.x * warps + (threadIdx.x >> 5); t < tiles; t += (long long)gridDim.x * warps) {
+    const int x = (int)(t % cols) * 32 + lane, y = (int)(t / cols);
+    if (x >= n) continue;
+    double vx[8], vy[8];
+    auto get = [&](int i, int xx, int yy) {
+      const bool in = xx >= 0 && xx < n && yy >= 0 && yy < n;
+      const double2 a = in ? u[(size_t)yy * n + xx] : make_double2(0.0, 0.0);
+      vx[i] = a.x;
+      vy[i] = a.y;
+    };
+#pragma unroll
+    for (int d = 1; d <= 2; ++d) {
+      get(4 * d - 4, x - d, y);
+      get(4 * d - 3, x + d, y);
+      get(4 * d - 2, x, y - d);
+      get(4 * d - 1, x, y + d);
+    }
+    const double2 a = u[(size_t)y * n + x];
+    const double p = P[(size_t)y * n + x];
+    double hx, hy;
+    f64_slope_2d<2>(a.x, a.y, vx, vy, f2_split(p), f64_in_range(p), &p, c, hx, hy);
+    v[0] = dfma(a.x, hx, dfma(a.y, hy, v[0]));
+    v[1] = dfma(a.x, hy, dfma(-a.y, hx, v[1]));
+    v[2] = dfma(a.x, a.x, dfma(a.y, a.y, v[2]));
+  }
+  diag_finish<3>(v, part, out);
 }
 
 template <typename T>
@@ -69,9 +246,8 @@ __global__ void __launch_bounds__(kDiagThreads) k_relerr(long long n, const void
                                                          const double2* __restrict__ b,
                                                          const double* __restrict__ P, double c12,
                                                          double c13, double c14,
-                                                         double* __restrict__ part) {
+                                                         double* __restrict__ part, double* __restrict__ out) {
   typedef typename C2<T>::type C;
-  __shared__ double sm[32 * 4];
   const C* a = reinterpret_cast<const C*>(a_);
   double v[4] = {0.0, 0.0, 0.0, 0.0};
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n;
@@ -87,9 +263,7 @@ __global__ void __launch_bounds__(kDiagThreads) k_relerr(long long n, const void
     v[2] += (na - nb) * (na - nb);
     v[3] += nb * nb;
   }
-  block_sum<4>(v, sm);
-  if (threadIdx.x == 0)
-    for (int k = 0; k < 4; ++k) part[blockIdx.x * 4 + k] = v[k];
+  diag_finish<4>(v, part, out);
 }
 
 // Damping integral of Solution.getDampingIntegral (nls/model.py:350-365): the rectangle rule of
@@ -97,59 +271,103 @@ __global__ void __launch_bounds__(kDiagThreads) k_relerr(long long n, const void
 // radial grid r_i = i * r_step (r_step = n dx / (n - 1), the spacing of linspace(0, n dx, n)) when
 // radial, else by dx^2.
 template <typename T>
+__device__ __forceinline__ double damping_term(typename C2<T>::type a, T P, double c12, double c13, double c14) {
+  const double d = (double)a.x * (double)a.x + (double)a.y * (double)a.y;
+  return (c12 * (double)P / (c13 + c14 * d) - 1.0) * d;
+}
+template <typename T>
 __global__ void __launch_bounds__(kDiagThreads) k_damping(long long n, const void* __restrict__ u_,
                                                           const void* __restrict__ P_, int radial,
                                                           double r_step, double dx, double c12, double c13,
-                                                          double c14, double* __restrict__ part) {
+                                                          double c14, double* __restrict__ part,
+                                                          double* __restrict__ out) {
   typedef typename C2<T>::type C;
-  __shared__ double sm[32 * 1];
   const C* u = reinterpret_cast<const C*>(u_);
   const T* P = reinterpret_cast<const T*>(P_);
   const double two_pi = 6.283185307179586476925286766559;
   double v[1] = {0.0};
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n;
        i += (long long)gridDim.x * blockDim.x) {
-    const C a = u[i];
-    const double d = (double)a.x * (double)a.x + (double)a.y * (double)a.y;
-    const double res = c12 * (double)P[i] / (c13 + c14 * d);
     const double w = radial ? two_pi * ((double)i * r_step) * dx : dx * dx;
-    v[0] += (res - 1.0) * d * w;
+    v[0] += damping_term<T>(u[i], P[i], c12, c13, c14) * w;
   }
-  block_sum<1>(v, sm);
-  if (threadIdx.x == 0) part[blockIdx.x] = v[0];
+  diag_finish<1>(v, part, out);
 }
-
-// Sum the per-block partials in a fixed order (one warp per value).
-__global__ void k_final(const double* __restrict__ part, int nblocks, int nv, double* __restrict__ out) {
-  const int k = threadIdx.x >> 5;
-  const int lane = threadIdx.x & 31;
-  if (k >= nv) return;
-  double s = 0.0;
-  for (int b = lane; b < nblocks; b += 32) s += part[b * nv + k];
-  for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
-  if (lane == 0) out[k] = s;
+// complex64 on a square grid: groups in float pairs, the reservoir as in the complex128 steps.
+__global__ void __launch_bounds__(kDiagThreads) k_damping_2d_c64(long long n, const float2* __restrict__ u,
+                                                                 const float* __restrict__ P, double dx, F64Consts c,
+                                                                 double c12, double c13, double c14,
+                                                                 double* __restrict__ part, double* __restrict__ out) {
+  double v[1] = {0.0};
+  const long long stride = (long long)gridDim.x * blockDim.x;
+  // c12 / (c13 + c14 d): the pump's constant is not folded into the pair of P (exact as it is)
+  const F2 p12 = {(float)c12, (float)(c12 - (double)(float)c12)};
+  for (long long i0 = (long long)blockIdx.x * blockDim.x + threadIdx.x; i0 < n; i0 += kGroup * stride) {
+    float2 a[kGroup];
+    float p[kGroup];
+#pragma unroll
+    for (int k = 0; k < kGroup; ++k) {
+      const bool in = i0 + k * stride < n;
+      a[k] = in ? u[i0 + k * stride] : make_float2(0.f, 0.f);
+      p[k] = in ? P[i0 + k * stride] : 0.f;
+    }
+    F2 s = {0.f, 0.f}, m = {0.f, 0.f};
+    bool ok = c.fast != 0;
+#pragma unroll
+    for (int k = 0; k < kGroup; ++k) {
+      const F2 xx = pair_prod(a[k].x, a[k].x), yy = pair_prod(a[k].y, a[k].y);
+      const F2 d = f2_density(xx, yy);
+      pair_add(m, d);
+      const F2 pc = f2_mul(p12, F2{p[k], 0.f});
+      bool dok;
+      const F2 r = f2_add(f2_reservoir(f2_quick(pc.h, pc.l), d, c, dok), F2{-1.f, 0.f});
+      ok = ok && dok && fabsf(p[k]) < 0x1p40f;
+      const F2 t = f2_mul(r, d);
+      pair_add(s, t);
+    }
+    if (ok && n >= kPairsFrom && pair_range(m.h) && fabsf(s.h) < 0x1p100f) {
+      v[0] += pair_value(s);
+    } else {
+#pragma unroll 1
+      for (int k = 0; k < kGroup; ++k) {
+        if (i0 + k * stride >= n) break;
+        v[0] += damping_term<float>(u[i0 + k * stride], P[i0 + k * stride], c12, c13, c14);
+      }
+    }
+  }
+  v[0] *= dx * dx;
+  diag_finish<1>(v, part, out);
 }
 
 static int blocks_for(long long n) {
-  long long b = (n + kDiagThreads - 1) / kDiagThreads;
-  return (int)(b < kDiagBlocks ? (b < 1 ? 1 : b) : kDiagBlocks);
+  const long long b = (n + kDiagThreads - 1) / kDiagThreads;
+  return (int)std::max<long long>(1, std::min<long long>(b, kDiagBlocks));
 }
 
-cudaError_t diag_norm(int dtype, long long n, const void* u, int mode, double dx, double* part,
-                      double* out, cudaStream_t st) {
-  const int nb = blocks_for(n);
-  if (dtype == NLS_C128) k_norm<double><<<nb, kDiagThreads, 0, st>>>(n, u, mode, dx, part);
-  else k_norm<float><<<nb, kDiagThreads, 0, st>>>(n, u, mode, dx, part);
-  k_final<<<1, 32 * 2, 0, st>>>(part, nb, 2, out);
+cudaError_t diag_norm(int dtype, long long n, const void* u, double* part, double* out, cudaStream_t st) {
+  if (dtype == NLS_C128) k_norm_c128<<<blocks_for(n), kDiagThreads, 0, st>>>(n, (const double2*)u, part, out);
+  else k_norm_c64<<<blocks_for((n + kGroup - 1) / kGroup), kDiagThreads, 0, st>>>(n, (const float2*)u, part, out);
   return cudaGetLastError();
 }
 
 cudaError_t diag_mu(int dtype, long long n, const void* u, const void* v, int mode, double dx,
                     double* part, double* out, cudaStream_t st) {
   const int nb = blocks_for(n);
-  if (dtype == NLS_C128) k_mu<double><<<nb, kDiagThreads, 0, st>>>(n, u, v, mode, dx, part);
-  else k_mu<float><<<nb, kDiagThreads, 0, st>>>(n, u, v, mode, dx, part);
-  k_final<<<1, 32 * 3, 0, st>>>(part, nb, 3, out);
+  if (dtype == NLS_C128) k_mu<double><<<nb, kDiagThreads, 0, st>>>(n, u, v, mode, dx, part, out);
+  else k_mu<float><<<nb, kDiagThreads, 0, st>>>(n, u, v, mode, dx, part, out);
+  return cudaGetLastError();
+}
+
+cudaError_t diag_mu_2d(int dtype, int n, const void* u, const void* P, const PhysD& ph, const Stencil2D& op,
+                       double* part, double* out, cudaStream_t st) {
+  const long long rows = dtype == NLS_C128 ? n : (n + kGroup - 1) / kGroup;
+  const int nb = blocks_for(rows * ((n + 31) / 32) * 32);
+  if (dtype == NLS_C128)
+    // (a step so small that the pairs' limit on dt |a| does not bind)
+    k_mu_2d_c128<<<nb, kDiagThreads, 0, st>>>(n, (const double2*)u, (const double*)P, make_f64(ph, 0x1p-60, op), part, out);
+  else
+    k_mu_2d_c64<<<nb, kDiagThreads, 0, st>>>(n, (const float2*)u, (const float*)P,
+                                             make_params<float>(ph, 0.0, op.center, op.w[0], op.w[1]), part, out);
   return cudaGetLastError();
 }
 
@@ -157,9 +375,20 @@ cudaError_t diag_damping(int dtype, long long n, const void* u, const void* P, i
                          double dx, double c12, double c13, double c14, double* part, double* out,
                          cudaStream_t st) {
   const int nb = blocks_for(n);
-  if (dtype == NLS_C128) k_damping<double><<<nb, kDiagThreads, 0, st>>>(n, u, P, radial, r_step, dx, c12, c13, c14, part);
-  else k_damping<float><<<nb, kDiagThreads, 0, st>>>(n, u, P, radial, r_step, dx, c12, c13, c14, part);
-  k_final<<<1, 32, 0, st>>>(part, nb, 1, out);
+  if (dtype == NLS_C128) {
+    k_damping<double><<<nb, kDiagThreads, 0, st>>>(n, u, P, radial, r_step, dx, c12, c13, c14, part, out);
+  } else if (radial) {
+    k_damping<float><<<nb, kDiagThreads, 0, st>>>(n, u, P, radial, r_step, dx, c12, c13, c14, part, out);
+  } else {
+    PhysD ph = {};
+    ph.c13 = c13;
+    ph.c14 = c14;
+    ph.c12 = c12;
+    F64Consts c = make_f64(ph, 0x1p-60);
+    if (!(std::fabs(c12) <= 0x1p20)) c.fast = 0;
+    k_damping_2d_c64<<<blocks_for((n + kGroup - 1) / kGroup), kDiagThreads, 0, st>>>(
+        n, (const float2*)u, (const float*)P, dx, c, c12, c13, c14, part, out);
+  }
   return cudaGetLastError();
 }
 
@@ -168,9 +397,8 @@ cudaError_t diag_relerr(int dtype_a, long long n, const void* a, const void* b, 
                         cudaStream_t st) {
   const int nb = blocks_for(n);
   const double2* bb = reinterpret_cast<const double2*>(b);
-  if (dtype_a == NLS_C128) k_relerr<double><<<nb, kDiagThreads, 0, st>>>(n, a, bb, P, c12, c13, c14, part);
-  else k_relerr<float><<<nb, kDiagThreads, 0, st>>>(n, a, bb, P, c12, c13, c14, part);
-  k_final<<<1, 32 * 4, 0, st>>>(part, nb, 4, out);
+  if (dtype_a == NLS_C128) k_relerr<double><<<nb, kDiagThreads, 0, st>>>(n, a, bb, P, c12, c13, c14, part, out);
+  else k_relerr<float><<<nb, kDiagThreads, 0, st>>>(n, a, bb, P, c12, c13, c14, part, out);
   return cudaGetLastError();
 }
 

@@ -569,35 +569,37 @@ static int solve_host(nls_ctx* ctx, int dtype, int dim, double dt, double dx, in
 // ------------------------------------------------------------------ diagnostics
 
 static int diag_ensure(nls_ctx* ctx) {
-  CK(ctx, ctx->diag.ensure(diag_partials_bytes(0) + 64 * sizeof(double)));
+  if (!ctx->diag.p) {
+    CK(ctx, ctx->diag.ensure(diag_partials_bytes(0)));
+    CK(ctx, cudaMemsetAsync(ctx->diag.p, 0, ctx->diag.bytes, ctx->stream));
+  }
+  // the sums are written straight to pinned host memory
   if (!ctx->h_diag) CK(ctx, cudaMallocHost(&ctx->h_diag, 64 * sizeof(double)));
   return NLS_OK;
 }
 
-static double* diag_out(nls_ctx* ctx) { return (double*)((char*)ctx->diag.p + diag_partials_bytes(0)); }
-
 // Sums of the chemical potential (nls/nls.f90:921-971) of a device state u: S = sum w conj(u) H(u)
 // and M = sum w |u|^2 (w = r_i in 1-D, 1 in 2-D), FP64, with H evaluated with the order-5
-// operator like the reference.  v is device scratch of the state's size.  Blocks until done.
+// operator like the reference.  dv is device scratch of the state's size (1-D only).  Blocks until
+// done.
 static int chem_pot_dev(nls_ctx* ctx, int dtype, int dim, double dx, int n, const double* coeffs,
                         const void* dP, const void* du, void* dv, double* s_re, double* s_im, double* m) {
   const PhysD ph = phys_of(coeffs);
-  const size_t N = dim == 1 ? (size_t)n : (size_t)n * n;
   int st = diag_ensure(ctx);
   if (st) return st;
   if (dim == 1) {
     Stencil1D op;
     if (host_stencil_1d(n, 5, dx, &op)) return fail(ctx, NLS_ERR_INVALID, "operator");
     CK(ctx, launch_rhs_1d(dtype, n, du, dP, dv, ph, op, ctx->stream));
+    CK(ctx, diag_mu(dtype, n, du, dv, 1, dx, (double*)ctx->diag.p, ctx->h_diag, ctx->stream));
+    ctx->launches += 2;
   } else {
     Stencil2D op;
     host_stencil_2d(5, dx, &op);
-    CK(ctx, launch_rhs_2d(dtype, n, du, dP, dv, ph, op, ctx->stream));
+    CK(ctx, diag_mu_2d(dtype, n, du, dP, ph, op, (double*)ctx->diag.p, ctx->h_diag, ctx->stream));
+    ctx->launches += 1;
   }
-  CK(ctx, diag_mu(dtype, (long long)N, du, dv, dim == 1 ? 1 : 0, dx, (double*)ctx->diag.p, diag_out(ctx), ctx->stream));
-  CK(ctx, cudaMemcpyAsync(ctx->h_diag, diag_out(ctx), 3 * sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
   CK(ctx, cudaStreamSynchronize(ctx->stream));
-  ctx->launches += 3;
   *s_re = ctx->h_diag[0];
   *s_im = ctx->h_diag[1];
   *m = ctx->h_diag[2];
@@ -1237,8 +1239,7 @@ NLS_API int nls_chemical_potential_device(nls_ctx* ctx, int dtype, const nls_pro
   if (dtype != NLS_C128 && dtype != NLS_C64) return fail(ctx, NLS_ERR_INVALID, "bad dtype");
   if ((pr->dim != 1 && pr->dim != 2) || pr->n < 5) return fail(ctx, NLS_ERR_INVALID, "dim 1 or 2 and n >= 5");
   CK(ctx, cudaSetDevice(ctx->device));
-  const size_t N = pr->dim == 1 ? (size_t)pr->n : (size_t)pr->n * pr->n;
-  CK(ctx, ctx->diagv.ensure(N * csize(dtype)));
+  if (pr->dim == 1) CK(ctx, ctx->diagv.ensure((size_t)pr->n * csize(dtype)));
   double sr, si, m;
   int st = chem_pot_dev(ctx, dtype, pr->dim, pr->dx, pr->n, pr->coeffs, pumping_dev, u_dev, ctx->diagv.p, &sr, &si, &m);
   if (st) return st;
@@ -1256,10 +1257,9 @@ NLS_API int nls_norm_device(nls_ctx* ctx, int dtype, int64_t count, const void* 
   CK(ctx, cudaSetDevice(ctx->device));
   int st = diag_ensure(ctx);
   if (st) return st;
-  CK(ctx, diag_norm(dtype, count, u_dev, 0, 0.0, (double*)ctx->diag.p, diag_out(ctx), ctx->stream));
-  CK(ctx, cudaMemcpyAsync(ctx->h_diag, diag_out(ctx), 2 * sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
+  CK(ctx, diag_norm(dtype, count, u_dev, (double*)ctx->diag.p, ctx->h_diag, ctx->stream));
   CK(ctx, cudaStreamSynchronize(ctx->stream));
-  ctx->launches += 2;
+  ctx->launches += 1;
   *sum_sq = ctx->h_diag[0];
   if (nonfinite) *nonfinite = (int64_t)ctx->h_diag[1];
   return ctx->h_diag[1] > 0 ? fail(ctx, NLS_ERR_NONFINITE, "non-finite values in state") : NLS_OK;
@@ -1279,10 +1279,9 @@ NLS_API int nls_damping_integral_device(nls_ctx* ctx, int dtype, const nls_probl
   const double r_step = pr->n > 1 ? (double)pr->n * pr->dx / (double)(pr->n - 1) : 0.0;
   const double* c = pr->coeffs;
   CK(ctx, diag_damping(dtype, N, u_dev, pumping_dev, pr->dim == 1 ? 1 : 0, r_step, pr->dx, c[11], c[12], c[13],
-                       (double*)ctx->diag.p, diag_out(ctx), ctx->stream));
-  CK(ctx, cudaMemcpyAsync(ctx->h_diag, diag_out(ctx), sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
+                       (double*)ctx->diag.p, ctx->h_diag, ctx->stream));
   CK(ctx, cudaStreamSynchronize(ctx->stream));
-  ctx->launches += 2;
+  ctx->launches += 1;
   *integral = ctx->h_diag[0];
   return NLS_OK;
 }
@@ -1299,10 +1298,9 @@ NLS_API int nls_density_error_device(nls_ctx* ctx, int dtype, int64_t count, con
   int st = diag_ensure(ctx);
   if (st) return st;
   CK(ctx, diag_relerr(dtype, count, u_dev, u_ref_c128_dev, pumping_f64_dev, c12, c13, c14,
-                      (double*)ctx->diag.p, diag_out(ctx), ctx->stream));
-  CK(ctx, cudaMemcpyAsync(ctx->h_diag, diag_out(ctx), 4 * sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
+                      (double*)ctx->diag.p, ctx->h_diag, ctx->stream));
   CK(ctx, cudaStreamSynchronize(ctx->stream));
-  ctx->launches += 2;
+  ctx->launches += 1;
   const double* v = ctx->h_diag;
   *rel_l2_density = v[1] > 0 ? std::sqrt(v[0] / v[1]) : std::sqrt(v[0]);
   *rel_l2_reservoir = v[3] > 0 ? std::sqrt(v[2] / v[3]) : std::sqrt(v[2]);
