@@ -79,25 +79,27 @@ __device__ __forceinline__ void async_commit_wait() {
 }
 __device__ __forceinline__ void async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 
-// Per-tile constants as broadcast pairs (both halves equal) for the packed pipe.  The stage
-// slopes are carried pre-multiplied by dt/2 (q = dt/2 * k), so the weights and coefficients of
-// the linear terms hold that factor and RK4 reads
-//   t2 = u + q1, t3 = u + q2, t4 = u + 2 q3, u' = u + (q1 + 2 q2 + 2 q3 + q4) / 3.
-// With L u = wc u + w1 s1 + w2 s2 (s_d: sum of the four neighbours at distance d),
-//   q = a u - i (b - wc) u + i (w1 s1 + w2 s2),   a = c3 r - c4,  b = c5 |u|^2 + c6 r.
+// Per-tile constants as broadcast pairs (both halves equal) for the packed pipe.  Slopes are carried
+// in units of the stencil's outermost weight w (1/h^2 at K = 1, 1/(12 h^2) at K = 2), in which the
+// stencil's weights are whole numbers, q = k / w:
+//   q = a u - i (b + C) u + i S,   a = c3 r - c4,  b = c5 |u|^2 + c6 r  (c3 .. c6 divided by w),
+//   K = 1: C = 4, S = s1;  K = 2: C = 60, S = 16 s1 - s2  (s_d: sum of the four neighbours at distance d)
+// and RK4 reads t2 = u + w dt/2 q1, t3 = u + w dt/2 q2, t4 = u + w dt q3,
+// u' = u + w dt/6 (q1 + 2 q2 + 2 q3 + q4): no multiplication by a stencil weight is left.
 struct RegConst {
-  float2 nwc, w1, w2, c3, nc4, c5, c6, c13, c14, two, third;
+  float2 cw, c16, n16, c3, nc4, c5, c6, c13, c14, two, m1, hw, dtw, dw6;
 };
 
+template <int K>
 __device__ __forceinline__ RegConst reg_const(const Params<float>& p) {
   RegConst c;
-  const float h = p.half_dt;
-  c.nwc = f2(-(h * p.wc), -(h * p.wc)); c.w1 = f2(h * p.w1, h * p.w1); c.w2 = f2(h * p.w2, h * p.w2);
-  c.c3 = f2(h * p.c3, h * p.c3); c.nc4 = f2(-(h * p.c4), -(h * p.c4));
-  c.c5 = f2(h * p.c5, h * p.c5); c.c6 = f2(h * p.c6, h * p.c6);
-  c.c13 = f2(p.c13, p.c13); c.c14 = f2(p.c14, p.c14);
-  c.two = f2(2.f, 2.f);
-  c.third = f2(1.f / 3.f, 1.f / 3.f);
+  auto both = [](float v) { return f2(v, v); };
+  c.cw = both(K == 1 ? 4.f : 60.f);
+  c.c16 = both(16.f); c.n16 = both(-16.f);
+  c.c3 = both(p.u3); c.nc4 = both(-p.u4); c.c5 = both(p.u5); c.c6 = both(p.u6);
+  c.c13 = both(p.c13); c.c14 = both(p.c14);
+  c.two = both(2.f); c.m1 = both(-1.f);
+  c.hw = both(p.hw); c.dtw = both(p.dtw); c.dw6 = both(p.dw6);
   return c;
 }
 
@@ -134,19 +136,17 @@ __device__ __forceinline__ void reg_stage(float2 (&tX)[NJ], float2 (&tY)[NJ], fl
   auto rowX = [&](int r) -> float2 { return r < 0 ? upX[K + r] : (r >= NJ ? dnX[r - NJ] : tX[r]); };
   auto rowY = [&](int r) -> float2 { return r < 0 ? upY[K + r] : (r >= NJ ? dnY[r - NJ] : tY[r]); };
 
-  float2 nX[NJ], nY[NJ];
+  float2 oX[NJ], oY[NJ];   // next stage's input
 #pragma unroll
   for (int j = 0; j < NJ; ++j) {
     const float2 X = tX[j], Y = tY[j];
-    float2 mX, mY;  // w1 s1 + w2 s2 per plane
+    float2 sX, nY;  // S of the real plane, -S of the imaginary one
     if (K == 1) {
       // left neighbour of the pair's first node, right neighbour of its second
       const float lx = __shfl_up_sync(0xffffffffu, X.y, 1), ly = __shfl_up_sync(0xffffffffu, Y.y, 1);
       const float rx = __shfl_down_sync(0xffffffffu, X.x, 1), ry = __shfl_down_sync(0xffffffffu, Y.x, 1);
-      const float2 sX = add2(add2(f2(lx + X.y, X.x + rx), rowX(j - 1)), rowX(j + 1));
-      const float2 sY = add2(add2(f2(ly + Y.y, Y.x + ry), rowY(j - 1)), rowY(j + 1));
-      mX = mul2(c.w1, sX);
-      mY = mul2(c.w1, sY);
+      sX = add2(add2(f2(lx + X.y, X.x + rx), rowX(j - 1)), rowX(j + 1));
+      nY = fma2(c.m1, rowY(j + 1), fma2(c.m1, rowY(j - 1), f2(-ly - Y.y, -Y.x - ry)));
     } else {
       // both nodes of the pairs to the left (L) and right (R)
       const float2 LX = f2(__shfl_up_sync(0xffffffffu, X.x, 1), __shfl_up_sync(0xffffffffu, X.y, 1));
@@ -155,10 +155,10 @@ __device__ __forceinline__ void reg_stage(float2 (&tX)[NJ], float2 (&tY)[NJ], fl
       const float2 RY = f2(__shfl_down_sync(0xffffffffu, Y.x, 1), __shfl_down_sync(0xffffffffu, Y.y, 1));
       const float2 s1X = add2(add2(f2(LX.y + X.y, X.x + RX.x), rowX(j - 1)), rowX(j + 1));
       const float2 s1Y = add2(add2(f2(LY.y + Y.y, Y.x + RY.x), rowY(j - 1)), rowY(j + 1));
-      const float2 s2X = add2(add2(add2(LX, RX), rowX(j - 2)), rowX(j + 2));
+      const float2 n2X = fma2(c.m1, rowX(j + 2), fma2(c.m1, rowX(j - 2), f2(-LX.x - RX.x, -LX.y - RX.y)));
       const float2 s2Y = add2(add2(add2(LY, RY), rowY(j - 2)), rowY(j + 2));
-      mX = fma2(c.w2, s2X, mul2(c.w1, s1X));
-      mY = fma2(c.w2, s2Y, mul2(c.w1, s1Y));
+      sX = fma2(c.c16, s1X, n2X);
+      nY = fma2(c.n16, s1Y, s2Y);
     }
     // r = c12 P / (c13 + c14 |u|^2), |u|^2 per node in scalar arithmetic (a packed square of a
     // register pair with itself costs extra register moves)
@@ -166,9 +166,9 @@ __device__ __forceinline__ void reg_stage(float2 (&tX)[NJ], float2 (&tY)[NJ], fl
     const float2 den = fma2(c.c14, sq, c.c13);
     const float2 r = mul2(pc[j], f2(rcp_approx(den.x), rcp_approx(den.y)));
     const float2 a = fma2(c.c3, r, c.nc4);
-    const float2 bw = fma2(c.c5, sq, fma2(c.c6, r, c.nwc));
-    const float2 kX = fma2(a, X, fma2(bw, Y, neg2(mY)));
-    const float2 kY = fma2(a, Y, fma2(neg2(bw), X, mX));
+    const float2 bw = fma2(c.c5, sq, fma2(c.c6, r, c.cw));
+    const float2 kX = fma2(a, X, fma2(bw, Y, nY));
+    const float2 kY = fma2(a, Y, fma2(neg2(bw), X, sX));
     if (S == 1) {
       aX[j] = kX;
       aY[j] = kY;
@@ -181,44 +181,41 @@ __device__ __forceinline__ void reg_stage(float2 (&tX)[NJ], float2 (&tY)[NJ], fl
     }
     if (S < 4) {
       float2 vX, vY;
-      // Next stage input u + q (u + 2 q before stage 4).  Packed or scalar by tile shape, as
-      // measured on the GB300: scalar is faster for strips of up to 10 rows and at order 5,
-      // packed for 12-row strips at order 3 (the register allocation differs, not the work).
+      // Next stage input.  Packed or scalar by tile shape, as measured on the GB300: scalar is
+      // faster for strips of up to 10 rows and at order 5, packed for 12-row strips at order 3 (the
+      // register allocation differs, not the work).
       constexpr bool kScalarUpdate = NJ <= 10 || K == 2;
+      const float2 w = S == 3 ? c.dtw : c.hw;
       if (kScalarUpdate) {
-        const float m = S == 3 ? 2.f : 1.f;
-        vX = f2(__fmaf_rn(m, kX.x, uX[j].x), __fmaf_rn(m, kX.y, uX[j].y));
-        vY = f2(__fmaf_rn(m, kY.x, uY[j].x), __fmaf_rn(m, kY.y, uY[j].y));
-      } else if (S == 3) {
-        vX = fma2(c.two, kX, uX[j]);
-        vY = fma2(c.two, kY, uY[j]);
+        vX = f2(__fmaf_rn(w.x, kX.x, uX[j].x), __fmaf_rn(w.x, kX.y, uX[j].y));
+        vY = f2(__fmaf_rn(w.x, kY.x, uY[j].x), __fmaf_rn(w.x, kY.y, uY[j].y));
       } else {
-        vX = add2(uX[j], kX);
-        vY = add2(uY[j], kY);
+        vX = fma2(w, kX, uX[j]);
+        vY = fma2(w, kY, uY[j]);
       }
       if (EDGE) {
         const bool i0 = (dom0 >> j) & 1u, i1 = (dom1 >> j) & 1u;
         vX = f2(i0 ? vX.x : 0.f, i1 ? vX.y : 0.f);
         vY = f2(i0 ? vY.x : 0.f, i1 ? vY.y : 0.f);
       }
-      nX[j] = vX;
-      nY[j] = vY;
+      oX[j] = vX;
+      oY[j] = vY;
     } else {
       if (NJ <= 10 || K == 2) {  // scalar for the same shapes as the stage-input update
-        const float th = 1.f / 3.f;
+        const float th = c.dw6.x;
         uX[j] = f2(__fmaf_rn(th, aX[j].x, uX[j].x), __fmaf_rn(th, aX[j].y, uX[j].y));
         uY[j] = f2(__fmaf_rn(th, aY[j].x, uY[j].x), __fmaf_rn(th, aY[j].y, uY[j].y));
       } else {
-        uX[j] = fma2(c.third, aX[j], uX[j]);
-        uY[j] = fma2(c.third, aY[j], uY[j]);
+        uX[j] = fma2(c.dw6, aX[j], uX[j]);
+        uY[j] = fma2(c.dw6, aY[j], uY[j]);
       }
     }
   }
   if (S < 4) {
 #pragma unroll
     for (int j = 0; j < NJ; ++j) {
-      tX[j] = nX[j];
-      tY[j] = nY[j];
+      tX[j] = oX[j];
+      tY[j] = oY[j];
     }
   }
 }
@@ -274,7 +271,7 @@ rk4_2d_reg(const Inst2D* __restrict__ insts, const TileItem* __restrict__ items,
     const int gy0 = ry0 + y0;
     const bool edge = rx0 < 0 || ry0 < 0 || rx0 + G::RX > n || ry0 + G::RY > n;
     const Params<float>& prm = I.pf;
-    const RegConst c = reg_const(prm);
+    const RegConst c = reg_const<K>(prm);
     const float2 c12 = f2(prm.c12, prm.c12);
     float2 uX[NJ], uY[NJ], pc[NJ];
     unsigned dom0 = 0, dom1 = 0;

@@ -15,7 +15,7 @@
 //     and the 4K rows of warm-up and drain at segment ends inside the grid;
 //   * horizontal neighbours come from the adjacent lanes by warp shuffle; at a strip edge that is
 //     the grid edge the missing neighbours are masked to zero (the reference's truncated
-//     operator), and columns beyond the grid hold zero state with a zero stencil weight, so their
+//     operator), and columns beyond the grid hold zero state with zero step weights, so their
 //     stage values stay exactly zero;
 //   * rows are prefetched D rows ahead with cp.async into a per-warp shared-memory ring (each lane
 //     copies and later reads only its own bytes, so no warp synchronisation is involved; rows
@@ -84,13 +84,14 @@ struct StreamCfg {
   static_assert(W >= 4 * K + 1 && R % W == 0 && R >= D + 2, "window and ring");
 };
 
-// Per-warp constants of an item: broadcast pairs of the step coefficients (pre-multiplied by
-// dt/2 like the register tile's, see RegConst) and per-lane stencil weights and edge masks.
+// Per-warp constants of an item: broadcast pairs of the coefficients in units of the stencil's
+// outermost weight (see RegConst), and per lane the step weights (zero for columns outside the grid,
+// whose stage values therefore stay zero) and the edge masks.
 struct StreamConst {
-  float2 w1, nw1, w2, nw2;     // +-dt/2 w_d, zero for columns outside the grid
-  float2 nwc, c3, nc4, c5, c6, c13, c14, c12, two, third;
+  float2 hw, dtw, dw6;
+  float2 cw, c16, n16, c3, nc4, c5, c6, c13, c14, c12, two, m1;
   float mL, mR;                // 0 where the left / right neighbour lies beyond the grid edge
-  float2 mL2, mR2;
+  float2 mL2, mR2, nmL2, nmR2;
 };
 
 template <int BYTES>
@@ -131,36 +132,19 @@ __device__ __forceinline__ void st_node_if(bool p, float2* dst, float a, float b
 #ifndef NLSG_STREAM_PACKED_SQ
 #define NLSG_STREAM_PACKED_SQ (K == 1)
 #endif
-// RK4 accumulation and stage-input updates in scalar FMAs (the packed FP32x2 operations all issue
-// to one FMA pipe, scalar ones can use the other).  Measured 0.3 % slower on a 4096^2 grid; so are
-// |u|^2 in scalar FMAs at order 3 (0.9 %) and the new state in four scalar FMAs (0.8 %).
-#ifndef NLSG_STREAM_SCALAR_UPDATE
-#define NLSG_STREAM_SCALAR_UPDATE 0
-#endif
-
-
-// c = m * a + b per component with a scalar multiplier (scalar FMAs)
-__device__ __forceinline__ float2 sfma(float m, float2 a, float2 b) {
-  return f2(__fmaf_rn(m, a.x, b.x), __fmaf_rn(m, a.y, b.y));
-}
-__device__ __forceinline__ float2 sadd(float2 a, float2 b) { return f2(a.x + b.x, a.y + b.y); }
-
-// Slope of one stage at the centre row of the window (slot C), pre-multiplied by dt/2:
-//   q = a u - i (b - wc) u + i L'u,  L'u = w1 s1 + w2 s2,  a = c3 r - c4,  b = c5 |u|^2 + c6 r,
-//   r = c12 P / (c13 + c14 |u|^2)                                     (nls/nls.f90:570-650)
+// Slope of one stage at the centre row of the window (slot C), in units of the stencil's outermost
+// weight: q = a u - i (b + C) u + i S (see RegConst; nls/nls.f90:570-650)
 template <int K, int W, int C>
 __device__ __forceinline__ void stream_slope(const float2 (&inX)[W], const float2 (&inY)[W], float2 pcv,
                                              const StreamConst& c, float2& qX, float2& qY) {
   constexpr int U1 = (C - 1 + W) % W, D1 = (C + 1) % W;
   const float2 X = inX[C], Y = inY[C];
-  float2 mX, nmY;
+  float2 sX, nY;   // S of the real plane, -S of the imaginary one
   if (K == 1) {
     const float lx = __shfl_up_sync(0xffffffffu, X.y, 1), ly = __shfl_up_sync(0xffffffffu, Y.y, 1);
     const float rx = __shfl_down_sync(0xffffffffu, X.x, 1), ry = __shfl_down_sync(0xffffffffu, Y.x, 1);
-    const float2 sX = add2(add2(f2(__fmaf_rn(c.mL, lx, X.y), __fmaf_rn(c.mR, rx, X.x)), inX[U1]), inX[D1]);
-    const float2 sY = add2(add2(f2(__fmaf_rn(c.mL, ly, Y.y), __fmaf_rn(c.mR, ry, Y.x)), inY[U1]), inY[D1]);
-    mX = mul2(c.w1, sX);
-    nmY = mul2(c.nw1, sY);
+    sX = add2(add2(f2(__fmaf_rn(c.mL, lx, X.y), __fmaf_rn(c.mR, rx, X.x)), inX[U1]), inX[D1]);
+    nY = fma2(c.m1, inY[D1], fma2(c.m1, inY[U1], f2(__fmaf_rn(-c.mL, ly, -Y.y), __fmaf_rn(-c.mR, ry, -Y.x))));
   } else {
     constexpr int U2 = (C - 2 + 2 * W) % W, D2 = (C + 2) % W;
     const float2 LX = f2(__shfl_up_sync(0xffffffffu, X.x, 1), __shfl_up_sync(0xffffffffu, X.y, 1));
@@ -169,19 +153,19 @@ __device__ __forceinline__ void stream_slope(const float2 (&inX)[W], const float
     const float2 RY = f2(__shfl_down_sync(0xffffffffu, Y.x, 1), __shfl_down_sync(0xffffffffu, Y.y, 1));
     const float2 s1X = add2(add2(f2(__fmaf_rn(c.mL, LX.y, X.y), __fmaf_rn(c.mR, RX.x, X.x)), inX[U1]), inX[D1]);
     const float2 s1Y = add2(add2(f2(__fmaf_rn(c.mL, LY.y, Y.y), __fmaf_rn(c.mR, RY.x, Y.x)), inY[U1]), inY[D1]);
-    const float2 s2X = add2(add2(fma2(c.mL2, LX, mul2(c.mR2, RX)), inX[U2]), inX[D2]);
+    const float2 n2X = fma2(c.m1, inX[D2], fma2(c.m1, inX[U2], fma2(c.nmL2, LX, mul2(c.nmR2, RX))));
     const float2 s2Y = add2(add2(fma2(c.mL2, LY, mul2(c.mR2, RY)), inY[U2]), inY[D2]);
-    mX = fma2(c.w2, s2X, mul2(c.w1, s1X));
-    nmY = fma2(c.nw2, s2Y, mul2(c.nw1, s1Y));
+    sX = fma2(c.c16, s1X, n2X);
+    nY = fma2(c.n16, s1Y, s2Y);
   }
   const float2 sq = NLSG_STREAM_PACKED_SQ ? fma2(X, X, mul2(Y, Y))
                                          : f2(__fmaf_rn(X.x, X.x, Y.x * Y.x), __fmaf_rn(X.y, X.y, Y.y * Y.y));
   const float2 den = fma2(c.c14, sq, c.c13);
   const float2 r = mul2(pcv, f2(rcp_approx(den.x), rcp_approx(den.y)));
   const float2 a = fma2(c.c3, r, c.nc4);
-  const float2 bw = fma2(c.c5, sq, fma2(c.c6, r, c.nwc));
-  qX = fma2(a, X, fma2(bw, Y, nmY));
-  qY = fma2(a, Y, fma2(neg2(bw), X, mX));
+  const float2 bw = fma2(c.c5, sq, fma2(c.c6, r, c.cw));
+  qX = fma2(a, X, fma2(bw, Y, nY));
+  qY = fma2(a, Y, fma2(neg2(bw), X, sX));
 }
 
 // The rolling windows of one warp (registers): state, c12 * pump, RK4 accumulator and the inputs
@@ -318,26 +302,28 @@ rk4_2d_stream(const Inst2D* __restrict__ insts, const StripItem* __restrict__ it
     StreamConst c;
     {
       const Params<float>& p = I.pf;
-      const float h = p.half_dt;
-      const float w1 = h * p.w1, w2 = h * p.w2;
-      c.w1 = f2(in0 ? w1 : 0.f, in1 ? w1 : 0.f);
-      c.nw1 = f2(in0 ? -w1 : 0.f, in1 ? -w1 : 0.f);
-      c.w2 = f2(in0 ? w2 : 0.f, in1 ? w2 : 0.f);
-      c.nw2 = f2(in0 ? -w2 : 0.f, in1 ? -w2 : 0.f);
-      c.nwc = f2(-(h * p.wc), -(h * p.wc));
-      c.c3 = f2(h * p.c3, h * p.c3);
-      c.nc4 = f2(-(h * p.c4), -(h * p.c4));
-      c.c5 = f2(h * p.c5, h * p.c5);
-      c.c6 = f2(h * p.c6, h * p.c6);
-      c.c13 = f2(p.c13, p.c13);
-      c.c14 = f2(p.c14, p.c14);
-      c.c12 = f2(p.c12, p.c12);
-      c.two = f2(2.f, 2.f);
-      c.third = f2(1.f / 3.f, 1.f / 3.f);
+      auto both = [](float v) { return f2(v, v); };
+      c.hw = f2(in0 ? p.hw : 0.f, in1 ? p.hw : 0.f);
+      c.dtw = f2(in0 ? p.dtw : 0.f, in1 ? p.dtw : 0.f);
+      c.dw6 = f2(in0 ? p.dw6 : 0.f, in1 ? p.dw6 : 0.f);
+      c.cw = both(K == 1 ? 4.f : 60.f);
+      c.c16 = both(16.f);
+      c.n16 = both(-16.f);
+      c.c3 = both(p.u3);
+      c.nc4 = both(-p.u4);
+      c.c5 = both(p.u5);
+      c.c6 = both(p.u6);
+      c.c13 = both(p.c13);
+      c.c14 = both(p.c14);
+      c.c12 = both(p.c12);
+      c.two = both(2.f);
+      c.m1 = both(-1.f);
       c.mL = (lane == 0 && it.x0 == 0) ? 0.f : 1.f;
       c.mR = (lane == 31 && (int)it.x0 + 64 == n) ? 0.f : 1.f;
       c.mL2 = f2(c.mL, c.mL);
       c.mR2 = f2(c.mR, c.mR);
+      c.nmL2 = f2(-c.mL, -c.mL);
+      c.nmR2 = f2(-c.mR, -c.mR);
     }
 
     const int ib = y0 - 4 * K > 0 ? y0 - 4 * K : 0;   // first row loaded
@@ -412,7 +398,7 @@ rk4_2d_stream(const Inst2D* __restrict__ insts, const StripItem* __restrict__ it
       async_commit();
       roff += (uint32_t)n;
 
-      // stage 1 at row i - K: input u, output t2 = u + q1, a = q1
+      // stage 1 at row i - K: input u, output t2 = u + w dt/2 q1, a = q1
       {
         constexpr int C = ((P - K) % W + W) % W;
         const int r = i - K;
@@ -427,11 +413,11 @@ rk4_2d_stream(const Inst2D* __restrict__ insts, const StripItem* __restrict__ it
           stream_slope<K, W, C>(w.uX, w.uY, w.pc[C], c, qX, qY);
           w.aX[C] = qX;
           w.aY[C] = qY;
-          w.t2X[C] = NLSG_STREAM_SCALAR_UPDATE ? sadd(w.uX[C], qX) : add2(w.uX[C], qX);
-          w.t2Y[C] = NLSG_STREAM_SCALAR_UPDATE ? sadd(w.uY[C], qY) : add2(w.uY[C], qY);
+          w.t2X[C] = fma2(c.hw, qX, w.uX[C]);
+          w.t2Y[C] = fma2(c.hw, qY, w.uY[C]);
         }
       }
-      // stage 2 at row i - 2K: input t2, output t3 = u + q2, a += 2 q2
+      // stage 2 at row i - 2K: input t2, output t3 = u + w dt/2 q2, a += 2 q2
       {
         constexpr int C = ((P - 2 * K) % W + W) % W;
         const int r = i - 2 * K;
@@ -441,20 +427,13 @@ rk4_2d_stream(const Inst2D* __restrict__ insts, const StripItem* __restrict__ it
         } else {
           float2 qX, qY;
           stream_slope<K, W, C>(w.t2X, w.t2Y, w.pc[C], c, qX, qY);
-          if (NLSG_STREAM_SCALAR_UPDATE) {
-            w.aX[C] = sfma(2.f, qX, w.aX[C]);
-            w.aY[C] = sfma(2.f, qY, w.aY[C]);
-            w.t3X[C] = sadd(w.uX[C], qX);
-            w.t3Y[C] = sadd(w.uY[C], qY);
-          } else {
-            w.aX[C] = fma2(c.two, qX, w.aX[C]);
-            w.aY[C] = fma2(c.two, qY, w.aY[C]);
-            w.t3X[C] = add2(w.uX[C], qX);
-            w.t3Y[C] = add2(w.uY[C], qY);
-          }
+          w.aX[C] = fma2(c.two, qX, w.aX[C]);
+          w.aY[C] = fma2(c.two, qY, w.aY[C]);
+          w.t3X[C] = fma2(c.hw, qX, w.uX[C]);
+          w.t3Y[C] = fma2(c.hw, qY, w.uY[C]);
         }
       }
-      // stage 3 at row i - 3K: input t3, output t4 = u + 2 q3, a += 2 q3
+      // stage 3 at row i - 3K: input t3, output t4 = u + w dt q3, a += 2 q3
       {
         constexpr int C = ((P - 3 * K) % W + W) % W;
         const int r = i - 3 * K;
@@ -464,20 +443,13 @@ rk4_2d_stream(const Inst2D* __restrict__ insts, const StripItem* __restrict__ it
         } else {
           float2 qX, qY;
           stream_slope<K, W, C>(w.t3X, w.t3Y, w.pc[C], c, qX, qY);
-          if (NLSG_STREAM_SCALAR_UPDATE) {
-            w.aX[C] = sfma(2.f, qX, w.aX[C]);
-            w.aY[C] = sfma(2.f, qY, w.aY[C]);
-            w.t4X[C] = sfma(2.f, qX, w.uX[C]);
-            w.t4Y[C] = sfma(2.f, qY, w.uY[C]);
-          } else {
-            w.aX[C] = fma2(c.two, qX, w.aX[C]);
-            w.aY[C] = fma2(c.two, qY, w.aY[C]);
-            w.t4X[C] = fma2(c.two, qX, w.uX[C]);
-            w.t4Y[C] = fma2(c.two, qY, w.uY[C]);
-          }
+          w.aX[C] = fma2(c.two, qX, w.aX[C]);
+          w.aY[C] = fma2(c.two, qY, w.aY[C]);
+          w.t4X[C] = fma2(c.dtw, qX, w.uX[C]);
+          w.t4Y[C] = fma2(c.dtw, qY, w.uY[C]);
         }
       }
-      // stage 4 at row i - 4K: input t4; u' = u + (q1 + 2 q2 + 2 q3 + q4) / 3, stored at the row
+      // stage 4 at row i - 4K: input t4; u' = u + w dt/6 (q1 + 2 q2 + 2 q3 + q4), stored at the row
       // offset soff (row i - 4K)
       {
         constexpr int C = ((P - 4 * K) % W + W) % W;
@@ -488,8 +460,8 @@ rk4_2d_stream(const Inst2D* __restrict__ insts, const StripItem* __restrict__ it
           float2 qX, qY;
           stream_slope<K, W, C>(w.t4X, w.t4Y, w.pc[C], c, qX, qY);
           float2* const gst = dst0 + soff;
-          const float2 nX = fma2(c.third, add2(w.aX[C], qX), w.uX[C]);
-          const float2 nY = fma2(c.third, add2(w.aY[C], qY), w.uY[C]);
+          const float2 nX = fma2(c.dw6, add2(w.aX[C], qX), w.uX[C]);
+          const float2 nY = fma2(c.dw6, add2(w.aY[C], qY), w.uY[C]);
           if (EVEN) {
             st_pair_if(out0, gst, nX.x, nY.x, nX.y, nY.y);
           } else {

@@ -58,7 +58,7 @@ rk4_2d_wide_reg(const __grid_constant__ Inst2D I, uint4* xbuf, uint32_t tag, int
   const int rx0 = txi * G::TX - H, ry0 = tyi * G::TY - H;   // grid position of region node (0, 0)
   const int gx = rx0 + x0, gy0 = ry0 + y0;
   const bool edge = rx0 < 0 || ry0 < 0 || rx0 + G::RX > n || ry0 + G::RY > n;
-  const RegConst c = reg_const(I.pf);
+  const RegConst c = reg_const<K>(I.pf);
   const float2 c12 = f2(I.pf.c12, I.pf.c12);
   float2* __restrict__ Ug = reinterpret_cast<float2*>(I.u[0]);
   const float* __restrict__ Pg = reinterpret_cast<const float*>(I.P);

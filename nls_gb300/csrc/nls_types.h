@@ -27,6 +27,9 @@ struct Params {
   T c3, c4, c5, c6, c12, c13, c14;   // coefficient slots 3-6 and 12-14
   T half_dt, dt, dt6;                // dt/2, dt, dt/6
   T wc, w1, w2;                      // 2-D cross-stencil weights (centre, distance 1, distance 2)
+  // 2-D in units of the stencil's outermost weight w (1/h^2 or 1/(12 h^2)), in which its weights are
+  // whole numbers: c3 / w .. c6 / w, and the step weights w dt/2, w dt, w dt/6
+  T u3, u4, u5, u6, hw, dtw, dw6;
 };
 
 // Constants of the complex128 right-hand side as float pairs and doubles (f64_node.cuh), in the
@@ -137,6 +140,10 @@ inline Params<T> make_params(const PhysD& ph, double dt, double wc, double w1, d
   p.c12 = (T)ph.c12; p.c13 = (T)ph.c13; p.c14 = (T)ph.c14;
   p.half_dt = (T)(dt * 0.5); p.dt = (T)dt; p.dt6 = (T)(dt / 6.0);
   p.wc = (T)wc; p.w1 = (T)w1; p.w2 = (T)w2;
+  const double w = w2 != 0.0 ? -w2 : w1;
+  const double iw = w != 0.0 ? 1.0 / w : 0.0;
+  p.u3 = (T)(ph.c3 * iw); p.u4 = (T)(ph.c4 * iw); p.u5 = (T)(ph.c5 * iw); p.u6 = (T)(ph.c6 * iw);
+  p.hw = (T)(0.5 * dt * w); p.dtw = (T)(dt * w); p.dw6 = (T)(dt * w / 6.0);
   return p;
 }
 
