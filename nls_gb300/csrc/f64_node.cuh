@@ -269,6 +269,25 @@ NLSG_HD inline bool f2_pump_ok(F2 p) { return p.l == p.l; }
 // (a warp alone on its sub-partition is bound by the latency of that arithmetic, which overlaps
 // only within one block of code), the plain forms only where one of them does not hold.  *P is the
 // pump that p was split from.
+// In two parts: f64_coeffs_2d needs the node alone and gives A and B - centre, f64_slope_2d the rest.
+NLSG_HD inline void f64_coeffs_2d(double ux, double uy, F2 p, bool p_ok, const double* P, const F64Consts& c, double& A,
+                                  double& bw) {
+  double B;
+  if (!f64_coeffs_pairs(ux, uy, p, p_ok, c, A, B)) f64_coeffs_plain(ux, uy, *P, c, A, B);
+  bw = dadd(B, -c.centre);
+}
+template <int K>
+NLSG_HD inline void f64_slope_2d(double ux, double uy, const double (&vx)[4 * K], const double (&vy)[4 * K], double A,
+                                 double bw, const F64Consts& c, double& kx, double& ky) {
+  bool okx, oky;
+  double sx = cross_sum_fixed<K>(vx, c, okx), sy = cross_sum_fixed<K>(vy, c, oky);
+  if (!(okx && oky)) {
+    if (!okx) sx = cross_sum_plain<K>(vx, c);
+    if (!oky) sy = cross_sum_plain<K>(vy, c);
+  }
+  kx = dfma(A, ux, dfma(bw, uy, -sy));
+  ky = dfma(A, uy, dfma(-bw, ux, sx));
+}
 template <int K>
 NLSG_HD inline void f64_slope_2d(double ux, double uy, const double (&vx)[4 * K], const double (&vy)[4 * K],
                                  F2 p, bool p_ok, const double* P, const F64Consts& c, double& kx, double& ky) {
@@ -360,22 +379,22 @@ __device__ __forceinline__ bool f64_coeffs_lanes(double mine, F2 p, bool p_ok, c
   const int other_ok = __shfl_xor_sync(0xffffffffu, (int)ok, 1);
   return ok && other_ok != 0;
 }
-// This lane's part of the slope: v the node, mine its own part, other the other part's neighbours.
+// The two parts of the slope for a lane of a pair: v the node, other the other part's neighbours.
+__device__ __forceinline__ void f64_coeffs_2d_lanes(double2 v, F2 p, bool p_ok, const double* P, const F64Lane& l,
+                                                    const F64Consts& c, double& A, double& bw) {
+  double B;
+  if (!f64_coeffs_lanes(l.part ? v.y : v.x, p, p_ok, l, c, A, B)) f64_coeffs_plain(v.x, v.y, *P, c, A, B);
+  bw = dadd(B, -c.centre);
+}
 template <int K>
-__device__ __forceinline__ double f64_slope_2d_lanes(double2 v, const double (&other)[4 * K], F2 p, bool p_ok, const double* P,
+__device__ __forceinline__ double f64_slope_2d_lanes(double2 v, const double (&other)[4 * K], double A, double bw,
                                                      const F64Lane& l, const F64Consts& c) {
-  const double mine = l.part ? v.y : v.x, his = l.part ? v.x : v.y;
-  double A, B;
   bool oks;
-  const bool ok = f64_coeffs_lanes(mine, p, p_ok, l, c, A, B);
   double s = cross_sum_fixed<K>(other, c, oks);
-  if (!(ok && oks)) {
-    if (!ok) f64_coeffs_plain(v.x, v.y, *P, c, A, B);
-    if (!oks) s = cross_sum_plain<K>(other, c);
-  }
+  if (!oks) s = cross_sum_plain<K>(other, c);
   // k_re = A u_re + m, k_im = A u_im - m with m = (B - centre) times the other part minus S
-  const double m = dfma(dadd(B, -c.centre), his, -s);
-  return dfma(A, mine, l.part ? -m : m);
+  const double m = dfma(bw, l.part ? v.x : v.y, -s);
+  return dfma(A, l.part ? v.y : v.x, l.part ? -m : m);
 }
 template <int K>
 __device__ __forceinline__ double f64_slope_1d_lanes(double2 v, const double (&other)[2 * K + 1],

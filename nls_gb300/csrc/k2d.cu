@@ -1027,16 +1027,22 @@ Wide2DPlan wide_2d_plan(int K, int n, int sms) {
       for (int lanes = 0; lanes < 2; ++lanes) {
         const int per = lanes ? 16 : 32;
         const int ew = (ring + per - 1) / per, iw = (inner + per - 1) / per, total = ew + iw;
-        const double cost = (lanes ? std::max(2800.0 + 40.0 * total, 236.0 * total)
-                                   : std::max(3100.0 + 140.0 * total, 263.0 * total)) +
-                            (gx * gy > 1 ? 100.0 : 0.0) + ring + 0.1 * gx * gy;
+        // warps beyond what a CTA gives the edge take their turn twice; the halo's size stands for
+        // publishing and fetching it
+        const int passes = (ew + (lanes ? 12 : 8) - 1) / (lanes ? 12 : 8);
+        const double cost = (lanes ? std::max(2600.0 + 40.0 * total + 1500.0 * (passes - 1), 236.0 * total)
+                                   : std::max(2900.0 + 140.0 * total + 2500.0 * (passes - 1), 263.0 * total)) +
+                            (gx * gy > 1 ? 100.0 : 0.0) + 3.0 * 2 * K * (w + h) + 0.1 * gx * gy;
         if (cost >= best_cost) continue;
         best_cost = cost;
         best.gx = gx;
         best.gy = gy;
         best.lanes = lanes != 0;
+        // fetching warps: up to four values a lane at a time
+        best.halo_warps = gx * gy > 1 ? std::min(4, (4 * K * (w + h) + 95) / 96) : 0;
         best.edge_warps = std::min(ew, lanes ? 12 : 8);
-        best.threads = 32 * (best.edge_warps + std::min(iw, (lanes ? 32 : 24) - best.edge_warps));
+        best.threads = 32 * (best.halo_warps + best.edge_warps +
+                             std::min(iw, (lanes ? 32 : 24) - best.halo_warps - best.edge_warps));
         best.smem = wide_2d_smem(K, w, h);
       }
     }
@@ -1047,7 +1053,7 @@ size_t wide_2d_slot_bytes(int n) { return (size_t)2 * 2 * n * n * sizeof(uint4);
 
 cudaError_t launch_2d_wide(int K, const Inst2D& I, const Wide2DPlan& p, void* xbuf, uint32_t tag, int* wait_flag,
                            cudaStream_t s) {
-  const Wide2D g{p.gx, p.gy, p.edge_warps};
+  const Wide2D g{p.gx, p.gy, p.halo_warps, p.edge_warps};
   auto go = [&](auto kern) -> cudaError_t {
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kWideSmem);
     if (e != cudaSuccess) return e;

@@ -6,9 +6,10 @@
 // in shared memory for all steps of the launch (72 bytes a node and two halo frames), and after each
 // stage the K outermost rows and columns of every tile pass to its neighbours through tagged slots
 // (exchange.cuh).  FP64 instructions bound the step (f64_node.cuh), so no halo is recomputed; the
-// exchange (540-950 cycles one way) hides behind the interior: the first warps of a CTA own the
-// tile's edge nodes -- they wait for the neighbours' values, evaluate, publish -- and the other
-// warps meanwhile evaluate the nodes that need no neighbour's value.  One CTA barrier a stage.
+// exchange (540-950 cycles one way) hides behind arithmetic: the first warps of a CTA fetch the
+// neighbours' values, the next own the tile's edge nodes -- they evaluate what their nodes need alone
+// (the reservoir and the coefficients) meanwhile, then the rest, and publish -- and the other warps
+// evaluate the nodes that need no neighbour's value.  One CTA barrier a stage.
 // LANES: two adjacent lanes share a node, one for each part, which shortens the chain of a node but
 // repeats the reservoir's quotient and the loop around it; for tiles of few warps, where the chain
 // bounds the stage.
@@ -16,9 +17,9 @@
 
 namespace nlsg {
 
-// Tiles along each axis and warps that own edge nodes.
+// Tiles along each axis, warps that fetch the halo (0: a single tile) and warps that own edge nodes.
 struct Wide2D {
-  int gx, gy, edge_warps;
+  int gx, gy, halo_warps, edge_warps;
 };
 
 template <int K>
@@ -96,8 +97,9 @@ __global__ void __launch_bounds__(LANES ? 1024 : 768) rk4_2d_wide_f64(const __gr
   F2* const P = reinterpret_cast<F2*>(acc + 2 * nodes);       // the pump as pairs
   int2* const hlist = reinterpret_cast<int2*>(P + nodes);     // frame offset, node in the grid (-1: none)
   int* const list = reinterpret_cast<int*>(hlist + T.halo);
-  const int edge_threads = 32 * g.edge_warps;
-  const bool edge = (int)threadIdx.x < edge_threads;
+  const int halo_threads = 32 * g.halo_warps, edge_threads = 32 * g.edge_warps;
+  const int tid = (int)threadIdx.x - halo_threads;   // negative: a fetching thread
+  const bool edge = tid >= 0 && tid < edge_threads;
   const int part = LANES ? threadIdx.x & 1 : 0;
   const F64Lane lane = f64_lane(part, I.f64);
   double* __restrict__ Ug = reinterpret_cast<double*>(I.u[0]);
@@ -113,10 +115,11 @@ __global__ void __launch_bounds__(LANES ? 1024 : 768) rk4_2d_wide_f64(const __gr
   }
   __syncthreads();   // zeroed frames, halo list
   // this thread's (pair's) nodes: list entries first, first + stride, .. below last
-  const int mine = (int)threadIdx.x >> SH, owners = edge_threads >> SH;
+  const int mine = tid >> SH, owners = edge_threads >> SH;
   const int first = edge ? mine : T.ring + mine - owners;
-  const int stride = edge ? owners : (int)(blockDim.x >> SH) - owners, last = edge ? T.ring : nodes;
-  for (int k = first; k < last; k += stride) {
+  const int stride = edge ? owners : ((int)blockDim.x - halo_threads >> SH) - owners;
+  const int last = tid < 0 ? 0 : (edge ? T.ring : nodes);   // a fetching thread owns none
+  for (int k = first; k < last && tid >= 0; k += stride) {
     const int off = T.node(k);
     list[k] = off;
     const size_t q = (size_t)grid_node(off);
@@ -133,36 +136,59 @@ __global__ void __launch_bounds__(LANES ? 1024 : 768) rk4_2d_wide_f64(const __gr
   const uint32_t extra = g_exchange_tag_extra;
   const size_t set_slots = 2 * (size_t)n * n;
   const int64_t steps = I.steps;
+  // exchange number 4 step + s - 1 brings the halo of stage s's input, from the set of its parity
+  if (tid < 0) {
+    for (int64_t step = 0; step < steps; ++step) {
+#pragma unroll 1
+      for (int s = 1; s <= 4; ++s, ++tag) {
+        double* const in = s == 1 ? U : (s == 3 ? T2 : T1);
+        const uint4* const from = xbuf + (size_t)((s - 1) & 1) * set_slots;
+        // element 2 k + part of the halo list
+        for (int k0 = threadIdx.x; k0 < 2 * T.halo; k0 += 4 * halo_threads) {
+          const uint4* want[4];
+          uint64_t got[4];
+          int at[4];
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            const int k = k0 + i * halo_threads;
+            const int2 h = k < 2 * T.halo ? hlist[k >> 1] : make_int2(0, -1);
+            at[i] = 2 * h.x + (k & 1);
+            want[i] = h.y >= 0 ? from + 2 * (size_t)h.y + (k & 1) : nullptr;
+          }
+          x_wait<4>(want, tag + extra, got, wait_flag, dead);
+#pragma unroll
+          for (int i = 0; i < 4; ++i)
+            if (want[i] && !dead) in[at[i]] = x_f64(got[i]);
+        }
+        __syncwarp();
+        asm volatile("barrier.arrive 1, %0;" ::"r"(halo_threads + edge_threads) : "memory");
+        __syncthreads();
+      }
+    }
+    return;
+  }
   for (int64_t step = 0; step < steps; ++step) {
 #pragma unroll 1
     for (int s = 1; s <= 4; ++s, ++tag) {
       double* const in = s == 1 ? U : (s == 3 ? T2 : T1);
       double* const out = s == 4 ? U : (s == 2 ? T2 : T1);
-      // exchange number 4 step + s - 1 brings the halo of this stage's input, into the set of its parity
-      const uint4* const from = xbuf + (size_t)((s - 1) & 1) * set_slots;
       uint4* const to = xbuf + (size_t)(s & 1) * set_slots;
-      if (edge) {
-        for (int k = mine; k < T.halo; k += 2 * owners) {
-          const int2 a = hlist[k];
-          const int2 b = k + owners < T.halo ? hlist[k + owners] : make_int2(0, -1);
-          const uint4* want[2 * PARTS];
-          uint64_t got[2 * PARTS];
-#pragma unroll
-          for (int c = 0; c < PARTS; ++c) {
-            want[c] = a.y >= 0 ? from + 2 * (size_t)a.y + part + c : nullptr;
-            want[PARTS + c] = b.y >= 0 ? from + 2 * (size_t)b.y + part + c : nullptr;
-          }
-          x_wait<2 * PARTS>(want, tag + extra, got, wait_flag, dead);
-#pragma unroll
-          for (int c = 0; c < PARTS; ++c) {
-            if (a.y >= 0 && !dead) in[2 * a.x + part + c] = x_f64(got[c]);
-            if (b.y >= 0 && !dead) in[2 * b.x + part + c] = x_f64(got[PARTS + c]);
-          }
-        }
-        // the lanes of a warp leave the loop at different times: together again before the barrier,
-        // which is the form that does not rely on it
+      // the coefficients of this thread's first node, which need no neighbour (idle lanes repeat one)
+      const bool any = LANES ? first - (mine & 15) < last : first < last;
+      const int k1 = first < last ? first : last - 1;
+      double A1 = 0.0, bw1 = 0.0;
+      auto coeffs = [&](int k, double& A, double& bw) {
+        const int off = list[k];
+        const double2 v = reinterpret_cast<const double2*>(in)[off];
+        const F2 p = P[k];
+        const double* const pg = Pg + grid_node(off);
+        if constexpr (LANES) f64_coeffs_2d_lanes(v, p, f2_pump_ok(p), pg, lane, I.f64, A, bw);
+        else f64_coeffs_2d(v.x, v.y, p, f2_pump_ok(p), pg, I.f64, A, bw);
+      };
+      if (any) coeffs(k1, A1, bw1);
+      if (edge && halo_threads) {
         __syncwarp();
-        asm volatile("barrier.sync 1, %0;" ::"r"(edge_threads) : "memory");
+        asm volatile("barrier.sync 1, %0;" ::"r"(halo_threads + edge_threads) : "memory");
       }
       const bool publish = edge && (s < 4 || step + 1 < steps);
       if constexpr (LANES) {
@@ -181,9 +207,9 @@ __global__ void __launch_bounds__(LANES ? 1024 : 768) rk4_2d_wide_f64(const __gr
             other[4 * d - 1] = o[2 * d * T.pitch];
           }
           const double2 v = *reinterpret_cast<const double2*>(in + 2 * off);
-          const F2 p = P[kk];
+          if (k != first) coeffs(kk, A1, bw1);
           double a = s > 1 ? acc[2 * kk + part] : 0.0;
-          const double q = f64_slope_2d_lanes<K>(v, other, p, f2_pump_ok(p), Pg + grid_node(off), lane, I.f64);
+          const double q = f64_slope_2d_lanes<K>(v, other, A1, bw1, lane, I.f64);
           const double t = f64_stage_lane(s, U[2 * off + part], a, q, I.f64);
           if (live) {
             if (s < 4) acc[2 * kk + part] = a;
@@ -204,8 +230,8 @@ __global__ void __launch_bounds__(LANES ? 1024 : 768) rk4_2d_wide_f64(const __gr
             vy[4 * d - 4] = n0.y; vy[4 * d - 3] = n1.y; vy[4 * d - 2] = n2.y; vy[4 * d - 1] = n3.y;
           }
           double2 q, a = s > 1 ? reinterpret_cast<double2*>(acc)[k] : make_double2(0.0, 0.0);
-          const F2 p = P[k];
-          f64_slope_2d<K>(v.x, v.y, vx, vy, p, f2_pump_ok(p), Pg + grid_node(off), I.f64, q.x, q.y);
+          if (k != first) coeffs(k, A1, bw1);
+          f64_slope_2d<K>(v.x, v.y, vx, vy, A1, bw1, I.f64, q.x, q.y);
           const double2 t = f64_stage(s, reinterpret_cast<double2*>(U)[off], a, q, I.f64);
           if (s < 4) reinterpret_cast<double2*>(acc)[k] = a;
           reinterpret_cast<double2*>(out)[off] = t;

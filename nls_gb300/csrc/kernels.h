@@ -145,7 +145,7 @@ void stream_deps(const std::vector<StripItem>& items, const std::vector<int>& ns
 // One complex128 grid over the whole GPU by a cooperative launch (k2d_wide.cuh).  gx = 0: not for
 // this size.  A launch of steps steps uses 4 steps + 1 tags; xbuf as for launch_1d_wide.
 struct Wide2DPlan {
-  int gx = 0, gy = 0, edge_warps = 0, threads = 0;
+  int gx = 0, gy = 0, halo_warps = 0, edge_warps = 0, threads = 0;
   bool lanes = false;
   size_t smem = 0;
 };
