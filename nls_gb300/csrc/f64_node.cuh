@@ -396,18 +396,39 @@ __device__ __forceinline__ double f64_slope_2d_lanes(double2 v, const double (&o
   const double m = dfma(bw, l.part ? v.x : v.y, -s);
   return dfma(A, l.part ? v.y : v.x, l.part ? -m : m);
 }
-template <int K>
+// between(): FP64 work of the caller that does not depend on this slope, placed like the products.
+template <int K, typename F>
 __device__ __forceinline__ double f64_slope_1d_lanes(double2 v, const double (&other)[2 * K + 1],
                                                      const double (&row)[2 * K + 1], F2 p, double P, bool p_ok,
-                                                     const F64Lane& l, const F64Consts& c) {
+                                                     const F64Lane& l, const F64Consts& c, F&& between) {
   const double mine = l.part ? v.y : v.x, his = l.part ? v.x : v.y;
-  double A, B;
-  const bool ok = f64_coeffs_lanes(mine, p, p_ok, l, c, A, B);
-  double s = dmul(row[0], other[0]);
+  // f64_coeffs_lanes with the operator's products placed where it waits (for the exchange of the
+  // squares, the reciprocal, the exchange of the results): a warp alone on its sub-partition has
+  // nothing else to issue there
+  double s;
+  auto tap = [&](int d) {
+    if (d == 0) asm volatile("mul.rn.f64 %0, %1, %2;" : "=d"(s) : "d"(row[0]), "d"(other[0]));
+    else asm volatile("fma.rn.f64 %0, %1, %2, %0;" : "+d"(s) : "d"(row[d]), "d"(other[d]));
+  };
+  const F2 x = f2_square(f2_split(mine));
+  const F2 o = F2{f64_other(x.h), f64_other(x.l)};
+  tap(0);
+  if (K > 1) tap(1);
+  const F2 q = l.part ? f2_density(o, x) : f2_density(x, o);
+  bool ok;
+  const F2 r = f2_reservoir(p, q, c, ok);
+  if (K > 2) tap(2);
+  tap(K + 1);
+  const F2 w = f2_add(f2_mul(l.alpha, l.part ? q : F2{1.f, 0.f}), f2_mul(l.beta, r));
+  const float aw = w.h < 0.f ? -w.h : w.h;
+  ok = ok && c.fast != 0 && p_ok && f64_in_range(mine) && aw < c.lim;
+  const double val = f2_join(w), hval = f64_other(val);
+  const int other_ok = __shfl_xor_sync(0xffffffffu, (int)ok, 1);
 #pragma unroll
-  for (int d = 1; d <= 2 * K; ++d)
-    if (d != K) s = dfma(row[d], other[d], s);
-  if (!ok) f64_coeffs_plain(v.x, v.y, P, c, A, B);
+  for (int d = K + 2; d <= 2 * K; ++d) tap(d);
+  between();
+  double A = l.part ? hval : val, B = l.part ? val : hval;
+  if (!(ok && other_ok != 0)) f64_coeffs_plain(v.x, v.y, P, c, A, B);
   const double m = dfma(dadd(B, -row[K]), his, -s);
   return dfma(A, mine, l.part ? -m : m);
 }

@@ -125,13 +125,15 @@ __global__ void __launch_bounds__(512) rk4_1d_wide_f64(const __grid_constant__ I
   const uint32_t extra = g_exchange_tag_extra;
   const F64Lane lane = f64_lane(part, I.f64);
   // reads of a stage: both parts of the node, the other part of its neighbours
-  auto slope = [&](const double2* buf) -> double {
+  auto slope = [&](const double2* buf, auto&& between) -> double {
     const double* o = reinterpret_cast<const double*>(buf + li) + (1 - part);
     double other[2 * K + 1];
 #pragma unroll
     for (int d = 0; d < 2 * K + 1; ++d) other[d] = o[2 * (d - K)];
-    return f64_slope_1d_lanes<K>(buf[li], other, nd.row, nd.p, nd.P, nd.p_ok, lane, I.f64);
+    return f64_slope_1d_lanes<K>(buf[li], other, nd.row, nd.p, nd.P, nd.p_ok, lane, I.f64, between);
   };
+  // acc += 2 q of the stage before, while the next stage waits for its exchanges
+  auto twice = [&](double q) { asm volatile("fma.rn.f64 %0, %1, %2, %0;" : "+d"(acc) : "d"(2.0), "d"(q)); };
   auto put = [&](double2* buf, double v) {
     if (in) reinterpret_cast<double*>(buf + li)[part] = v;
     __syncthreads();
@@ -152,16 +154,14 @@ __global__ void __launch_bounds__(512) rk4_1d_wide_f64(const __grid_constant__ I
     const int run = left < g.S ? (int)left : g.S;
     left -= run;
     for (int k = 0; k < run; ++k) {
-      double q = slope(buf0);
-      acc = q;
-      put(buf1, dfma(I.f64.half_dt, q, u));
-      q = slope(buf1);
-      acc = dfma(2.0, q, acc);
-      put(buf0, dfma(I.f64.half_dt, q, u));
-      q = slope(buf0);
-      acc = dfma(2.0, q, acc);
-      put(buf1, dfma(I.f64.dt, q, u));
-      q = slope(buf1);
+      const double q1 = slope(buf0, [] {});
+      acc = q1;
+      put(buf1, dfma(I.f64.half_dt, q1, u));
+      const double q2 = slope(buf1, [] {});
+      put(buf0, dfma(I.f64.half_dt, q2, u));
+      const double q3 = slope(buf0, [&] { twice(q2); });
+      put(buf1, dfma(I.f64.dt, q3, u));
+      const double q = slope(buf1, [&] { twice(q3); });
       u = dfma(I.f64.dt6, dadd(acc, q), u);
       if (k + 1 < run) put(buf0, u);
       else __syncthreads();   // buf1 is read until here, buf0 is written after the next exchange
