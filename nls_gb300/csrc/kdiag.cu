@@ -20,7 +20,8 @@ static constexpr int kDiagThreads = 256;
 static constexpr int kDiagMaxNV = 4;
 static constexpr int kGroup = 16;         // nodes added up in float pairs
 // Grids from which the groups are added up in pairs: their errors, independent of one another, leave
-// 2^-46 / sqrt(groups), below 2^-52 of the sum of the terms' sizes; smaller grids cost FP64 nothing.
+// 2^-46 / sqrt(groups), below 2^-52 of the sum of the terms' sizes.  Smaller grids are added up in
+// FP64, one node a thread: what counts there is the length of a thread's chain.
 static constexpr long long kPairsFrom = 65536;
 
 size_t diag_partials_bytes(long long) { return (size_t)kDiagBlocks * kDiagMaxNV * sizeof(double) + 256; }
@@ -88,7 +89,7 @@ __global__ void __launch_bounds__(kDiagThreads) k_norm_c64(long long n, const fl
       pair_add(s, pair_prod(a[k].x, a[k].x));
       pair_add(s, pair_prod(a[k].y, a[k].y));
     }
-    if (n >= kPairsFrom && pair_range(s.h)) {
+    if (pair_range(s.h)) {
       v[0] += pair_value(s);
     } else {
 #pragma unroll 1
@@ -104,12 +105,13 @@ __global__ void __launch_bounds__(kDiagThreads) k_norm_c64(long long n, const fl
   diag_finish<2>(v, part, out);
 }
 
-__global__ void __launch_bounds__(kDiagThreads) k_norm_c128(long long n, const double2* __restrict__ u,
-                                                            double* __restrict__ part, double* __restrict__ out) {
+template <typename T>
+__global__ void __launch_bounds__(kDiagThreads) k_norm(long long n, const typename C2<T>::type* __restrict__ u,
+                                                       double* __restrict__ part, double* __restrict__ out) {
   double v[2] = {0.0, 0.0};
   int bad = 0;
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-    const double2 a = u[i];
+    const double2 a = make_double2(u[i].x, u[i].y);
     v[0] = dfma(a.x, a.x, dfma(a.y, a.y, v[0]));
     // exponent all ones: infinite or NaN
     bad += ((dhi(a.x) & 0x7ff00000u) == 0x7ff00000u || (dhi(a.y) & 0x7ff00000u) == 0x7ff00000u) ? 1 : 0;
@@ -140,10 +142,11 @@ __global__ void __launch_bounds__(kDiagThreads) k_mu(long long n, const void* __
   diag_finish<3>(v, part, out);
 }
 
-// The same on a square grid with H(u) (order 5) formed on the way: a warp walks kGroup rows of 32
-// columns with the five rows of its column in registers.  complex64: H in single precision as
+// The same on a square grid with H(u) (order 5) formed on the way: a warp walks G rows of 32
+// columns with the five rows of its column in registers (G = kGroup, or 1 without pairs).  complex64: H in single precision as
 // before, the sums in float pairs; complex128: f64_slope_2d and FP64 sums.  Before, H was written
 // and read back by launches of their own and every term added in FP64.
+template <int G>
 __global__ void __launch_bounds__(kDiagThreads) k_mu_2d_c64(int n, const float2* __restrict__ u,
                                                             const float* __restrict__ P, Params<float> prm,
                                                             double* __restrict__ part, double* __restrict__ out) {
@@ -151,10 +154,10 @@ __global__ void __launch_bounds__(kDiagThreads) k_mu_2d_c64(int n, const float2*
   const Phys<float> ph = phys_of<float>(prm);
   const int lane = threadIdx.x & 31;
   const int cols = (n + 31) / 32;
-  const long long tiles = (long long)cols * ((n + kGroup - 1) / kGroup);
+  const long long tiles = (long long)cols * ((n + G - 1) / G);
   const int warps = blockDim.x >> 5;
   for (long long t = (long long)blockIdx.x * warps + (threadIdx.x >> 5); t < tiles; t += (long long)gridDim.x * warps) {
-    const int x = (int)(t % cols) * 32 + lane, y0 = (int)(t / cols) * kGroup;
+    const int x = (int)(t % cols) * 32 + lane, y0 = (int)(t / cols) * G;
     if (x >= n) continue;
     auto at = [&](int xx, int y) -> float2 {
       return xx >= 0 && xx < n && y >= 0 && y < n ? u[(size_t)y * n + xx] : make_float2(0.f, 0.f);
@@ -171,7 +174,7 @@ __global__ void __launch_bounds__(kDiagThreads) k_mu_2d_c64(int n, const float2*
     for (int k = 0; k < 4; ++k) w[k] = at(x, y0 - 2 + k);
     F2 re = {0.f, 0.f}, im = {0.f, 0.f}, m = {0.f, 0.f};
 #pragma unroll
-    for (int j = 0; j < kGroup; ++j) {
+    for (int j = 0; j < G; ++j) {
       const int y = y0 + j;
       w[(j + 4) % 5] = at(x, y + 2);
       const float2 c = w[(j + 2) % 5];
@@ -187,13 +190,13 @@ __global__ void __launch_bounds__(kDiagThreads) k_mu_2d_c64(int n, const float2*
         pair_add(m, pair_prod(c.y, c.y));
       }
     }
-    if ((long long)n * n >= kPairsFrom && pair_range(m.h) && fabsf(re.h) < 0x1p100f && fabsf(im.h) < 0x1p100f) {
+    if (G > 1 && pair_range(m.h) && fabsf(re.h) < 0x1p100f && fabsf(im.h) < 0x1p100f) {
       v[0] += pair_value(re);
       v[1] += pair_value(im);
       v[2] += pair_value(m);
     } else {
 #pragma unroll 1
-      for (int y = y0; y < y0 + kGroup && y < n; ++y) {
+      for (int y = y0; y < y0 + G && y < n; ++y) {
         const float2 c = at(x, y);
         const float2 h = slope(c, sum4(at(x - 1, y), at(x + 1, y), at(x, y - 1), at(x, y + 1)),
                                sum4(at(x - 2, y), at(x + 2, y), at(x, y - 2), at(x, y + 2)), P[(size_t)y * n + x]);
@@ -325,7 +328,7 @@ __global__ void __launch_bounds__(kDiagThreads) k_damping_2d_c64(long long n, co
       const F2 t = f2_mul(r, d);
       pair_add(s, t);
     }
-    if (ok && n >= kPairsFrom && pair_range(m.h) && fabsf(s.h) < 0x1p100f) {
+    if (ok && pair_range(m.h) && fabsf(s.h) < 0x1p100f) {
       v[0] += pair_value(s);
     } else {
 #pragma unroll 1
@@ -345,7 +348,8 @@ static int blocks_for(long long n) {
 }
 
 cudaError_t diag_norm(int dtype, long long n, const void* u, double* part, double* out, cudaStream_t st) {
-  if (dtype == NLS_C128) k_norm_c128<<<blocks_for(n), kDiagThreads, 0, st>>>(n, (const double2*)u, part, out);
+  if (dtype == NLS_C128) k_norm<double><<<blocks_for(n), kDiagThreads, 0, st>>>(n, (const double2*)u, part, out);
+  else if (n < kPairsFrom) k_norm<float><<<blocks_for(n), kDiagThreads, 0, st>>>(n, (const float2*)u, part, out);
   else k_norm_c64<<<blocks_for((n + kGroup - 1) / kGroup), kDiagThreads, 0, st>>>(n, (const float2*)u, part, out);
   return cudaGetLastError();
 }
@@ -360,14 +364,14 @@ cudaError_t diag_mu(int dtype, long long n, const void* u, const void* v, int mo
 
 cudaError_t diag_mu_2d(int dtype, int n, const void* u, const void* P, const PhysD& ph, const Stencil2D& op,
                        double* part, double* out, cudaStream_t st) {
-  const long long rows = dtype == NLS_C128 ? n : (n + kGroup - 1) / kGroup;
-  const int nb = blocks_for(rows * ((n + 31) / 32) * 32);
+  const int rows = dtype == NLS_C128 || (long long)n * n < kPairsFrom ? 1 : kGroup;   // of a warp at a time
+  const int nb = blocks_for((long long)((n + rows - 1) / rows) * ((n + 31) / 32) * 32);
   if (dtype == NLS_C128)
     // (a step so small that the pairs' limit on dt |a| does not bind)
     k_mu_2d_c128<<<nb, kDiagThreads, 0, st>>>(n, (const double2*)u, (const double*)P, make_f64(ph, 0x1p-60, op), part, out);
   else
-    k_mu_2d_c64<<<nb, kDiagThreads, 0, st>>>(n, (const float2*)u, (const float*)P,
-                                             make_params<float>(ph, 0.0, op.center, op.w[0], op.w[1]), part, out);
+    (rows == 1 ? k_mu_2d_c64<1> : k_mu_2d_c64<kGroup>)<<<nb, kDiagThreads, 0, st>>>(
+        n, (const float2*)u, (const float*)P, make_params<float>(ph, 0.0, op.center, op.w[0], op.w[1]), part, out);
   return cudaGetLastError();
 }
 
@@ -377,7 +381,7 @@ cudaError_t diag_damping(int dtype, long long n, const void* u, const void* P, i
   const int nb = blocks_for(n);
   if (dtype == NLS_C128) {
     k_damping<double><<<nb, kDiagThreads, 0, st>>>(n, u, P, radial, r_step, dx, c12, c13, c14, part, out);
-  } else if (radial) {
+  } else if (radial || n < kPairsFrom) {
     k_damping<float><<<nb, kDiagThreads, 0, st>>>(n, u, P, radial, r_step, dx, c12, c13, c14, part, out);
   } else {
     PhysD ph = {};
