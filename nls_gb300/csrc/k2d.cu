@@ -9,8 +9,6 @@
 // tile list may span many independent solves (batched and served forms), each with its own size,
 // coefficients and ping-pong buffers; the persistent grid strides over the list.
 //
-// rk4_2d_wide_f64 (k2d_wide.cuh): a single complex128 grid held on chip by all SMs.
-//
 // rk4_2d_stage: one RK4 stage from global memory (no halo recomputation), used where tiles would
 // be too small to amortise their halo (double precision on modest grids) and as the general path.
 #include <cuda.h>
@@ -224,9 +222,6 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity) {
 
 #include "k2d_reg.cuh"
 #include "k2d_stream.cuh"
-#include "exchange.cuh"
-#include "k2d_wide.cuh"
-#include "k2d_wide_reg.cuh"
 
 namespace nlsg {
 
@@ -1005,116 +1000,6 @@ void stream_sort_items(std::vector<StripItem>& items) {
   std::stable_sort(items.begin(), items.end(), [](const StripItem& a, const StripItem& b) {
     return (a.y1 - a.y0) > (b.y1 - b.y0);
   });
-}
-
-// ---- one complex128 grid over the whole GPU (k2d_wide.cuh)
-
-static constexpr size_t kWideSmem = 227 * 1024;
-
-// The tiling with the shortest stage by a model in cycles fitted to measured stages (order 3): one
-// lane a node 3240 at one warp a CTA (40^2), 3830 at 4 (128^2), 4960 at 14 (256^2), 14 230 at 54
-// (512^2); two lanes a node 2900 at 1, 3120 at 8, 6600 at 28 warps (the same grids).  So two lanes
-// up to about 300 nodes a CTA, one beyond, and above 1800 nodes a CTA the stage kernels, whose
-// launches amortise there (600^2: 40.2 us a step against 41.1 here; 512^2: 30.3 against 27.8).
-Wide2DPlan wide_2d_plan(int K, int n, int sms) {
-  Wide2DPlan best;
-  double best_cost = 1e300;
-  for (int gx = 1; gx <= std::min(sms, n); ++gx)
-    for (int gy = 1; gx * gy <= sms && gy <= n; ++gy) {
-      const int w = (n + gx - 1) / gx, h = (n + gy - 1) / gy;
-      if (w * h > 1800 || wide_2d_smem(K, w, h) > kWideSmem) continue;
-      const int inner = w > 2 * K && h > 2 * K ? (w - 2 * K) * (h - 2 * K) : 0, ring = w * h - inner;
-      for (int lanes = 0; lanes < 2; ++lanes) {
-        const int per = lanes ? 16 : 32;
-        const int ew = (ring + per - 1) / per, iw = (inner + per - 1) / per, total = ew + iw;
-        // warps beyond what a CTA gives the edge take their turn twice; the halo's size stands for
-        // publishing and fetching it
-        const int passes = (ew + (lanes ? 12 : 8) - 1) / (lanes ? 12 : 8);
-        const double cost = (lanes ? std::max(2600.0 + 40.0 * total + 1500.0 * (passes - 1), 236.0 * total)
-                                   : std::max(2900.0 + 140.0 * total + 2500.0 * (passes - 1), 263.0 * total)) +
-                            (gx * gy > 1 ? 100.0 : 0.0) + 3.0 * 2 * K * (w + h) + 0.1 * gx * gy;
-        if (cost >= best_cost) continue;
-        best_cost = cost;
-        best.gx = gx;
-        best.gy = gy;
-        best.lanes = lanes != 0;
-        // fetching warps: up to four values a lane at a time
-        best.halo_warps = gx * gy > 1 ? std::min(4, (4 * K * (w + h) + 95) / 96) : 0;
-        best.edge_warps = std::min(ew, lanes ? 12 : 8);
-        best.threads = 32 * (best.halo_warps + best.edge_warps +
-                             std::min(iw, (lanes ? 32 : 24) - best.halo_warps - best.edge_warps));
-        best.smem = wide_2d_smem(K, w, h);
-      }
-    }
-  return best;
-}
-
-size_t wide_2d_slot_bytes(int n) { return (size_t)2 * 2 * n * n * sizeof(uint4); }
-
-cudaError_t launch_2d_wide(int K, const Inst2D& I, const Wide2DPlan& p, void* xbuf, uint32_t tag, int* wait_flag,
-                           cudaStream_t s) {
-  const Wide2D g{p.gx, p.gy, p.halo_warps, p.edge_warps};
-  auto go = [&](auto kern) -> cudaError_t {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kWideSmem);
-    if (e != cudaSuccess) return e;
-    return launch_coop(kern, dim3(p.gx * p.gy), dim3(p.threads), p.smem, s, I, g, (uint4*)xbuf, tag, wait_flag);
-  };
-  if (K == 1) return p.lanes ? go(rk4_2d_wide_f64<1, true>) : go(rk4_2d_wide_f64<1, false>);
-  if (K == 2) return p.lanes ? go(rk4_2d_wide_f64<2, true>) : go(rk4_2d_wide_f64<2, false>);
-  return cudaErrorInvalidValue;
-}
-
-// ---- one complex64 grid over the whole GPU (k2d_wide_reg.cuh)
-
-// Calls f(kernel, config) for the region of shape `shape` (rows 16, 32, 64, 96).
-template <typename F>
-static cudaError_t wide_reg_shape(int K, int shape, F&& f) {
-#define NLSG_WIDE_REG(NW, NJ)                                                                    if (K == 1) return f(rk4_2d_wide_reg<1, NW, NJ>, WideRegCfg<1, NW, NJ>());                     if (K == 2) return f(rk4_2d_wide_reg<2, NW, NJ>, WideRegCfg<2, NW, NJ>());
-  switch (shape) {
-    case 0: if (K == 1) return f(rk4_2d_wide_reg<1, 8, 2>, WideRegCfg<1, 8, 2>()); break;
-    case 1: NLSG_WIDE_REG(8, 4) break;
-    case 2: NLSG_WIDE_REG(16, 4) break;
-    case 3: NLSG_WIDE_REG(12, 8) break;
-  }
-#undef NLSG_WIDE_REG
-  return cudaErrorInvalidValue;
-}
-
-// The lowest region whose tiles all fit: fewer rows a warp, shorter stages.  us a step, order 3, by
-// rows of the region (16 / 32 / 64): 128^2 2.05 / 2.59 / 3.65, 256^2 - / 2.58 / 3.74; streaming 9.3
-// and 9.4.  96 rows as 12 warps of 8 (6.40 at 777^2) rather than 8 of 12 (6.68).  Beyond one tile an
-// SM (840 a side at order 3, 720 at order 5) the streaming and tile kernels; the largest here against
-// those: 840^2 6.35 and 11.6, order 5 700^2 9.03 and 9.83.
-WideReg2DPlan wide_reg_2d_plan(int K, int n, int sms) {
-  WideReg2DPlan best;
-  for (int shape = K == 1 ? 0 : 1; shape <= 3 && !best.tiles; ++shape) {
-    wide_reg_shape(K, shape, [&](auto, auto cfg) {
-      typedef typename decltype(cfg)::G G;
-      const int tx = (n + G::TX - 1) / G::TX, ty = (n + G::TY - 1) / G::TY;
-      if (tx * ty > sms) return cudaSuccess;
-      best.shape = shape;
-      best.tiles_x = tx;
-      best.tiles = tx * ty;
-      return cudaSuccess;
-    });
-  }
-  return best;
-}
-
-size_t wide_reg_2d_slot_bytes(int n) { return (size_t)2 * n * n * sizeof(uint4); }
-
-cudaError_t launch_2d_wide_reg(int K, const Inst2D& I, const WideReg2DPlan& p, void* xbuf, uint32_t tag, int* wait_flag,
-                               cudaStream_t s) {
-  return wide_reg_shape(K, p.shape, [&](auto kern, auto cfg) -> cudaError_t {
-    typedef decltype(cfg) C;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::SMEM);
-    if (e != cudaSuccess) return e;
-    return launch_coop(kern, dim3(p.tiles), dim3(C::G::NT), C::SMEM, s, I, (uint4*)xbuf, tag, wait_flag);
-  });
-}
-
-cudaError_t exchange_tag_extra_set_2d(unsigned extra) {
-  return cudaMemcpyToSymbol(g_exchange_tag_extra, &extra, sizeof(extra));
 }
 
 // Rows of 32 nodes per CTA of the stage kernels.  Two (64-thread CTAs) spread a small grid evenly

@@ -14,6 +14,8 @@
 // (540-950 cycles one way) a step.
 #pragma once
 
+#include "k2d_reg_stage.cuh"
+
 namespace nlsg {
 
 template <int K, int NW, int NJ>
@@ -47,7 +49,7 @@ __global__ void __launch_bounds__(NW * 32, 1)
 rk4_2d_wide_reg(const __grid_constant__ Inst2D I, uint4* xbuf, uint32_t tag, int* wait_flag) {
   typedef WideRegCfg<K, NW, NJ> C;
   typedef RegCfg<K, NW, NJ> G;
-  constexpr int H = G::H, BATCH = 5;
+  constexpr int H = G::H, NH = (C::HALO + G::NT - 1) / G::NT;   // halo nodes a thread fetches
   extern __shared__ __align__(128) unsigned char smem_raw[];
   float4* const exch = reinterpret_cast<float4*>(smem_raw);
   float2* const hbuf = reinterpret_cast<float2*>(smem_raw + G::EXCH);
@@ -82,6 +84,17 @@ rk4_2d_wide_reg(const __grid_constant__ Inst2D I, uint4* xbuf, uint32_t tag, int
     out |= (unsigned)o << j;
     frame |= (unsigned)(o && (x0 < 2 * H || x0 >= G::RX - 2 * H || y < 2 * H || y >= G::RY - 2 * H)) << j;
   }
+  // the nodes this thread fetches (-1: none, or outside the grid)
+  int fetch[NH];
+#pragma unroll
+  for (int i = 0; i < NH; ++i) {
+    const int k = threadIdx.x + i * G::NT;
+    int x = 0, y = 0;
+    C::node(k < C::HALO ? k : 0, x, y);
+    x += rx0;
+    y += ry0;
+    fetch[i] = k < C::HALO && x >= 0 && x < n && y >= 0 && y < n ? y * n + x : -1;
+  }
   bool dead = false;
   const uint32_t extra = g_exchange_tag_extra;
   const size_t set_slots = (size_t)n * n;
@@ -96,25 +109,18 @@ rk4_2d_wide_reg(const __grid_constant__ Inst2D I, uint4* xbuf, uint32_t tag, int
         if ((dom1 >> j) & 1u) x_put(s + 1, x_pack(f2(uX[j].y, uY[j].y)), tag);
       }
     __syncwarp();   // no lane waits before every lane of its warp has published
-    for (int k0 = threadIdx.x; k0 < C::HALO; k0 += BATCH * G::NT) {
-      const uint4* want[BATCH];
-      uint64_t got[BATCH];
+    const uint4* want[NH];
+    uint64_t got[NH];
 #pragma unroll
-      for (int i = 0; i < BATCH; ++i) {
-        const int k = k0 + i * G::NT;
-        int x = 0, y = 0;
-        C::node(k < C::HALO ? k : 0, x, y);
-        x += rx0;
-        y += ry0;
-        want[i] = k < C::HALO && x >= 0 && x < n && y >= 0 && y < n ? slots + (size_t)y * n + x : nullptr;
-        got[i] = 0;
-      }
-      x_wait<BATCH>(want, tag + extra, got, wait_flag, dead);
+    for (int i = 0; i < NH; ++i) {
+      want[i] = fetch[i] >= 0 ? slots + fetch[i] : nullptr;
+      got[i] = 0;   // outside the grid: zero
+    }
+    x_wait<NH>(want, tag + extra, got, wait_flag, dead);
 #pragma unroll
-      for (int i = 0; i < BATCH; ++i) {
-        const int k = k0 + i * G::NT;
-        if (k < C::HALO) hbuf[k] = want[i] ? x_c64(got[i]) : f2(0.f, 0.f);
-      }
+    for (int i = 0; i < NH; ++i) {
+      const int k = threadIdx.x + i * G::NT;
+      if (k < C::HALO) hbuf[k] = x_c64(got[i]);
     }
     __syncthreads();
 #pragma unroll
