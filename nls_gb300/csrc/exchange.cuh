@@ -12,7 +12,8 @@
 // symmetric: two CTAs exchange when one's nodes lie within the halo width of the other's).
 //
 // All CTAs of the launch are resident together (cooperative launch), so every wait ends; each is
-// bounded all the same (about a second).  One that expires sets the context's status word; waits
+// bounded all the same: about a second, and several for a launch's first exchange, which also waits
+// for CTAs that another stream's kernel still keeps from starting.  One that expires sets the context's status word; waits
 // that see it set, or that belong to a thread that has given up, end at once, the kernel runs to
 // its end on whatever values it has and the host reports the timeout.
 #pragma once
@@ -36,13 +37,14 @@ __device__ __forceinline__ void x_get(const uint4* slot, uint64_t& data, uint32_
   tag = (uint32_t)(top >> 32);
 }
 
-// Bound of a wait: polls of about 600 cycles each.
-constexpr unsigned kExchangePolls = 1u << 21;
+// Bounds of a wait: polls of about 600 cycles each.
+constexpr unsigned kExchangePolls = 1u << 21, kExchangeFirstPolls = 1u << 23;
 
-// Waits for the N slots (null: none) to carry `tag` and reads their payloads.
+// Waits for the N slots (null: none) to carry `tag` and reads their payloads; gives up after limit
+// polls.
 template <int N>
 __device__ __forceinline__ void x_wait(const uint4* const (&slot)[N], uint32_t tag, uint64_t (&data)[N],
-                                       int* wait_flag, bool& dead) {
+                                       unsigned limit, int* wait_flag, bool& dead) {
   for (unsigned polls = 0; !dead; ++polls) {
     uint32_t got[N];
     bool all = true;
@@ -52,7 +54,7 @@ __device__ __forceinline__ void x_wait(const uint4* const (&slot)[N], uint32_t t
 #pragma unroll
     for (int i = 0; i < N; ++i) all = all && (!slot[i] || got[i] == tag);
     if (all) return;
-    if (polls >= kExchangePolls) {
+    if (polls >= limit) {
       atomicExch(wait_flag, 1);
       dead = true;
     } else if ((polls & 255u) == 255u && *reinterpret_cast<volatile int*>(wait_flag) != 0) {

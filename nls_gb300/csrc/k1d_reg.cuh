@@ -129,7 +129,7 @@ __device__ __forceinline__ Reg1DEx reg1d_exchange(float2* ex, int warp, int lane
 // by shuffle, across a warp boundary from the neighbouring warp's published end nodes (stage
 // parity double-buffers them, so one CTA barrier per stage suffices), zero beyond the CTA.  Without
 // branches: every lane reads a neighbour's end and selects (branches cost a lone warp a quarter of a
-// stage: 8192 nodes on one warp per sub-partition ran at 930 cycles a stage, 250 of them resolving).
+// stage: 4096 nodes on one CTA ran at 930 cycles a stage, 250 of them resolving).
 template <int K, int NPT, int S>
 __device__ __forceinline__ void reg1d_halo(const float2 (&t)[NPT], float2 (&L)[K], float2 (&R)[K], const Reg1DEx& e,
                                            int lane) {

@@ -18,7 +18,9 @@ static constexpr size_t kWideSmem = 227 * 1024;
 // lane a node 3240 at one warp a CTA (40^2), 3830 at 4 (128^2), 4960 at 14 (256^2), 14 230 at 54
 // (512^2); two lanes a node 2900 at 1, 3120 at 8, 6600 at 28 warps (the same grids).  So two lanes
 // up to about 300 nodes a CTA, one beyond, and above 1800 nodes a CTA the stage kernels, whose
-// launches amortise there (600^2: 40.2 us a step against 41.1 here; 512^2: 30.3 against 27.8).
+// launches amortise there (600^2: 40.2 us a step against 41.1 here; 512^2: 30.3 against 27.8).  The
+// stages above are those of warps that fetched their own halo; with fetching warps 40^2 takes 5.2 us a
+// step, 128^2 5.7, 256^2 9.8 (stage kernels 8.5, 9.1 and 13.6).
 Wide2DPlan wide_2d_plan(int K, int n, int sms) {
   Wide2DPlan best;
   double best_cost = 1e300;

@@ -1,7 +1,7 @@
 // k2d_wide_reg.cuh -- one complex64 square grid held in registers by all SMs (sm_103a).
 //
 // The streaming step walks each strip of a grid row by row: a chain of rows that a small or middling
-// grid has too few strips to hide (777^2: 12 us a step, a quarter of the rate of 4096^2; 128^2: 5 us),
+// grid has too few strips to hide (777^2: 12.1 us a step, a quarter of the rate of 4096^2; 128^2: 9.2 us),
 // and one launch a step.  Here every CTA of a cooperative launch keeps one register tile
 // (k2d_reg.cuh) for all steps of the launch.  It evaluates its output tile and a halo of H = 4K nodes
 // around it, so the four stages of a step need CTA barriers only; then the tiles exchange the frames
@@ -11,7 +11,8 @@
 //
 // The arithmetic is reg_stage's, which agrees bit for bit with the streaming kernel's.  What bounds it:
 // the stages' arithmetic over the region (latency at 2-4 warps a scheduler), then one exchange
-// (540-950 cycles one way) a step.
+// (540-950 cycles one way) a step.  Measured, order 3: 128^2 2.1 us a step, 777^2 6.0 (1442 warp
+// instructions a step, issue slots 44 % busy).
 #pragma once
 
 #include "k2d_reg_stage.cuh"
@@ -116,7 +117,7 @@ rk4_2d_wide_reg(const __grid_constant__ Inst2D I, uint4* xbuf, uint32_t tag, int
       want[i] = fetch[i] >= 0 ? slots + fetch[i] : nullptr;
       got[i] = 0;   // outside the grid: zero
     }
-    x_wait<NH>(want, tag + extra, got, wait_flag, dead);
+    x_wait<NH>(want, tag + extra, got, step == 0 ? kExchangeFirstPolls : kExchangePolls, wait_flag, dead);
 #pragma unroll
     for (int i = 0; i < NH; ++i) {
       const int k = threadIdx.x + i * G::NT;

@@ -209,13 +209,11 @@ static cudaError_t replay(nls_ctx* ctx, int64_t reps, F&& body) {
 
 // ------------------------------------------------------------------ single solves
 
-// Exchange slots of at least `bytes` and the first of `count` tags no earlier launch on them used.
-static cudaError_t exchange_slots(nls_ctx* ctx, size_t bytes, int64_t count, uint32_t* first) {
-  const bool grow = bytes > ctx->xbuf.bytes;
-  cudaError_t e = ctx->xbuf.ensure(bytes);
-  if (e != cudaSuccess) return e;
-  if (grow || (int64_t)ctx->xtag + count >= (int64_t)0x7fffffff) {
-    if ((e = cudaMemsetAsync(ctx->xbuf.p, 0, ctx->xbuf.bytes, ctx->stream)) != cudaSuccess) return e;
+// First of `count` tags that no earlier launch on the exchange slots used.
+static cudaError_t exchange_tags(nls_ctx* ctx, int64_t count, uint32_t* first) {
+  if ((int64_t)ctx->xtag + count >= (int64_t)0x7fffffff) {
+    cudaError_t e = cudaMemsetAsync(ctx->xbuf.p, 0, ctx->xbuf.bytes, ctx->stream);
+    if (e != cudaSuccess) return e;
     ctx->xtag = 0;
   }
   *first = ctx->xtag + 1;
@@ -225,6 +223,42 @@ static cudaError_t exchange_slots(nls_ctx* ctx, size_t bytes, int64_t count, uin
 
 // RK4 steps per cooperative launch (bounds a launch to well under a second).
 static constexpr int64_t kCoopStepsPerLaunch = 16384;
+
+// Advances one solve by cooperative launches of up to kCoopStepsPerLaunch steps: launch(steps, tag)
+// enqueues one, using tags(steps) tags.  false: not possible here -- no memory for the slots, a grid
+// that cannot be resident on the SMs this process may use, or a stream under capture, whose replays
+// would use the same tags again -- and nothing was enqueued; the other kernels take the solve.
+template <typename Tags, typename Launch>
+static bool solve_coop(nls_ctx* ctx, int64_t iters, size_t slot_bytes, Tags&& tags, Launch&& launch, int* status) {
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(ctx->stream, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) {
+    cudaGetLastError();
+    return false;
+  }
+  *status = NLS_OK;
+  cudaError_t e = cudaSuccess;
+  if (slot_bytes > ctx->xbuf.bytes) {
+    if (ctx->xbuf.ensure(slot_bytes) != cudaSuccess) {
+      cudaGetLastError();
+      return false;
+    }
+    e = cudaMemsetAsync(ctx->xbuf.p, 0, ctx->xbuf.bytes, ctx->stream);
+    ctx->xtag = 0;
+  }
+  for (int64_t done = 0, steps; done < iters && e == cudaSuccess; done += steps) {
+    steps = std::min(kCoopStepsPerLaunch, iters - done);
+    uint32_t tag;
+    if ((e = exchange_tags(ctx, tags(steps), &tag)) != cudaSuccess) break;
+    e = launch(steps, tag);
+    if (e == cudaErrorCooperativeLaunchTooLarge && done == 0) {
+      cudaGetLastError();
+      return false;
+    }
+    if (e == cudaSuccess) ctx->launches += 1;
+  }
+  if (e != cudaSuccess) *status = fail_cuda(ctx, e, "cooperative launch");
+  return true;
+}
 
 static int solve_1d_dev(nls_ctx* ctx, int dtype, const nls_problem* pr, int64_t iters,
                         const void* P, void* u) {
@@ -245,16 +279,14 @@ static int solve_1d_dev(nls_ctx* ctx, int dtype, const nls_problem* pr, int64_t 
     // would take computes with other roundings (complex64 on more than 8 CTAs).
     const Wide1DPlan plan = pr->variant == -1 && (dtype == NLS_C128 || cl <= 8)
                                 ? wide_1d_plan(dtype, op.K, n, ctx->sm_count) : Wide1DPlan();
-    if (plan.grid) {
-      for (int64_t done = 0; done < iters; done += I.steps) {
-        I.steps = std::min(kCoopStepsPerLaunch, iters - done);
-        uint32_t tag;
-        CK(ctx, exchange_slots(ctx, wide_1d_slot_bytes(dtype, n), (I.steps + plan.S - 1) / plan.S, &tag));
-        CK(ctx, launch_1d_wide(dtype, op.K, I, plan, ctx->xbuf.p, tag, ctx->wait_flag, ctx->stream));
-        ctx->launches += 1;
-      }
-      return NLS_OK;
-    }
+    if (plan.grid && solve_coop(ctx, iters, wide_1d_slot_bytes(dtype, n),
+                                [&](int64_t steps) { return (steps + plan.S - 1) / plan.S; },
+                                [&](int64_t steps, uint32_t tag) {
+                                  I.steps = steps;
+                                  return launch_1d_wide(dtype, op.K, I, plan, ctx->xbuf.p, tag, ctx->wait_flag, ctx->stream);
+                                }, &st))
+      return st;
+    I.steps = iters;
     CK(ctx, ctx->desc.ensure(sizeof(Inst1D)));
     CK(ctx, cudaMemcpyAsync(ctx->desc.p, &I, sizeof(I), cudaMemcpyHostToDevice, ctx->stream));
     const int seg = (n + cl - 1) / cl;
@@ -436,14 +468,13 @@ static int solve_2d_dev(nls_ctx* ctx, int dtype, const nls_problem* pr, int64_t 
       std::memset(&I, 0, sizeof(I));
       I.u[0] = u; I.P = P; I.n = n; I.dt = pr->dt; I.ph = ph; I.op = op;
       set_params(I);
-      for (int64_t done = 0; done < iters; done += I.steps) {
-        I.steps = std::min(kCoopStepsPerLaunch, iters - done);
-        uint32_t tag;
-        CK(ctx, exchange_slots(ctx, wide_2d_slot_bytes(n), 4 * I.steps + 1, &tag));
-        CK(ctx, launch_2d_wide(op.K, I, plan, ctx->xbuf.p, tag, ctx->wait_flag, ctx->stream));
-        ctx->launches += 1;
-      }
-      return NLS_OK;
+      int st = NLS_OK;
+      if (solve_coop(ctx, iters, wide_2d_slot_bytes(n), [](int64_t steps) { return 4 * steps + 1; },
+                     [&](int64_t steps, uint32_t tag) {
+                       I.steps = steps;
+                       return launch_2d_wide(op.K, I, plan, ctx->xbuf.p, tag, ctx->wait_flag, ctx->stream);
+                     }, &st))
+        return st;
     }
     CK(ctx, ctx->scratch.ensure(3 * cb));
     char* base = (char*)ctx->scratch.p;
@@ -472,14 +503,13 @@ static int solve_2d_dev(nls_ctx* ctx, int dtype, const nls_problem* pr, int64_t 
     std::memset(&I, 0, sizeof(I));
     I.u[0] = u; I.P = P; I.n = n; I.tiles_x = plan.tiles_x; I.dt = pr->dt; I.ph = ph; I.op = op;
     set_params(I);
-    for (int64_t done = 0; done < iters; done += I.steps) {
-      I.steps = std::min(kCoopStepsPerLaunch, iters - done);
-      uint32_t tag;
-      CK(ctx, exchange_slots(ctx, wide_reg_2d_slot_bytes(n), I.steps, &tag));
-      CK(ctx, launch_2d_wide_reg(op.K, I, plan, ctx->xbuf.p, tag, ctx->wait_flag, ctx->stream));
-      ctx->launches += 1;
-    }
-    return NLS_OK;
+    int st = NLS_OK;
+    if (solve_coop(ctx, iters, wide_reg_2d_slot_bytes(n), [](int64_t steps) { return steps; },
+                   [&](int64_t steps, uint32_t tag) {
+                     I.steps = steps;
+                     return launch_2d_wide_reg(op.K, I, plan, ctx->xbuf.p, tag, ctx->wait_flag, ctx->stream);
+                   }, &st))
+      return st;
   }
   if (shape == TILE_STREAM) return solve_2d_stream(ctx, pr, op, ph, iters, P, u);
   // fused: ping-pong between the caller's buffer and one scratch buffer
