@@ -33,8 +33,8 @@ static bool radial_taps(int order, int* K, const int** d1, const int** d2, int* 
   return false;
 }
 
-// Dense-row form: A(p, q) for |q - p| <= K; returns 0 or a status.
-static int radial_rows(int n, int order, double h, std::vector<double>& rows /* n x (2K+1) */,
+// Dense-row form: A(p, q) for |q - p| <= K of the first `count` rows; returns 0 or a status.
+static int radial_rows(int n, int count, int order, double h, std::vector<double>& rows /* count x (2K+1) */,
                        double* w1_out, double* w2_out) {
   int K, den1, den2;
   const int *t1, *t2;
@@ -46,9 +46,9 @@ static int radial_rows(int n, int order, double h, std::vector<double>& rows /* 
   if (w1_out) std::memcpy(w1_out, w1, sizeof(double) * (2 * K + 1));
   if (w2_out) std::memcpy(w2_out, w2, sizeof(double) * (2 * K + 1));
   const int W = 2 * K + 1;
-  rows.assign((size_t)n * W, 0.0);
+  rows.assign((size_t)count * W, 0.0);
   std::vector<double> a1(W), a2(W);
-  for (int p = 0; p < n; ++p) {
+  for (int p = 0; p < count; ++p) {
     std::fill(a1.begin(), a1.end(), 0.0);
     std::fill(a2.begin(), a2.end(), 0.0);
     for (int d = -K; d <= K; ++d) {
@@ -70,7 +70,7 @@ static int radial_rows(int n, int order, double h, std::vector<double>& rows /* 
 
 int host_make_laplacian(int n, int order, double h, double* op) {
   std::vector<double> rows;
-  int st = radial_rows(n, order, h, rows, nullptr, nullptr);
+  int st = radial_rows(n, n, order, h, rows, nullptr, nullptr);
   if (st) return st;
   const int K = (order - 1) / 2, W = 2 * K + 1;
   // band storage: op(K + p - q, q) = A(p, q), column-major (order, n)
@@ -87,7 +87,8 @@ int host_make_laplacian(int n, int order, double h, double* op) {
 int host_stencil_1d(int n, int order, double h, Stencil1D* s) {
   std::vector<double> rows;
   std::memset(s, 0, sizeof(*s));
-  int st = radial_rows(n, order, h, rows, s->w1, s->w2);
+  // the near-axis rows only (at most 3; a grid has at least order rows)
+  int st = radial_rows(n, n < 3 ? n : 3, order, h, rows, s->w1, s->w2);
   if (st) return st;
   s->order = order;
   s->K = (order - 1) / 2;
