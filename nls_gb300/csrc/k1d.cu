@@ -644,7 +644,7 @@ static size_t wide_smem(int dtype, int K, int threads) {
 // four stages (longer when an SM's sub-partitions hold several warps) plus the exchange over the S
 // steps between two.  Constants from the measured instruction rates: a complex128 stage of one warp
 // per sub-partition has 550 to 900 cycles (orders 3 to 7) of FP64 instructions, which add up with more
-// warps; a complex64 one is latency (180 cycles the shortest chain, 430 measured at order 5), of which
+// warps; a complex64 one is latency (180 cycles the shortest chain, 350 measured at order 5), of which
 // more warps fill a part.  Only the ratios decide: among equal CTAs the largest S that fits the GPU wins.  Grids that fit one CTA,
 // or too large for all CTAs to be resident, stay on the kernels of one CTA or cluster.
 Wide1DPlan wide_1d_plan(int dtype, int K, int n, int sms) {

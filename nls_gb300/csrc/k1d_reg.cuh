@@ -38,16 +38,26 @@ __device__ __forceinline__ Reg1DConst<K> reg1d_const(const Inst1D& I) {
   return c;
 }
 
+// The part of a node's slope that needs no neighbour: a and b of q = (a - i b) u + i L u, with
+// r = c12 P / (c13 + c14 |u|^2), a = c3 r - c4, b = c5 |u|^2 + c6 r.
+template <int K>
+__device__ __forceinline__ float2 reg1d_point(float2 v, float pc, const Reg1DConst<K>& c) {
+  const float sq = __fmaf_rn(v.x, v.x, v.y * v.y);
+  const float r = pc * rcp_approx(__fmaf_rn(c.c14, sq, c.c13));
+  return f2(__fmaf_rn(c.c3, r, c.nc4), __fmaf_rn(c.c5, sq, c.c6 * r));
+}
+
 // One RK4 stage S over the thread's NPT nodes.  t holds the stage input (re, im per node); on
 // return it holds the next stage's input (S < 4), or u the new state (S = 4).  L / R: the K nodes
 // before the thread's first and after its last node.  Nodes at or beyond n stay zero.  NEAR: the
 // warp holds the nodes at the axis (a warp-uniform choice; within it every lane evaluates both
-// forms of its first K nodes and thread 0 takes the near-axis rows).
+// forms of its first K nodes and thread 0 takes the near-axis rows).  ab: the nodes' reg1d_point, or
+// null to evaluate it here.
 template <int K, int NPT, int S, bool NEAR>
 __device__ __forceinline__ void reg1d_stage_form(float2 (&t)[NPT], float2 (&acc)[NPT], float2 (&u)[NPT],
                                                  const float (&pc)[NPT], const float (&ir)[NPT],
                                                  const float2 (&L)[K], const float2 (&R)[K], int p0, int n,
-                                                 const Reg1DConst<K>& c) {
+                                                 const Reg1DConst<K>& c, const float2* ab) {
   auto at = [&](int idx) -> float2 { return idx < 0 ? L[K + idx] : (idx >= NPT ? R[idx - NPT] : t[idx]); };
   float2 nt[NPT];
 #pragma unroll
@@ -72,12 +82,10 @@ __device__ __forceinline__ void reg1d_stage_form(float2 (&t)[NPT], float2 (&acc)
       for (int d = 1; d <= 2 * K; ++d) ln = fma2(c.near[i < K ? i : 0][d], at(i - K + d), ln);
       lu = f2(p0 == 0 ? ln.x : lu.x, p0 == 0 ? ln.y : lu.y);
     }
-    // q = (a - i b) u + i L u, r = c12 P / (c13 + c14 |u|^2), a = c3 r - c4, b = c5 |u|^2 + c6 r
+    // q = (a - i b) u + i L u
     const float2 v = t[i];
-    const float sq = __fmaf_rn(v.x, v.x, v.y * v.y);
-    const float r = pc[i] * rcp_approx(__fmaf_rn(c.c14, sq, c.c13));
-    const float a = __fmaf_rn(c.c3, r, c.nc4);
-    const float b = __fmaf_rn(c.c5, sq, c.c6 * r);
+    const float2 w_ab = ab ? ab[i] : reg1d_point<K>(v, pc[i], c);
+    const float a = w_ab.x, b = w_ab.y;
     const float2 q = f2(__fmaf_rn(a, v.x, __fmaf_rn(b, v.y, -lu.y)), __fmaf_rn(a, v.y, __fmaf_rn(-b, v.x, lu.x)));
     if (S == 1) acc[i] = q;
     else if (S == 4) acc[i] = add2(acc[i], q);
@@ -100,9 +108,9 @@ template <int K, int NPT, int S>
 __device__ __forceinline__ void reg1d_stage(float2 (&t)[NPT], float2 (&acc)[NPT], float2 (&u)[NPT],
                                             const float (&pc)[NPT], const float (&ir)[NPT],
                                             const float2 (&L)[K], const float2 (&R)[K], int p0, bool near, int n,
-                                            const Reg1DConst<K>& c) {
-  if (near) reg1d_stage_form<K, NPT, S, true>(t, acc, u, pc, ir, L, R, p0, n, c);
-  else reg1d_stage_form<K, NPT, S, false>(t, acc, u, pc, ir, L, R, p0, n, c);
+                                            const Reg1DConst<K>& c, const float2* ab = nullptr) {
+  if (near) reg1d_stage_form<K, NPT, S, true>(t, acc, u, pc, ir, L, R, p0, n, c, ab);
+  else reg1d_stage_form<K, NPT, S, false>(t, acc, u, pc, ir, L, R, p0, n, c, ab);
 }
 
 // Exchange of warp-end nodes within a CTA: [2 parities][nw + 2 warps][2 ends][K] values in shared

@@ -10,14 +10,14 @@
 // starts with an exchange, so a CTA reads and writes only its own segment of the state in global
 // memory and the update in place is safe.
 //
-// What bounds it: complex64, the latency of four dependent stages (about 430 cycles each at order 5)
+// What bounds it: complex64, the latency of four dependent stages (about 350 cycles each at order 5)
 // and the exchange, 540-950 cycles over S steps; complex128, the chain of a stage and the FP64
 // instructions of one warp per sub-partition (f64_node.cuh) -- so there two lanes share a node, one
 // for the real and one for the imaginary part, which halves them: 227 warp instructions and 1250
 // cycles a stage at order 5, the FP64 pipe 43 % busy.
 //
 // Measured, us a step, one CTA or cluster before and this kernel: complex64 order 5, 4096 nodes 4.64
-// and 0.86; complex128 order 5, 1000 nodes 5.3 and 2.5; order 7, 2501 nodes 8.5 and 3.0.
+// and 0.70; complex128 order 5, 1000 nodes 5.3 and 2.5; order 7, 2501 nodes 8.5 and 3.0.
 #pragma once
 
 namespace nlsg {
@@ -26,6 +26,39 @@ namespace nlsg {
 struct Wide1D {
   int seg, S;
 };
+
+// reg1d_halo and reg1d_stage in one: a warp alone on its sub-partition evaluates what its nodes need
+// alone between publishing its ends and the CTA barrier, where the two calls leave it to wait (order 5,
+// 4096 nodes: 0.86 -> 0.70 us a step; orders 3 and 7 the same).  Waiting for the neighbouring warps
+// alone, through tagged slots of shared memory, took 1.1: the polls cost more than the barrier.
+template <int K, int NPT, int S>
+__device__ __forceinline__ void wide_1d_stage(float2 (&t)[NPT], float2 (&acc)[NPT], float2 (&u)[NPT],
+                                              const float (&pc)[NPT], const float (&ir)[NPT], int p0, bool near, int n,
+                                              const Reg1DConst<K>& c, const Reg1DEx& e, int lane) {
+  const int off = (S & 1) ? e.parity : 0;
+  const bool first = lane == 0, lastl = lane == 31;
+  if (first || lastl) {
+#pragma unroll
+    for (int k = 0; k < K; ++k)
+      e.mine[off + k] = f2(lastl ? t[NPT - K + k].x : t[k].x, lastl ? t[NPT - K + k].y : t[k].y);
+  }
+  float2 L[K], R[K], ab[NPT];
+#pragma unroll
+  for (int k = 0; k < K; ++k) {
+    L[k] = f2(__shfl_up_sync(0xffffffffu, t[NPT - K + k].x, 1), __shfl_up_sync(0xffffffffu, t[NPT - K + k].y, 1));
+    R[k] = f2(__shfl_down_sync(0xffffffffu, t[k].x, 1), __shfl_down_sync(0xffffffffu, t[k].y, 1));
+  }
+#pragma unroll
+  for (int i = 0; i < NPT; ++i) ab[i] = reg1d_point<K>(t[i], pc[i], c);
+  __syncthreads();
+#pragma unroll
+  for (int k = 0; k < K; ++k) {
+    const float2 v = e.nb[off + k];
+    L[k] = f2(first ? v.x : L[k].x, first ? v.y : L[k].y);
+    R[k] = f2(lastl ? v.x : R[k].x, lastl ? v.y : R[k].y);
+  }
+  reg1d_stage<K, NPT, S>(t, acc, u, pc, ir, L, R, p0, near, n, c, ab);
+}
 
 template <int K, int NPT>
 __global__ void __launch_bounds__(256) rk4_1d_wide(const __grid_constant__ Inst1D I, Wide1D g, uint4* xbuf,
@@ -60,7 +93,6 @@ __global__ void __launch_bounds__(256) rk4_1d_wide(const __grid_constant__ Inst1
     edge[i] = own && ((q0 > 0 && p < q0 + H) || (q1 < n && p >= q1 - H));
     any_halo = any_halo || halo[i];
   }
-  float2 L[K], R[K];
   bool dead = false;
   const uint32_t extra = g_exchange_tag_extra;
   int set = 0;
@@ -85,14 +117,10 @@ __global__ void __launch_bounds__(256) rk4_1d_wide(const __grid_constant__ Inst1
     for (int k = 0; k < run; ++k) {
 #pragma unroll
       for (int i = 0; i < NPT; ++i) t[i] = u[i];
-      reg1d_halo<K, NPT, 1>(t, L, R, e, lane);
-      reg1d_stage<K, NPT, 1>(t, acc, u, pc, ir, L, R, p0, near, hi, c);
-      reg1d_halo<K, NPT, 2>(t, L, R, e, lane);
-      reg1d_stage<K, NPT, 2>(t, acc, u, pc, ir, L, R, p0, near, hi, c);
-      reg1d_halo<K, NPT, 3>(t, L, R, e, lane);
-      reg1d_stage<K, NPT, 3>(t, acc, u, pc, ir, L, R, p0, near, hi, c);
-      reg1d_halo<K, NPT, 4>(t, L, R, e, lane);
-      reg1d_stage<K, NPT, 4>(t, acc, u, pc, ir, L, R, p0, near, hi, c);
+      wide_1d_stage<K, NPT, 1>(t, acc, u, pc, ir, p0, near, hi, c, e, lane);
+      wide_1d_stage<K, NPT, 2>(t, acc, u, pc, ir, p0, near, hi, c, e, lane);
+      wide_1d_stage<K, NPT, 3>(t, acc, u, pc, ir, p0, near, hi, c, e, lane);
+      wide_1d_stage<K, NPT, 4>(t, acc, u, pc, ir, p0, near, hi, c, e, lane);
     }
   }
 #pragma unroll

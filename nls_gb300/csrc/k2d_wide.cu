@@ -98,7 +98,7 @@ static bool wide_reg_shape(int K, int shape, F&& f) {
 // order 3; 96 as 16 of 6 takes 5.7).  us a step, order 3, by rows of the region (16 / 24 / 32): 64^2
 // 1.99 / 2.09 / 2.32, 128^2 2.07 / 2.28 / 2.58; 512^2 3.14 with 48 rows, 3.78 with 64; streaming 8.7 to
 // 9.3.  Beyond one tile an SM (840 a side at order 3, 720 at order 5) the streaming and tile kernels;
-// the largest here against those: 840^2 6.1 and 11.1, order 5 700^2 7.5 and 9.5.
+// the largest here against those: 840^2 5.5 and 11.1, order 5 700^2 7.5 and 9.5.
 WideReg2DPlan wide_reg_2d_plan(int K, int n, int sms) {
   WideReg2DPlan best;
   bool more = true;
