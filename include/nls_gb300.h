@@ -45,7 +45,7 @@ typedef struct nls_pool nls_pool;
 
 /* One solve: dim 1 is the radial 1-D model of solve_nls (nls/nls.f90:797-813), dim 2 the
  * Cartesian model of solve_nls_2d (nls/nls.f90:903-919).  variant selects a kernel shape chosen by
- * the autotuner (-1 = built-in choice): 1-D = CTAs per solve (cluster size 1..16; complex64 runs
+ * the autotuner (-1 = built-in choice; a single solve then may spread over the whole GPU): 1-D = CTAs per solve (cluster size 1..16; complex64 runs
  * the register-resident kernel on 1 CTA and its cluster form on 2..8 CTAs whenever each segment
  * holds at least 4K nodes; 0 = unfused stage kernels); 2-D = 0 unfused, or a fused tile region (threads): 1 = 64x64 (512),
  * 2 = 128x32 (512), 3 = 32x32 (256), 4 = 64x64 (1024), 5 = 128x32 (1024),
