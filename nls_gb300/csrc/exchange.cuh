@@ -12,10 +12,14 @@
 // symmetric: two CTAs exchange when one's nodes lie within the halo width of the other's).
 //
 // All CTAs of the launch are resident together (cooperative launch), so every wait ends; each is
-// bounded all the same: about a second, and several for a launch's first exchange, which also waits
-// for CTAs that another stream's kernel still keeps from starting.  One that expires sets the context's status word; waits
-// that see it set, or that belong to a thread that has given up, end at once, the kernel runs to
-// its end on whatever values it has and the host reports the timeout.
+// bounded all the same, by two to three seconds.  CTAs do not wait for one another to start: beside
+// a kernel of another stream that held 24 SMs for longer than that bound, grids that need those SMs
+// started when it had ended (144 and 150 CTAs; a grid that fits beside it ran at once), and of two
+// contexts' cooperative grids the second starts after the first.
+// A wait that expires sets the context's status word; waits that see it set, or that belong to a
+// thread that has given up, end at once.  The values a thread gave up on are NaN from then on, and
+// NaN spreads with the stencil as the values would have, so a node of the final state is either
+// right or NaN, and the host reports the timeout.
 #pragma once
 
 #include <stdint.h>
@@ -37,14 +41,17 @@ __device__ __forceinline__ void x_get(const uint4* slot, uint64_t& data, uint32_
   tag = (uint32_t)(top >> 32);
 }
 
-// Bounds of a wait: polls of about 600 cycles each.
-constexpr unsigned kExchangePolls = 1u << 21, kExchangeFirstPolls = 1u << 23;
+// Bound of a wait: polls of about 600 cycles each.
+constexpr unsigned kExchangePolls = 1u << 23;
 
-// Waits for the N slots (null: none) to carry `tag` and reads their payloads; gives up after limit
-// polls.
+// A NaN as a double and in both parts of a complex64 payload.
+constexpr uint64_t kExchangeNaN = ~0ull;
+
+// Waits for the N slots (null: none) to carry `tag` and reads their payloads.  dead: given up, now
+// or earlier; the payloads are then NaN.
 template <int N>
 __device__ __forceinline__ void x_wait(const uint4* const (&slot)[N], uint32_t tag, uint64_t (&data)[N],
-                                       unsigned limit, int* wait_flag, bool& dead) {
+                                       int* wait_flag, bool& dead) {
   for (unsigned polls = 0; !dead; ++polls) {
     uint32_t got[N];
     bool all = true;
@@ -54,13 +61,16 @@ __device__ __forceinline__ void x_wait(const uint4* const (&slot)[N], uint32_t t
 #pragma unroll
     for (int i = 0; i < N; ++i) all = all && (!slot[i] || got[i] == tag);
     if (all) return;
-    if (polls >= limit) {
+    if (polls >= kExchangePolls) {
       atomicExch(wait_flag, 1);
       dead = true;
     } else if ((polls & 255u) == 255u && *reinterpret_cast<volatile int*>(wait_flag) != 0) {
       dead = true;
     }
   }
+#pragma unroll
+  for (int i = 0; i < N; ++i)
+    if (slot[i]) data[i] = kExchangeNaN;
 }
 
 __device__ __forceinline__ uint64_t x_pack(float2 v) {

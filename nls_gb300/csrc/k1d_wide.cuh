@@ -107,10 +107,10 @@ __global__ void __launch_bounds__(256) rk4_1d_wide(const __grid_constant__ Inst1
       uint64_t got[NPT];
 #pragma unroll
       for (int i = 0; i < NPT; ++i) want[i] = halo[i] ? slots + p0 + i : nullptr;
-      x_wait<NPT>(want, tag + extra, got, left == I.steps ? kExchangeFirstPolls : kExchangePolls, wait_flag, dead);
+      x_wait<NPT>(want, tag + extra, got, wait_flag, dead);
 #pragma unroll
       for (int i = 0; i < NPT; ++i)
-        if (halo[i] && !dead) u[i] = x_c64(got[i]);
+        if (halo[i]) u[i] = x_c64(got[i]);
     }
     const int run = left < g.S ? (int)left : g.S;
     left -= run;
@@ -179,8 +179,8 @@ __global__ void __launch_bounds__(512) rk4_1d_wide_f64(const __grid_constant__ I
     if (halo) {
       const uint4* want[1] = {slots + 2 * (size_t)p + part};
       uint64_t got[1];
-      x_wait<1>(want, tag + extra, got, left == I.steps ? kExchangeFirstPolls : kExchangePolls, wait_flag, dead);
-      if (!dead) u = x_f64(got[0]);
+      x_wait<1>(want, tag + extra, got, wait_flag, dead);
+      u = x_f64(got[0]);
     }
     put(buf0, u);
     const int run = left < g.S ? (int)left : g.S;

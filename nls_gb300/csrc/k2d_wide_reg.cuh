@@ -117,7 +117,7 @@ rk4_2d_wide_reg(const __grid_constant__ Inst2D I, uint4* xbuf, uint32_t tag, int
       want[i] = fetch[i] >= 0 ? slots + fetch[i] : nullptr;
       got[i] = 0;   // outside the grid: zero
     }
-    x_wait<NH>(want, tag + extra, got, step == 0 ? kExchangeFirstPolls : kExchangePolls, wait_flag, dead);
+    x_wait<NH>(want, tag + extra, got, wait_flag, dead);
 #pragma unroll
     for (int i = 0; i < NH; ++i) {
       const int k = threadIdx.x + i * G::NT;
