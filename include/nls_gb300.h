@@ -29,7 +29,9 @@ extern "C" {
 #define NLS_ERR_ORDER 2       /* unsupported stencil order (1-D: 3, 5, 7; 2-D: 3, 5) */
 #define NLS_ERR_CUDA 3        /* CUDA runtime error; nls_last_error() has the text */
 #define NLS_ERR_NONFINITE 4   /* NaN or Inf found in a result by the FP64 diagnostics */
-#define NLS_ERR_TIMEOUT 5     /* a bounded wait expired */
+#define NLS_ERR_TIMEOUT 5     /* a bounded wait inside a kernel expired: the state of a solve since the last
+                               * report is not valid; from the calls that block (synchronize, host-buffer
+                               * solves, diagnostics, pool) */
 #define NLS_ERR_NOMEM 6       /* device memory exhausted */
 #define NLS_ERR_BUSY 7        /* serving pool: no slot or admission budget for this request now */
 #define NLS_ERR_NOT_READY 8   /* serving pool: nothing finished yet */
@@ -264,8 +266,8 @@ int nls_test_set_stream_steps_per_launch(int mode);
 
 /* No counterpart in the reference.  Test control of the failure path of the bounded waits of the
  * solves spread over the whole GPU: with extra > 0 every wait for another CTA's values on `device`
- * asks for a tag that far ahead of the one published, so it gives up after its bound (about a
- * second), sets the context's status word, and the synchronising call returns NLS_ERR_TIMEOUT; 0
+ * asks for a tag that far ahead of the one published, so it gives up after its bound (two to
+ * three seconds), sets the context's status word, and the synchronising call returns NLS_ERR_TIMEOUT; 0
  * restores normal operation.  No fault is raised and the context stays usable.  Not for production
  * use. */
 int nls_test_set_exchange_tag_extra(int device, unsigned extra);

@@ -17,7 +17,7 @@ namespace nlsg {
 
 static constexpr int kDiagBlocks = 1216;  // 8 x 152 SMs
 static constexpr int kDiagThreads = 256;
-static constexpr int kDiagMaxNV = 4;
+static constexpr int kDiagMaxNV = kDiagStatus;
 static constexpr int kGroup = 16;         // nodes added up in float pairs
 // Grids from which the groups are added up in pairs: their errors, independent of one another, leave
 // 2^-46 / sqrt(groups), below 2^-52 of the sum of the terms' sizes.  Smaller grids are added up in
@@ -30,10 +30,12 @@ __device__ __forceinline__ double weight(int mode, long long i, double dx) {
   return mode == 1 ? (double)i * dx : 1.0;
 }
 
-// Block sums to part; the last block of the launch adds all blocks' and writes out.  The word after
-// the partials counts finished blocks; it starts at zero and is left at zero.
+// Block sums to part; the last block of the launch adds all blocks' and writes out, and after the sums
+// the context's status word, so that the host learns with them whether the state can be trusted.  The
+// word after the partials counts finished blocks; it starts at zero and is left at zero.
 template <int NV>
-__device__ __forceinline__ void diag_finish(double (&v)[NV], double* __restrict__ part, double* __restrict__ out) {
+__device__ __forceinline__ void diag_finish(double (&v)[NV], const DiagOut& d) {
+  double* const part = d.partials;
   __shared__ double sm[32 * NV];
   __shared__ bool last;
   block_sum<NV>(v, sm);
@@ -53,9 +55,11 @@ __device__ __forceinline__ void diag_finish(double (&v)[NV], double* __restrict_
 #pragma unroll
     for (int k = 0; k < NV; ++k) v[k] += __ldcg(part + b * NV + k);
   block_sum<NV>(v, sm);
-  if (threadIdx.x == 0)
+  if (threadIdx.x == 0) {
 #pragma unroll
-    for (int k = 0; k < NV; ++k) out[k] = v[k];
+    for (int k = 0; k < NV; ++k) d.out[k] = v[k];
+    d.out[kDiagStatus] = (double)*reinterpret_cast<const volatile int*>(d.wait_flag);
+  }
 }
 
 // acc += t, the error of the high sum kept in the low one.
@@ -76,7 +80,7 @@ __device__ __forceinline__ bool pair_range(float sum_sq) { return sum_sq >= 0x1p
 __device__ __forceinline__ double pair_value(F2 a) { return f2_join(f2_sum(a.h, a.l)); }
 
 __global__ void __launch_bounds__(kDiagThreads) k_norm_c64(long long n, const float2* __restrict__ u,
-                                                           double* __restrict__ part, double* __restrict__ out) {
+                                                           DiagOut out) {
   double v[2] = {0.0, 0.0};
   const long long stride = (long long)gridDim.x * blockDim.x;
   for (long long i0 = (long long)blockIdx.x * blockDim.x + threadIdx.x; i0 < n; i0 += kGroup * stride) {
@@ -102,12 +106,12 @@ __global__ void __launch_bounds__(kDiagThreads) k_norm_c64(long long n, const fl
       }
     }
   }
-  diag_finish<2>(v, part, out);
+  diag_finish<2>(v, out);
 }
 
 template <typename T>
 __global__ void __launch_bounds__(kDiagThreads) k_norm(long long n, const typename C2<T>::type* __restrict__ u,
-                                                       double* __restrict__ part, double* __restrict__ out) {
+                                                       DiagOut out) {
   double v[2] = {0.0, 0.0};
   int bad = 0;
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
@@ -117,14 +121,14 @@ __global__ void __launch_bounds__(kDiagThreads) k_norm(long long n, const typena
     bad += ((dhi(a.x) & 0x7ff00000u) == 0x7ff00000u || (dhi(a.y) & 0x7ff00000u) == 0x7ff00000u) ? 1 : 0;
   }
   v[1] = (double)bad;
-  diag_finish<2>(v, part, out);
+  diag_finish<2>(v, out);
 }
 
 // Sums of conj(u) H(u) and |u|^2 over one array pair (the radial grids, weighted by r).
 template <typename T>
 __global__ void __launch_bounds__(kDiagThreads) k_mu(long long n, const void* __restrict__ u_,
                                                      const void* __restrict__ h_, int mode, double dx,
-                                                     double* __restrict__ part, double* __restrict__ out) {
+                                                     DiagOut out) {
   typedef typename C2<T>::type C;
   const C* u = reinterpret_cast<const C*>(u_);
   const C* hv = reinterpret_cast<const C*>(h_);
@@ -139,7 +143,7 @@ __global__ void __launch_bounds__(kDiagThreads) k_mu(long long n, const void* __
     v[1] += w * (ax * by - ay * bx);
     v[2] += w * (ax * ax + ay * ay);
   }
-  diag_finish<3>(v, part, out);
+  diag_finish<3>(v, out);
 }
 
 // The same on a square grid with H(u) (order 5) formed on the way: a warp walks G rows of 32
@@ -149,7 +153,7 @@ __global__ void __launch_bounds__(kDiagThreads) k_mu(long long n, const void* __
 template <int G>
 __global__ void __launch_bounds__(kDiagThreads) k_mu_2d_c64(int n, const float2* __restrict__ u,
                                                             const float* __restrict__ P, Params<float> prm,
-                                                            double* __restrict__ part, double* __restrict__ out) {
+                                                            DiagOut out) {
   double v[3] = {0.0, 0.0, 0.0};
   const Phys<float> ph = phys_of<float>(prm);
   const int lane = threadIdx.x & 31;
@@ -207,12 +211,12 @@ __global__ void __launch_bounds__(kDiagThreads) k_mu_2d_c64(int n, const float2*
       }
     }
   }
-  diag_finish<3>(v, part, out);
+  diag_finish<3>(v, out);
 }
 
 __global__ void __launch_bounds__(kDiagThreads) k_mu_2d_c128(int n, const double2* __restrict__ u,
                                                              const double* __restrict__ P, F64Consts c,
-                                                             double* __restrict__ part, double* __restrict__ out) {
+                                                             DiagOut out) {
   double v[3] = {0.0, 0.0, 0.0};
   const int cols = (n + 31) / 32, lane = threadIdx.x & 31, warps = blockDim.x >> 5;
   const long long tiles = (long long)cols * n;
@@ -241,7 +245,7 @@ __global__ void __launch_bounds__(kDiagThreads) k_mu_2d_c128(int n, const double
     v[1] = dfma(a.x, hy, dfma(-a.y, hx, v[1]));
     v[2] = dfma(a.x, a.x, dfma(a.y, a.y, v[2]));
   }
-  diag_finish<3>(v, part, out);
+  diag_finish<3>(v, out);
 }
 
 template <typename T>
@@ -249,7 +253,7 @@ __global__ void __launch_bounds__(kDiagThreads) k_relerr(long long n, const void
                                                          const double2* __restrict__ b,
                                                          const double* __restrict__ P, double c12,
                                                          double c13, double c14,
-                                                         double* __restrict__ part, double* __restrict__ out) {
+                                                         DiagOut out) {
   typedef typename C2<T>::type C;
   const C* a = reinterpret_cast<const C*>(a_);
   double v[4] = {0.0, 0.0, 0.0, 0.0};
@@ -266,7 +270,7 @@ __global__ void __launch_bounds__(kDiagThreads) k_relerr(long long n, const void
     v[2] += (na - nb) * (na - nb);
     v[3] += nb * nb;
   }
-  diag_finish<4>(v, part, out);
+  diag_finish<4>(v, out);
 }
 
 // Damping integral of Solution.getDampingIntegral (nls/model.py:350-365): the rectangle rule of
@@ -282,8 +286,7 @@ template <typename T>
 __global__ void __launch_bounds__(kDiagThreads) k_damping(long long n, const void* __restrict__ u_,
                                                           const void* __restrict__ P_, int radial,
                                                           double r_step, double dx, double c12, double c13,
-                                                          double c14, double* __restrict__ part,
-                                                          double* __restrict__ out) {
+                                                          double c14, DiagOut out) {
   typedef typename C2<T>::type C;
   const C* u = reinterpret_cast<const C*>(u_);
   const T* P = reinterpret_cast<const T*>(P_);
@@ -294,13 +297,13 @@ __global__ void __launch_bounds__(kDiagThreads) k_damping(long long n, const voi
     const double w = radial ? two_pi * ((double)i * r_step) * dx : dx * dx;
     v[0] += damping_term<T>(u[i], P[i], c12, c13, c14) * w;
   }
-  diag_finish<1>(v, part, out);
+  diag_finish<1>(v, out);
 }
 // complex64 on a square grid: groups in float pairs, the reservoir as in the complex128 steps.
 __global__ void __launch_bounds__(kDiagThreads) k_damping_2d_c64(long long n, const float2* __restrict__ u,
                                                                  const float* __restrict__ P, double dx, F64Consts c,
                                                                  double c12, double c13, double c14,
-                                                                 double* __restrict__ part, double* __restrict__ out) {
+                                                                 DiagOut out) {
   double v[1] = {0.0};
   const long long stride = (long long)gridDim.x * blockDim.x;
   // c12 / (c13 + c14 d): the pump's constant is not folded into the pair of P (exact as it is)
@@ -339,7 +342,7 @@ __global__ void __launch_bounds__(kDiagThreads) k_damping_2d_c64(long long n, co
     }
   }
   v[0] *= dx * dx;
-  diag_finish<1>(v, part, out);
+  diag_finish<1>(v, out);
 }
 
 static int blocks_for(long long n) {
@@ -347,42 +350,41 @@ static int blocks_for(long long n) {
   return (int)std::max<long long>(1, std::min<long long>(b, kDiagBlocks));
 }
 
-cudaError_t diag_norm(int dtype, long long n, const void* u, double* part, double* out, cudaStream_t st) {
-  if (dtype == NLS_C128) k_norm<double><<<blocks_for(n), kDiagThreads, 0, st>>>(n, (const double2*)u, part, out);
-  else if (n < kPairsFrom) k_norm<float><<<blocks_for(n), kDiagThreads, 0, st>>>(n, (const float2*)u, part, out);
-  else k_norm_c64<<<blocks_for((n + kGroup - 1) / kGroup), kDiagThreads, 0, st>>>(n, (const float2*)u, part, out);
+cudaError_t diag_norm(int dtype, long long n, const void* u, const DiagOut& out, cudaStream_t st) {
+  if (dtype == NLS_C128) k_norm<double><<<blocks_for(n), kDiagThreads, 0, st>>>(n, (const double2*)u, out);
+  else if (n < kPairsFrom) k_norm<float><<<blocks_for(n), kDiagThreads, 0, st>>>(n, (const float2*)u, out);
+  else k_norm_c64<<<blocks_for((n + kGroup - 1) / kGroup), kDiagThreads, 0, st>>>(n, (const float2*)u, out);
   return cudaGetLastError();
 }
 
 cudaError_t diag_mu(int dtype, long long n, const void* u, const void* v, int mode, double dx,
-                    double* part, double* out, cudaStream_t st) {
+                    const DiagOut& out, cudaStream_t st) {
   const int nb = blocks_for(n);
-  if (dtype == NLS_C128) k_mu<double><<<nb, kDiagThreads, 0, st>>>(n, u, v, mode, dx, part, out);
-  else k_mu<float><<<nb, kDiagThreads, 0, st>>>(n, u, v, mode, dx, part, out);
+  if (dtype == NLS_C128) k_mu<double><<<nb, kDiagThreads, 0, st>>>(n, u, v, mode, dx, out);
+  else k_mu<float><<<nb, kDiagThreads, 0, st>>>(n, u, v, mode, dx, out);
   return cudaGetLastError();
 }
 
 cudaError_t diag_mu_2d(int dtype, int n, const void* u, const void* P, const PhysD& ph, const Stencil2D& op,
-                       double* part, double* out, cudaStream_t st) {
+                       const DiagOut& out, cudaStream_t st) {
   const int rows = dtype == NLS_C128 || (long long)n * n < kPairsFrom ? 1 : kGroup;   // of a warp at a time
   const int nb = blocks_for((long long)((n + rows - 1) / rows) * ((n + 31) / 32) * 32);
   if (dtype == NLS_C128)
     // (a step so small that the pairs' limit on dt |a| does not bind)
-    k_mu_2d_c128<<<nb, kDiagThreads, 0, st>>>(n, (const double2*)u, (const double*)P, make_f64(ph, 0x1p-60, op), part, out);
+    k_mu_2d_c128<<<nb, kDiagThreads, 0, st>>>(n, (const double2*)u, (const double*)P, make_f64(ph, 0x1p-60, op), out);
   else
     (rows == 1 ? k_mu_2d_c64<1> : k_mu_2d_c64<kGroup>)<<<nb, kDiagThreads, 0, st>>>(
-        n, (const float2*)u, (const float*)P, make_params<float>(ph, 0.0, op.center, op.w[0], op.w[1]), part, out);
+        n, (const float2*)u, (const float*)P, make_params<float>(ph, 0.0, op.center, op.w[0], op.w[1]), out);
   return cudaGetLastError();
 }
 
 cudaError_t diag_damping(int dtype, long long n, const void* u, const void* P, int radial, double r_step,
-                         double dx, double c12, double c13, double c14, double* part, double* out,
-                         cudaStream_t st) {
+                         double dx, double c12, double c13, double c14, const DiagOut& out, cudaStream_t st) {
   const int nb = blocks_for(n);
   if (dtype == NLS_C128) {
-    k_damping<double><<<nb, kDiagThreads, 0, st>>>(n, u, P, radial, r_step, dx, c12, c13, c14, part, out);
+    k_damping<double><<<nb, kDiagThreads, 0, st>>>(n, u, P, radial, r_step, dx, c12, c13, c14, out);
   } else if (radial || n < kPairsFrom) {
-    k_damping<float><<<nb, kDiagThreads, 0, st>>>(n, u, P, radial, r_step, dx, c12, c13, c14, part, out);
+    k_damping<float><<<nb, kDiagThreads, 0, st>>>(n, u, P, radial, r_step, dx, c12, c13, c14, out);
   } else {
     PhysD ph = {};
     ph.c13 = c13;
@@ -391,18 +393,17 @@ cudaError_t diag_damping(int dtype, long long n, const void* u, const void* P, i
     F64Consts c = make_f64(ph, 0x1p-60);
     if (!(std::fabs(c12) <= 0x1p20)) c.fast = 0;
     k_damping_2d_c64<<<blocks_for((n + kGroup - 1) / kGroup), kDiagThreads, 0, st>>>(
-        n, (const float2*)u, (const float*)P, dx, c, c12, c13, c14, part, out);
+        n, (const float2*)u, (const float*)P, dx, c, c12, c13, c14, out);
   }
   return cudaGetLastError();
 }
 
 cudaError_t diag_relerr(int dtype_a, long long n, const void* a, const void* b, const double* P,
-                        double c12, double c13, double c14, double* part, double* out,
-                        cudaStream_t st) {
+                        double c12, double c13, double c14, const DiagOut& out, cudaStream_t st) {
   const int nb = blocks_for(n);
   const double2* bb = reinterpret_cast<const double2*>(b);
-  if (dtype_a == NLS_C128) k_relerr<double><<<nb, kDiagThreads, 0, st>>>(n, a, bb, P, c12, c13, c14, part, out);
-  else k_relerr<float><<<nb, kDiagThreads, 0, st>>>(n, a, bb, P, c12, c13, c14, part, out);
+  if (dtype_a == NLS_C128) k_relerr<double><<<nb, kDiagThreads, 0, st>>>(n, a, bb, P, c12, c13, c14, out);
+  else k_relerr<float><<<nb, kDiagThreads, 0, st>>>(n, a, bb, P, c12, c13, c14, out);
   return cudaGetLastError();
 }
 

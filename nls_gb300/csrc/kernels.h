@@ -168,27 +168,32 @@ cudaError_t launch_2d_stage(int dtype, int n, int s, const void* src, void* u, c
                             cudaStream_t st);
 
 // ---- diagnostics (FP64 sums, deterministic; one launch each)
-// d_partials: diag_partials_bytes, zeroed once when allocated; out: device-accessible (pinned host
-// memory), written by the last block.  Sums over n nodes:
+// partials: diag_partials_bytes, zeroed once when allocated; out: device-accessible (pinned host
+// memory), written by the last block, the sums from out[0] and the context's status word in
+// out[kDiagStatus].  Sums over n nodes:
 //   norm:   out[0] = sum |u_i|^2, out[1] = number of nodes with a non-finite component
 //   mu:     out[0..2] = sum w conj(u) v (re, im), sum w |u|^2
 //   relerr: out[0] = sum (|a|^2 - |b|^2)^2, out[1] = sum |b|^4,
 //           out[2] = sum (n_a - n_b)^2,     out[3] = sum n_b^2,  n = c12 P / (c13 + c14 |.|^2)
 // weight mode: 0 = 1, 1 = radial r_i = i * dx (1-D chemical potential, nls/nls.f90:941-946)
+constexpr int kDiagStatus = 4;
+struct DiagOut {
+  double* partials;
+  double* out;
+  const int* wait_flag;
+};
 size_t diag_partials_bytes(long long n);
-cudaError_t diag_norm(int dtype, long long n, const void* u, double* d_partials, double* out, cudaStream_t st);
+cudaError_t diag_norm(int dtype, long long n, const void* u, const DiagOut& out, cudaStream_t st);
 cudaError_t diag_mu(int dtype, long long n, const void* u, const void* v, int weight_mode,
-                    double dx, double* d_partials, double* out, cudaStream_t st);
+                    double dx, const DiagOut& out, cudaStream_t st);
 // the sums of mu on a square grid of side n with v = H(u) (op: order 5), weight 1
 cudaError_t diag_mu_2d(int dtype, int n, const void* u, const void* P, const PhysD& ph, const Stencil2D& op,
-                       double* d_partials, double* out, cudaStream_t st);
+                       const DiagOut& out, cudaStream_t st);
 // damping: out[0] = sum w_i (c12 P_i / (c13 + c14 |u_i|^2) - 1) |u_i|^2, w_i = 2 pi (i r_step) dx
 // (radial) or dx^2
 cudaError_t diag_damping(int dtype, long long n, const void* u, const void* P, int radial, double r_step,
-                         double dx, double c12, double c13, double c14, double* d_partials, double* out,
-                         cudaStream_t st);
+                         double dx, double c12, double c13, double c14, const DiagOut& out, cudaStream_t st);
 cudaError_t diag_relerr(int dtype_a, long long n, const void* a, const void* b_c128,
-                        const double* P, double c12, double c13, double c14, double* d_partials,
-                        double* out, cudaStream_t st);
+                        const double* P, double c12, double c13, double c14, const DiagOut& out, cudaStream_t st);
 
 }  // namespace nlsg

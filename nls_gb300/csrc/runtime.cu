@@ -72,8 +72,8 @@ struct nls_ctx {
   DevBuf xbuf;      // tagged exchange slots of cooperative launches, zeroed when allocated
   uint32_t xtag = 0;    // last tag used in xbuf
   double* h_diag = nullptr;  // pinned
-  // Status word of the bounded tile waits of this context's launches (a device int set by a
-  // fused 2-D kernel whose copy wait expired), and its pinned host mirror.
+  // Status word of the bounded waits of this context's launches (a device int set by a kernel whose
+  // wait expired), and its pinned host mirror.
   int* wait_flag = nullptr;
   int* h_wait_flag = nullptr;
 };
@@ -98,17 +98,23 @@ static int fail_cuda(nls_ctx* ctx, cudaError_t e, const char* what) {
 
 static size_t align256(size_t b) { return (b + 255) & ~(size_t)255; }
 
-// A bounded wait inside one of this context's tile kernels that expired leaves the context's
-// status word set; report it once (then clear it).  Synchronises the context's stream.
+// A bounded wait inside one of this context's kernels that expired leaves the context's status word
+// set; it is reported once (then cleared).
+static int report_timeout(nls_ctx* ctx) {
+  if (cudaMemsetAsync(ctx->wait_flag, 0, sizeof(int), ctx->stream) != cudaSuccess)
+    return fail(ctx, NLS_ERR_CUDA, "clearing the status word of the bounded waits failed");
+  return fail(ctx, NLS_ERR_TIMEOUT,
+              "a wait inside a kernel (for a tile copy, an item or another CTA's values) expired; the state is not valid");
+}
+// Reads the status word.  Synchronises the context's stream.
 static int check_timeout(nls_ctx* ctx) {
   if (cudaMemcpyAsync(ctx->h_wait_flag, ctx->wait_flag, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream) !=
           cudaSuccess ||
       cudaStreamSynchronize(ctx->stream) != cudaSuccess)
-    return fail(ctx, NLS_ERR_CUDA, "reading the tile-wait status word failed");
+    return fail(ctx, NLS_ERR_CUDA, "reading the status word of the bounded waits failed");
   if (*ctx->h_wait_flag) {
     *ctx->h_wait_flag = 0;
-    cudaMemsetAsync(ctx->wait_flag, 0, sizeof(int), ctx->stream);
-    return fail(ctx, NLS_ERR_TIMEOUT, "a tile copy did not arrive within its bounded wait");
+    return report_timeout(ctx);
   }
   return NLS_OK;
 }
@@ -607,6 +613,14 @@ static int diag_ensure(nls_ctx* ctx) {
   if (!ctx->h_diag) CK(ctx, cudaMallocHost(&ctx->h_diag, 64 * sizeof(double)));
   return NLS_OK;
 }
+static DiagOut diag_out(nls_ctx* ctx) { return DiagOut{(double*)ctx->diag.p, ctx->h_diag, ctx->wait_flag}; }
+
+// Waits for a diagnostic of `launches` launches; an error if a solve before it left the state invalid.
+static int diag_wait(nls_ctx* ctx, int launches) {
+  CK(ctx, cudaStreamSynchronize(ctx->stream));
+  ctx->launches += launches;
+  return ctx->h_diag[kDiagStatus] != 0.0 ? report_timeout(ctx) : NLS_OK;
+}
 
 // Sums of the chemical potential (nls/nls.f90:921-971) of a device state u: S = sum w conj(u) H(u)
 // and M = sum w |u|^2 (w = r_i in 1-D, 1 in 2-D), FP64, with H evaluated with the order-5
@@ -621,15 +635,13 @@ static int chem_pot_dev(nls_ctx* ctx, int dtype, int dim, double dx, int n, cons
     Stencil1D op;
     if (host_stencil_1d(n, 5, dx, &op)) return fail(ctx, NLS_ERR_INVALID, "operator");
     CK(ctx, launch_rhs_1d(dtype, n, du, dP, dv, ph, op, ctx->stream));
-    CK(ctx, diag_mu(dtype, n, du, dv, 1, dx, (double*)ctx->diag.p, ctx->h_diag, ctx->stream));
-    ctx->launches += 2;
+    CK(ctx, diag_mu(dtype, n, du, dv, 1, dx, diag_out(ctx), ctx->stream));
   } else {
     Stencil2D op;
     host_stencil_2d(5, dx, &op);
-    CK(ctx, diag_mu_2d(dtype, n, du, dP, ph, op, (double*)ctx->diag.p, ctx->h_diag, ctx->stream));
-    ctx->launches += 1;
+    CK(ctx, diag_mu_2d(dtype, n, du, dP, ph, op, diag_out(ctx), ctx->stream));
   }
-  CK(ctx, cudaStreamSynchronize(ctx->stream));
+  if ((st = diag_wait(ctx, dim == 1 ? 2 : 1))) return st;
   *s_re = ctx->h_diag[0];
   *s_im = ctx->h_diag[1];
   *m = ctx->h_diag[2];
@@ -1287,9 +1299,8 @@ NLS_API int nls_norm_device(nls_ctx* ctx, int dtype, int64_t count, const void* 
   CK(ctx, cudaSetDevice(ctx->device));
   int st = diag_ensure(ctx);
   if (st) return st;
-  CK(ctx, diag_norm(dtype, count, u_dev, (double*)ctx->diag.p, ctx->h_diag, ctx->stream));
-  CK(ctx, cudaStreamSynchronize(ctx->stream));
-  ctx->launches += 1;
+  CK(ctx, diag_norm(dtype, count, u_dev, diag_out(ctx), ctx->stream));
+  if ((st = diag_wait(ctx, 1))) return st;
   *sum_sq = ctx->h_diag[0];
   if (nonfinite) *nonfinite = (int64_t)ctx->h_diag[1];
   return ctx->h_diag[1] > 0 ? fail(ctx, NLS_ERR_NONFINITE, "non-finite values in state") : NLS_OK;
@@ -1309,9 +1320,8 @@ NLS_API int nls_damping_integral_device(nls_ctx* ctx, int dtype, const nls_probl
   const double r_step = pr->n > 1 ? (double)pr->n * pr->dx / (double)(pr->n - 1) : 0.0;
   const double* c = pr->coeffs;
   CK(ctx, diag_damping(dtype, N, u_dev, pumping_dev, pr->dim == 1 ? 1 : 0, r_step, pr->dx, c[11], c[12], c[13],
-                       (double*)ctx->diag.p, ctx->h_diag, ctx->stream));
-  CK(ctx, cudaStreamSynchronize(ctx->stream));
-  ctx->launches += 1;
+                       diag_out(ctx), ctx->stream));
+  if ((st = diag_wait(ctx, 1))) return st;
   *integral = ctx->h_diag[0];
   return NLS_OK;
 }
@@ -1328,9 +1338,8 @@ NLS_API int nls_density_error_device(nls_ctx* ctx, int dtype, int64_t count, con
   int st = diag_ensure(ctx);
   if (st) return st;
   CK(ctx, diag_relerr(dtype, count, u_dev, u_ref_c128_dev, pumping_f64_dev, c12, c13, c14,
-                      (double*)ctx->diag.p, ctx->h_diag, ctx->stream));
-  CK(ctx, cudaStreamSynchronize(ctx->stream));
-  ctx->launches += 1;
+                      diag_out(ctx), ctx->stream));
+  if ((st = diag_wait(ctx, 1))) return st;
   const double* v = ctx->h_diag;
   *rel_l2_density = v[1] > 0 ? std::sqrt(v[0] / v[1]) : std::sqrt(v[0]);
   *rel_l2_reservoir = v[3] > 0 ? std::sqrt(v[2] / v[3]) : std::sqrt(v[2]);

@@ -116,3 +116,33 @@ def test_expired_waits_leave_nan_where_the_state_is_not_right(gpu, kind):  # noq
         bad = np.isnan(got)
         assert bad.any() and np.array_equal(got[~bad], want[~bad])
         assert np.array_equal(_device_solve(gpu, s, steps, dtype, -1), want)
+
+
+@pytest.mark.parametrize("call", ["norm", "chemical_potential", "damping_integral", "density_errors"])
+@pytest.mark.parametrize("kind", ["1d c128", "2d c64"])
+def test_a_diagnostic_after_an_expired_solve_reports_it(gpu, kind, call):  # noqa: F811
+    """The usual loop of solving in place and logging: the first blocking call says that the state is
+    not valid, the next is the ordinary one again."""
+    torch = gpu
+    from nls_gb300 import _lib, device
+    s, dtype = (_spec_1d(700, 5) if kind[0] == "1" else _spec_2d(100, 3)), CASES[kind][1]
+    u, P = _tensors(torch, s, dtype)
+    kw = dict(order=s.order, dt=s.dt, dx=s.dx, coeffs=s.coeffs, iters=1)
+
+    def diagnostic(v):
+        if call == "norm":
+            return device.norm(v)
+        if call == "density_errors":
+            return device.density_errors(v, u.to(torch.complex128), P.double(), s.coeffs)
+        return getattr(device, call)(v, P, dx=s.dx, coeffs=s.coeffs)
+    want = diagnostic(device.solve_(u.clone(), P, **kw))
+    assert _lib.lib().nls_test_set_exchange_tag_extra(0, 1 << 20) == _lib.NLS_OK
+    try:
+        v = device.solve_(u.clone(), P, **kw)
+        with pytest.raises(_lib.NativeError) as err:
+            diagnostic(v)
+        assert err.value.status == _lib.NLS_ERR_TIMEOUT
+    finally:
+        assert _lib.lib().nls_test_set_exchange_tag_extra(0, 0) == _lib.NLS_OK
+    device.context(0).synchronize()
+    assert diagnostic(device.solve_(u.clone(), P, **kw)) == want
