@@ -272,6 +272,13 @@ int nls_test_set_stream_steps_per_launch(int mode);
  * use. */
 int nls_test_set_exchange_tag_extra(int device, unsigned extra);
 
+/* No counterpart in the reference.  Test control of the routes around those solves: last_tag, if
+ * larger than the last tag this context used, becomes it (tags end at 2^31 - 1, where the slots are
+ * cleared); decline = 1 lets this context's solves find no memory for the slots, 2 no room for all
+ * CTAs at once, 0 neither, so that with 1 and 2 the kernels of batches take them.  Not for production
+ * use. */
+int nls_test_set_exchange_state(nls_ctx* ctx, unsigned last_tag, int decline);
+
 #ifdef __cplusplus
 }
 #endif

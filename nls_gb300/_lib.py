@@ -103,6 +103,7 @@ SIGNATURES = {
     "nls_test_set_stream_dep_extra": (_i, [_i, ctypes.c_uint]),
     "nls_test_set_stream_steps_per_launch": (_i, [_i]),
     "nls_test_set_exchange_tag_extra": (_i, [_i, ctypes.c_uint]),
+    "nls_test_set_exchange_state": (_i, [_p, ctypes.c_uint, _i]),
 }
 
 _lib = None

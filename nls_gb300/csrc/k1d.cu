@@ -642,11 +642,13 @@ static size_t wide_smem(int dtype, int K, int threads) {
 
 // Segment length, steps per exchange and CTA size: the cheapest by a model of a step in cycles, the
 // four stages (longer when an SM's sub-partitions hold several warps) plus the exchange over the S
-// steps between two.  Constants from the measured instruction rates: a complex128 stage of one warp
-// per sub-partition has 550 to 900 cycles (orders 3 to 7) of FP64 instructions, which add up with more
+// steps between two.  Its constants: a complex128 stage, 900 cycles for one warp per sub-partition
+// whatever the order (its FP64 instructions take 550 to 900 at orders 3 to 7), which add up with more
 // warps; a complex64 one is latency (180 cycles the shortest chain, 350 measured at order 5), of which
-// more warps fill a part.  Only the ratios decide: among equal CTAs the largest S that fits the GPU wins.  Grids that fit one CTA,
-// or too large for all CTAs to be resident, stay on the kernels of one CTA or cluster.
+// more warps fill a part.  Only the ratios decide: among equal CTAs the largest S that fits the GPU wins.
+// Any grid that makes two segments is spread, also one that a single CTA could hold; grids no longer than
+// the smallest segment (orders 3, 5, 7: 64, 128, 320 nodes in complex64, 8, 16, 16 in complex128), and those
+// too large for all CTAs to be resident, stay on the kernels of one CTA or cluster.
 Wide1DPlan wide_1d_plan(int dtype, int K, int n, int sms) {
   Wide1DPlan best;
   const int per = dtype == NLS_C128 ? 0 : (K == 1 ? 1 : (K == 2 ? 2 : 4));   // nodes a thread

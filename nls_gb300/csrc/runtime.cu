@@ -71,6 +71,7 @@ struct nls_ctx {
   DevBuf diagv;     // H(u) scratch of the device chemical potential
   DevBuf xbuf;      // tagged exchange slots of cooperative launches, zeroed when allocated
   uint32_t xtag = 0;    // last tag used in xbuf
+  int test_decline = 0; // test control: cooperative launches find no memory (1) or no room (2)
   double* h_diag = nullptr;  // pinned
   // Status word of the bounded waits of this context's launches (a device int set by a kernel whose
   // wait expired), and its pinned host mirror.
@@ -243,19 +244,21 @@ static bool solve_coop(nls_ctx* ctx, int64_t iters, size_t slot_bytes, Tags&& ta
   }
   *status = NLS_OK;
   cudaError_t e = cudaSuccess;
+  if (ctx->test_decline == 1) slot_bytes = SIZE_MAX;
   if (slot_bytes > ctx->xbuf.bytes) {
     if (ctx->xbuf.ensure(slot_bytes) != cudaSuccess) {
       cudaGetLastError();
       return false;
     }
-    e = cudaMemsetAsync(ctx->xbuf.p, 0, ctx->xbuf.bytes, ctx->stream);
     ctx->xtag = 0;
+    e = cudaMemsetAsync(ctx->xbuf.p, 0, ctx->xbuf.bytes, ctx->stream);
+    if (e != cudaSuccess) ctx->xbuf.release();   // slots that were never cleared are not used
   }
   for (int64_t done = 0, steps; done < iters && e == cudaSuccess; done += steps) {
     steps = std::min(kCoopStepsPerLaunch, iters - done);
     uint32_t tag;
     if ((e = exchange_tags(ctx, tags(steps), &tag)) != cudaSuccess) break;
-    e = launch(steps, tag);
+    e = ctx->test_decline == 2 ? cudaErrorCooperativeLaunchTooLarge : launch(steps, tag);
     if (e == cudaErrorCooperativeLaunchTooLarge && done == 0) {
       cudaGetLastError();
       return false;
@@ -281,8 +284,10 @@ static int solve_1d_dev(nls_ctx* ctx, int dtype, const nls_problem* pr, int64_t 
     std::memset(&I, 0, sizeof(I));
     I.u = u; I.P = P; I.n = n; I.cl = cl; I.steps = iters; I.dt = pr->dt; I.ph = ph; I.op = op;
     set_params(I);
-    // A solve on its own: spread over the whole GPU, unless it fits one CTA or the kernel a batch
-    // would take computes with other roundings (complex64 on more than 8 CTAs).
+    // A solve on its own: spread over the whole GPU wherever that makes two segments or more (also
+    // grids that one CTA could hold: complex64 order 5, 4096 nodes, 4.6 us a step on one CTA, 0.7
+    // spread), unless the kernel a batch would take computes with other roundings (complex64 on more
+    // than 8 CTAs).
     const Wide1DPlan plan = pr->variant == -1 && (dtype == NLS_C128 || cl <= 8)
                                 ? wide_1d_plan(dtype, op.K, n, ctx->sm_count) : Wide1DPlan();
     if (plan.grid && solve_coop(ctx, iters, wide_1d_slot_bytes(dtype, n),
@@ -1387,6 +1392,14 @@ NLS_API int nls_test_set_stream_dep_extra(int device, unsigned extra_steps) {
 NLS_API int nls_test_set_exchange_tag_extra(int device, unsigned extra) {
   if (cudaSetDevice(device) != cudaSuccess) return NLS_ERR_CUDA;
   return exchange_tag_extra_set_1d(extra) == cudaSuccess && exchange_tag_extra_set_2d(extra) == cudaSuccess ? NLS_OK : NLS_ERR_CUDA;
+}
+
+NLS_API int nls_test_set_exchange_state(nls_ctx* ctx, unsigned last_tag, int decline) {
+  if (!ctx || decline < 0 || decline > 2) return NLS_ERR_INVALID;
+  std::lock_guard<std::mutex> lk(ctx->mu);
+  if (last_tag > ctx->xtag) ctx->xtag = last_tag;   // a tag is never used twice
+  ctx->test_decline = decline;
+  return NLS_OK;
 }
 
 NLS_API int nls_batch_set(nls_batch* b, int index, const void* pumping, const void* u0) {

@@ -1,5 +1,5 @@
-"""GPU: solves spread over the whole GPU beside other work on the GPU, and what their results hold when
-a wait between their CTAs has expired."""
+"""GPU: solves spread over the whole GPU beside other work on the GPU, what their results hold when a
+wait between their CTAs has expired, and the kernels that take them where they cannot run."""
 
 import ctypes
 import threading
@@ -146,3 +146,70 @@ def test_a_diagnostic_after_an_expired_solve_reports_it(gpu, kind, call):  # noq
         assert _lib.lib().nls_test_set_exchange_tag_extra(0, 0) == _lib.NLS_OK
     device.context(0).synchronize()
     assert diagnostic(device.solve_(u.clone(), P, **kw)) == want
+
+
+@pytest.mark.parametrize("decline", [1, 2])
+@pytest.mark.parametrize("kind", list(CASES))
+def test_without_memory_or_room_the_other_kernels_take_the_solve(gpu, kind, decline):  # noqa: F811
+    """No memory for the exchange slots (1), no room for all CTAs at once (2): the same bits, by other
+    launches, and by the first ones again afterwards."""
+    from nls_gb300 import _lib, device
+    s, dtype = (_spec_1d(700, 5) if kind[0] == "1" else _spec_2d(100, 3)), CASES[kind][1]
+    want = _device_solve(gpu, s, 23, dtype, -1)
+    ctx = device.context(0)
+    assert _lib.lib().nls_test_set_exchange_state(ctx.handle, 0, decline) == _lib.NLS_OK
+    try:
+        before = ctx.launches
+        assert np.array_equal(_device_solve(gpu, s, 23, dtype, -1), want)
+        # one launch for all steps on a single CTA or cluster, else one or four a step
+        assert ctx.launches - before == {"1d c64": 1, "1d c128": 1, "2d c128": 4 * 23, "2d c64": 23}[kind]
+    finally:
+        assert _lib.lib().nls_test_set_exchange_state(ctx.handle, 0, 0) == _lib.NLS_OK
+    before = ctx.launches
+    assert np.array_equal(_device_solve(gpu, s, 23, dtype, -1), want)
+    assert ctx.launches - before == 1
+
+
+@pytest.mark.parametrize("kind", list(CASES))
+def test_tags_start_again_when_they_run_out(gpu, kind):  # noqa: F811
+    """Solves of a few steps across the end of the tags, with the slots full of the largest ones."""
+    from nls_gb300 import _lib
+    s, dtype = (_spec_1d(700, 5) if kind[0] == "1" else _spec_2d(100, 3)), CASES[kind][1]
+    want = _device_solve(gpu, s, 9, dtype, -1)
+    u, P = _tensors(gpu, s, dtype)
+    gpu.cuda.synchronize()
+    ctx = _lib.Context(0)
+    _solve_on(ctx, s, u.clone(), P, 1)      # allocates the slots
+    assert _lib.lib().nls_test_set_exchange_state(ctx.handle, (1 << 31) - 1 - 100, 0) == _lib.NLS_OK
+    for _ in range(40):
+        v = u.clone()
+        gpu.cuda.synchronize()
+        _solve_on(ctx, s, v, P, 9)
+        ctx.synchronize()
+        got = v.cpu().numpy()
+        assert np.array_equal(got.T if s.dim == 2 else got, want)
+
+
+def test_under_capture_the_stage_kernels_take_the_solve(gpu):  # noqa: F811
+    """A graph replays its launches with the same arguments, tags included: a captured solve takes the
+    kernels without an exchange, and every replay advances the state."""
+    torch = gpu
+    from nls_gb300 import device
+    s = _spec_2d(100, 3)
+    u, P = _tensors(torch, s, np.complex128)
+    kw = dict(order=s.order, dt=s.dt, dx=s.dx, coeffs=s.coeffs)
+    want = device.solve_(u.clone(), P, iters=9, **kw)
+    v = u.clone()
+    device.solve_(v, P, iters=3, variant=0, **kw)      # allocates the stage buffers
+    torch.cuda.synchronize()
+    side = torch.cuda.Stream()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.stream(side):
+        graph.capture_begin()
+        device.solve_(v, P, iters=3, **kw)
+        graph.capture_end()
+    torch.cuda.synchronize()
+    for _ in range(2):
+        graph.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(v, want)
