@@ -3,8 +3,8 @@
 // finish adds them in a fixed order, so a result never depends on what else runs on the GPU.
 //
 // The FP64 pipe would bound these sums, not memory (a DFMA of a warp takes 19 cycles of its SM, a
-// conversion 16; 8 bytes a lane arrive in 12).  The complex64 forms therefore add up groups of 16
-// nodes in pairs of floats (f64_node.cuh) -- products of floats are exact as pairs, the group's sum
+// conversion 16; 8 bytes a lane arrive in 12).  The complex64 forms of the norm and the chemical
+// potential therefore add up groups of 16 nodes in pairs of floats (f64_node.cuh) -- products of floats are exact as pairs, the group's sum
 // good to 2^-46 of the sum of its terms' sizes, independently from group to group -- and add the
 // groups in FP64.  Small grids and groups whose values the pairs cannot hold (non-finite, squares near the ends of
 // single precision) are added in FP64 node by node.
@@ -299,47 +299,41 @@ __global__ void __launch_bounds__(kDiagThreads) k_damping(long long n, const voi
   }
   diag_finish<1>(v, out);
 }
-// complex64 on a square grid: groups in float pairs, the reservoir as in the complex128 steps.
+// A float as a double by integer operations (a conversion takes 16 cycles of its SM); ok is cleared for
+// denormal, infinite and NaN values.
+__device__ __forceinline__ double widen(float f, bool& ok) {
+  const uint32_t b = bitsf(f), mag = b & 0x7fffffffu;
+  ok = ok && (mag == 0u || mag - 0x00800000u < 0x7f000000u);
+  return mag == 0u ? 0.0 : dbits((mag >> 3) + (896u << 20) | (b & 0x80000000u), b << 29);
+}
+// complex64 on a square grid, every term in FP64: near balance of gain and loss, the usual state of a
+// condensate, n_res - 1 is small beside n_res, so it is formed as (c12 P - D) / D with D = c13 + c14 |u|^2,
+// the difference first.  The quotient is t = t0 + y (N - t0 D), t0 = N y, y = 1/D by one Newton step in
+// single precision (2^-45), so t is good to a double's last place.  Eight FP64 instructions a node bound
+// it: 2048^2 takes 70 us, the caches cold.  Float pairs for the whole term took 29 us, but lost 2^-45 of
+// n_res: 4e-13 of the sum of the terms' sizes at n_res within 1e-3 of 1, against 1e-15 in FP64.
 __global__ void __launch_bounds__(kDiagThreads) k_damping_2d_c64(long long n, const float2* __restrict__ u,
-                                                                 const float* __restrict__ P, double dx, F64Consts c,
-                                                                 double c12, double c13, double c14,
-                                                                 DiagOut out) {
+                                                                 const float* __restrict__ P, double dx, double c12,
+                                                                 double c13, double c14, DiagOut out) {
   double v[1] = {0.0};
   const long long stride = (long long)gridDim.x * blockDim.x;
-  // c12 / (c13 + c14 d): the pump's constant is not folded into the pair of P (exact as it is)
-  const F2 p12 = {(float)c12, (float)(c12 - (double)(float)c12)};
-  for (long long i0 = (long long)blockIdx.x * blockDim.x + threadIdx.x; i0 < n; i0 += kGroup * stride) {
-    float2 a[kGroup];
-    float p[kGroup];
-#pragma unroll
-    for (int k = 0; k < kGroup; ++k) {
-      const bool in = i0 + k * stride < n;
-      a[k] = in ? u[i0 + k * stride] : make_float2(0.f, 0.f);
-      p[k] = in ? P[i0 + k * stride] : 0.f;
-    }
-    F2 s = {0.f, 0.f}, m = {0.f, 0.f};
-    bool ok = c.fast != 0;
-#pragma unroll
-    for (int k = 0; k < kGroup; ++k) {
-      const F2 xx = pair_prod(a[k].x, a[k].x), yy = pair_prod(a[k].y, a[k].y);
-      const F2 d = f2_density(xx, yy);
-      pair_add(m, d);
-      const F2 pc = f2_mul(p12, F2{p[k], 0.f});
-      bool dok;
-      const F2 r = f2_add(f2_reservoir(f2_quick(pc.h, pc.l), d, c, dok), F2{-1.f, 0.f});
-      ok = ok && dok && fabsf(p[k]) < 0x1p40f;
-      const F2 t = f2_mul(r, d);
-      pair_add(s, t);
-    }
-    if (ok && pair_range(m.h) && fabsf(s.h) < 0x1p100f) {
-      v[0] += pair_value(s);
-    } else {
-#pragma unroll 1
-      for (int k = 0; k < kGroup; ++k) {
-        if (i0 + k * stride >= n) break;
-        v[0] += damping_term<float>(u[i0 + k * stride], P[i0 + k * stride], c12, c13, c14);
-      }
-    }
+#pragma unroll 2
+  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
+    const float2 a = u[i];
+    const float p = P[i];
+    bool ok = true;
+    const double x = widen(a.x, ok), y = widen(a.y, ok), pd = widen(p, ok);
+    const double d = dfma(x, x, dmul(y, y));
+    const double den = dfma(c14, d, c13), num = dfma(c12, pd, -den);
+    // |den| in [2^-58, 2^58)
+    ok = ok && (dhi(den) & 0x7fffffffu) - ((1023u - 58u) << 20) < (116u << 20);
+    const F2 s = f2_split(den);
+    const float yr = frcp(s.h);
+    const double inv = f2_join(f2_quick(yr, fmul(yr, ffma(-s.l, yr, ffma(-s.h, yr, 1.f)))));
+    const double t0 = dmul(num, inv);
+    const double t = dfma(dfma(-t0, den, num), inv, t0);
+    if (ok) v[0] = dfma(t, d, v[0]);
+    else v[0] += damping_term<float>(a, p, c12, c13, c14);
   }
   v[0] *= dx * dx;
   diag_finish<1>(v, out);
@@ -383,17 +377,10 @@ cudaError_t diag_damping(int dtype, long long n, const void* u, const void* P, i
   const int nb = blocks_for(n);
   if (dtype == NLS_C128) {
     k_damping<double><<<nb, kDiagThreads, 0, st>>>(n, u, P, radial, r_step, dx, c12, c13, c14, out);
-  } else if (radial || n < kPairsFrom) {
+  } else if (radial) {
     k_damping<float><<<nb, kDiagThreads, 0, st>>>(n, u, P, radial, r_step, dx, c12, c13, c14, out);
   } else {
-    PhysD ph = {};
-    ph.c13 = c13;
-    ph.c14 = c14;
-    ph.c12 = c12;
-    F64Consts c = make_f64(ph, 0x1p-60);
-    if (!(std::fabs(c12) <= 0x1p20)) c.fast = 0;
-    k_damping_2d_c64<<<blocks_for((n + kGroup - 1) / kGroup), kDiagThreads, 0, st>>>(
-        n, (const float2*)u, (const float*)P, dx, c, c12, c13, c14, out);
+    k_damping_2d_c64<<<nb, kDiagThreads, 0, st>>>(n, (const float2*)u, (const float*)P, dx, c12, c13, c14, out);
   }
   return cudaGetLastError();
 }
