@@ -157,10 +157,10 @@ __global__ void __launch_bounds__(LANES ? 1024 : 768) rk4_2d_wide_f64(const __gr
             at[i] = 2 * h.x + (k & 1);
             want[i] = h.y >= 0 ? from + 2 * (size_t)h.y + (k & 1) : nullptr;
           }
-          x_wait<4>(want, tag + extra, got, wait_flag, dead);
+          x_wait<4, false>(want, tag + extra, got, wait_flag, dead);
 #pragma unroll
           for (int i = 0; i < 4; ++i)
-            if (want[i]) in[at[i]] = x_f64(got[i]);
+            if (want[i]) in[at[i]] = x_f64(dead ? kExchangeNaN : got[i]);
         }
         __syncwarp();
         asm volatile("barrier.arrive 1, %0;" ::"r"(halo_threads + edge_threads) : "memory");
