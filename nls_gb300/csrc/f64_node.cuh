@@ -86,13 +86,15 @@ static inline double dadd(double a, double b) { return a + b; }
 static inline double dmul(double a, double b) { return a * b; }
 #endif
 
-// Quotient of the plain expressions: a * (1/b), the reciprocal by one Newton step from an FP32
-// seed (2^-42); denominators outside the FP32 normal range take the IEEE division.
+// Quotient of the plain expressions: a * (1/b), the reciprocal by two Newton steps from an FP32
+// seed (good to a double's last place; one step leaves 2^-42); denominators outside the FP32 normal
+// range take the IEEE division.
 NLSG_HD inline double f64_div(double a, double b) {
   const float bf = (float)b;
   const float m = bf < 0.f ? -bf : bf;
   if (!(m >= 1e-30f && m <= 1e30f)) return a / b;
   double y = (double)frcp(bf);
+  y = dfma(y, dfma(-b, y, 1.0), y);
   y = dfma(y, dfma(-b, y, 1.0), y);
   return a * y;
 }

@@ -146,10 +146,11 @@ __global__ void __launch_bounds__(kDiagThreads) k_mu(long long n, const void* __
   diag_finish<3>(v, out);
 }
 
-// The same on a square grid with H(u) (order 5) formed on the way: a warp walks G rows of 32
-// columns with the five rows of its column in registers (G = kGroup, or 1 without pairs).  complex64: H in single precision as
-// before, the sums in float pairs; complex128: f64_slope_2d and FP64 sums.  Before, H was written
-// and read back by launches of their own and every term added in FP64.
+// The same on a square grid with H(u) (order 5) formed on the way: a warp walks G rows of 32 columns
+// with the five rows of its column in registers (G = kGroup, or 1 without pairs).  complex64: H in single
+// precision as before, the sums in float pairs; complex128: the coefficients in plain FP64 (a step's
+// float pairs, f64_node.cuh, would leave 2^-45 of them in the result) and FP64 sums.  Before, H was
+// written and read back by launches of their own and every term added in FP64.
 template <int G>
 __global__ void __launch_bounds__(kDiagThreads) k_mu_2d_c64(int n, const float2* __restrict__ u,
                                                             const float* __restrict__ P, Params<float> prm,
@@ -240,7 +241,9 @@ __global__ void __launch_bounds__(kDiagThreads) k_mu_2d_c128(int n, const double
     const double2 a = u[(size_t)y * n + x];
     const double p = P[(size_t)y * n + x];
     double hx, hy;
-    f64_slope_2d<2>(a.x, a.y, vx, vy, f2_split(p), f64_in_range(p), &p, c, hx, hy);
+    double A, B;
+    f64_coeffs_plain(a.x, a.y, p, c, A, B);
+    f64_slope_2d<2>(a.x, a.y, vx, vy, A, dadd(B, -c.centre), c, hx, hy);
     v[0] = dfma(a.x, hx, dfma(a.y, hy, v[0]));
     v[1] = dfma(a.x, hy, dfma(-a.y, hx, v[1]));
     v[2] = dfma(a.x, a.x, dfma(a.y, a.y, v[2]));
@@ -364,8 +367,7 @@ cudaError_t diag_mu_2d(int dtype, int n, const void* u, const void* P, const Phy
   const int rows = dtype == NLS_C128 || (long long)n * n < kPairsFrom ? 1 : kGroup;   // of a warp at a time
   const int nb = blocks_for((long long)((n + rows - 1) / rows) * ((n + 31) / 32) * 32);
   if (dtype == NLS_C128)
-    // (a step so small that the pairs' limit on dt |a| does not bind)
-    k_mu_2d_c128<<<nb, kDiagThreads, 0, st>>>(n, (const double2*)u, (const double*)P, make_f64(ph, 0x1p-60, op), out);
+    k_mu_2d_c128<<<nb, kDiagThreads, 0, st>>>(n, (const double2*)u, (const double*)P, make_f64(ph, 0.0, op), out);
   else
     (rows == 1 ? k_mu_2d_c64<1> : k_mu_2d_c64<kGroup>)<<<nb, kDiagThreads, 0, st>>>(
         n, (const float2*)u, (const float*)P, make_params<float>(ph, 0.0, op.center, op.w[0], op.w[1]), out);

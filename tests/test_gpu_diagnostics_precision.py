@@ -79,3 +79,32 @@ def test_damping_integral_values_at_the_ends(gpu, case):  # noqa: F811
         assert not math.isfinite(got) and math.isnan(got) == math.isnan(float(term.sum()))
     else:
         assert abs(got - math.fsum(term.ravel())) <= 24 * EPS * size
+
+
+@pytest.mark.parametrize("power", [0.0, 2.0])
+def test_complex128_chemical_potential_of_a_uniform_density(gpu, power):  # noqa: F811
+    """|u|^2 and the pump the same at every node, so that a node's error does not average out.  About
+    ten roundings a node and twenty levels of sums, each 2^-53 / sqrt(3) of the terms' sizes rms, so
+    3.2 times 2^-53 over many amplitudes: at most 8."""
+    torch = gpu
+    from nls_gb300 import device, workloads as w
+    getcontext().prec = 40
+    c, dx, n = w.coeffs(), 1.0, 24
+    cf = [Decimal(float(v)) for v in c]
+    # the order-5 Laplacian of a constant, mean over the grid: the neighbours outside it are missing
+    wt = {1: Decimal(16) / 12, 2: Decimal(-1) / 12}
+    lost = sum(wt[d] for i in range(n) for d in (1, 2) for j in (i - d, i + d) if not 0 <= j < n)
+    lap = -2 * n * lost / (n * n)
+    errors = []
+    for amp in np.random.default_rng(1).uniform(3, 30, 80):
+        u = np.full((n, n), amp * np.exp(0.7j))
+        mu = device.chemical_potential(torch.tensor(u, device="cuda"), torch.full((n, n), power, dtype=torch.float64,
+                                                                                 device="cuda"), dx=dx, coeffs=c)
+        x, y, p = Decimal(float(u[0, 0].real)), Decimal(float(u[0, 0].imag)), Decimal(power)
+        s = x * x + y * y
+        r = cf[11] * p / (cf[12] + cf[13] * s)
+        a, b = cf[2] * r - cf[3], cf[4] * s + cf[5] * r
+        # <u, H u> / <u, u> = a - i b + i lap, and mu is i times that
+        size = float(abs(cf[2] * r) + cf[3] + b) + 5.0 + 68 / 12
+        errors += [float(Decimal(mu.real) - (b - lap)) / size, float(Decimal(mu.imag) - a) / size]
+    assert math.sqrt(np.mean(np.square(errors))) <= 8 * EPS
