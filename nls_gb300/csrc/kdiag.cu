@@ -4,10 +4,14 @@
 //
 // The FP64 pipe would bound these sums, not memory (a DFMA of a warp takes 19 cycles of its SM, a
 // conversion 16; 8 bytes a lane arrive in 12).  The complex64 forms of the norm and the chemical
-// potential therefore add up groups of 16 nodes in pairs of floats (f64_node.cuh) -- products of floats are exact as pairs, the group's sum
-// good to 2^-46 of the sum of its terms' sizes, independently from group to group -- and add the
-// groups in FP64.  Small grids and groups whose values the pairs cannot hold (non-finite, squares near the ends of
-// single precision) are added in FP64 node by node.
+// potential therefore add up groups of 16 nodes in single precision without loss -- a product of floats
+// is exact as a pair, and the group's sum is kept in three floats, whose additions leave 2^-66 of the
+// sum of its terms' sizes -- and add the groups in FP64: one rounding to a double's last place a group,
+// where FP64 sums round for every node.  (Two floats a group lost 2^-48 an addition: 8e-15 of the norm of
+// a nearly uniform state, against 2.5e-15 for FP64 sums and below 1e-15 here; 2048^2, the caches cold: norm
+// 21 us with two floats and 24 with three, chemical potential 56 and 64.)  Small grids and groups with
+// values outside single precision's range (non-finite, squares near its ends) are added in FP64 node by
+// node.
 #include <algorithm>
 
 #include "kernels.h"
@@ -18,10 +22,9 @@ namespace nlsg {
 static constexpr int kDiagBlocks = 1216;  // 8 x 152 SMs
 static constexpr int kDiagThreads = 256;
 static constexpr int kDiagMaxNV = kDiagStatus;
-static constexpr int kGroup = 16;         // nodes added up in float pairs
-// Grids from which the groups are added up in pairs: their errors, independent of one another, leave
-// 2^-46 / sqrt(groups), below 2^-52 of the sum of the terms' sizes.  Smaller grids are added up in
-// FP64, one node a thread: what counts there is the length of a thread's chain.
+static constexpr int kGroup = 16;         // nodes added up in single precision
+// Grids from which groups are added up so.  Smaller grids are added up in FP64, one node a thread: what
+// counts there is the length of a thread's chain.
 static constexpr long long kPairsFrom = 65536;
 
 size_t diag_partials_bytes(long long) { return (size_t)kDiagBlocks * kDiagMaxNV * sizeof(double) + 256; }
@@ -62,11 +65,17 @@ __device__ __forceinline__ void diag_finish(double (&v)[NV], const DiagOut& d) {
   }
 }
 
-// acc += t, the error of the high sum kept in the low one.
-__device__ __forceinline__ void pair_add(F2& acc, F2 t) {
+// A sum held as h + m + l.
+struct F3 {
+  float h, m, l;
+};
+// acc += t: exact but for the additions to l, which is about 2^-48 of the terms.
+__device__ __forceinline__ void sum_add(F3& acc, F2 t) {
   const F2 s = f2_sum(acc.h, t.h);
+  const F2 a = f2_sum(acc.m, t.l), b = f2_sum(a.h, s.l);
   acc.h = s.h;
-  acc.l = fadd(acc.l, fadd(s.l, t.l));
+  acc.m = b.h;
+  acc.l = fadd(acc.l, fadd(a.l, b.l));
 }
 __device__ __forceinline__ F2 pair_prod(float a, float b) {
   F2 r;
@@ -74,27 +83,34 @@ __device__ __forceinline__ F2 pair_prod(float a, float b) {
   r.l = ffma(a, b, -r.h);
   return r;
 }
-// A group's sum of squares from which what single precision loses below 2^-100 is below a double's
-// last place, and no square overflowed (false for NaN).
-__device__ __forceinline__ bool pair_range(float sum_sq) { return sum_sq >= 0x1p-40f && sum_sq < 0x1p100f; }
-__device__ __forceinline__ double pair_value(F2 a) { return f2_join(f2_sum(a.h, a.l)); }
+// A group's sum of squares of which what products of floats lose (2^-149 each) is below 2^-60, and no
+// square overflowed (false for NaN).
+__device__ __forceinline__ bool sum_range(float sum_sq) { return sum_sq >= 0x1p-80f && sum_sq < 0x1p100f; }
+// v + the sum, rounded to a double's last place; what that leaves goes to rest.
+__device__ __forceinline__ double sum_to(double v, F3 a, float& rest) {
+  const F2 s = f2_sum(a.h, a.m), q = f2_sum(s.l, a.l);
+  rest = fadd(rest, q.l);
+  if (fabsf(s.h) < 0x1p-64f) return v + ((double)s.h + (double)q.h);   // f2_join would drop q.h
+  return v + f2_join(f2_quick(s.h, q.h));
+}
 
 __global__ void __launch_bounds__(kDiagThreads) k_norm_c64(long long n, const float2* __restrict__ u,
                                                            DiagOut out) {
   double v[2] = {0.0, 0.0};
+  float rest = 0.f;
   const long long stride = (long long)gridDim.x * blockDim.x;
   for (long long i0 = (long long)blockIdx.x * blockDim.x + threadIdx.x; i0 < n; i0 += kGroup * stride) {
     float2 a[kGroup];
 #pragma unroll
     for (int k = 0; k < kGroup; ++k) a[k] = i0 + k * stride < n ? u[i0 + k * stride] : make_float2(0.f, 0.f);
-    F2 s = {0.f, 0.f};
+    F3 s = {0.f, 0.f, 0.f};
 #pragma unroll
     for (int k = 0; k < kGroup; ++k) {
-      pair_add(s, pair_prod(a[k].x, a[k].x));
-      pair_add(s, pair_prod(a[k].y, a[k].y));
+      sum_add(s, pair_prod(a[k].x, a[k].x));
+      sum_add(s, pair_prod(a[k].y, a[k].y));
     }
-    if (pair_range(s.h)) {
-      v[0] += pair_value(s);
+    if (sum_range(s.h)) {
+      v[0] = sum_to(v[0], s, rest);
     } else {
 #pragma unroll 1
       for (int k = 0; k < kGroup; ++k) {
@@ -106,6 +122,7 @@ __global__ void __launch_bounds__(kDiagThreads) k_norm_c64(long long n, const fl
       }
     }
   }
+  v[0] += (double)rest;
   diag_finish<2>(v, out);
 }
 
@@ -148,7 +165,7 @@ __global__ void __launch_bounds__(kDiagThreads) k_mu(long long n, const void* __
 
 // The same on a square grid with H(u) (order 5) formed on the way: a warp walks G rows of 32 columns
 // with the five rows of its column in registers (G = kGroup, or 1 without pairs).  complex64: H in single
-// precision as before, the sums in float pairs; complex128: the coefficients in plain FP64 (a step's
+// precision as before, the sums without loss as above; complex128: the coefficients in plain FP64 (a step's
 // float pairs, f64_node.cuh, would leave 2^-45 of them in the result) and FP64 sums.  Before, H was
 // written and read back by launches of their own and every term added in FP64.
 template <int G>
@@ -156,6 +173,7 @@ __global__ void __launch_bounds__(kDiagThreads) k_mu_2d_c64(int n, const float2*
                                                             const float* __restrict__ P, Params<float> prm,
                                                             DiagOut out) {
   double v[3] = {0.0, 0.0, 0.0};
+  float rest[3] = {0.f, 0.f, 0.f};
   const Phys<float> ph = phys_of<float>(prm);
   const int lane = threadIdx.x & 31;
   const int cols = (n + 31) / 32;
@@ -177,7 +195,7 @@ __global__ void __launch_bounds__(kDiagThreads) k_mu_2d_c64(int n, const float2*
     float2 w[5];
 #pragma unroll
     for (int k = 0; k < 4; ++k) w[k] = at(x, y0 - 2 + k);
-    F2 re = {0.f, 0.f}, im = {0.f, 0.f}, m = {0.f, 0.f};
+    F3 re = {0.f, 0.f, 0.f}, im = re, m = re;
 #pragma unroll
     for (int j = 0; j < G; ++j) {
       const int y = y0 + j;
@@ -187,18 +205,18 @@ __global__ void __launch_bounds__(kDiagThreads) k_mu_2d_c64(int n, const float2*
       const float2 h = slope(c, sum4(at(x - 1, y), at(x + 1, y), w[(j + 1) % 5], w[(j + 3) % 5]),
                              sum4(at(x - 2, y), at(x + 2, y), w[j % 5], w[(j + 4) % 5]), p);
       if (y < n) {
-        pair_add(re, pair_prod(c.x, h.x));
-        pair_add(re, pair_prod(c.y, h.y));
-        pair_add(im, pair_prod(c.x, h.y));
-        pair_add(im, pair_prod(-c.y, h.x));
-        pair_add(m, pair_prod(c.x, c.x));
-        pair_add(m, pair_prod(c.y, c.y));
+        sum_add(re, pair_prod(c.x, h.x));
+        sum_add(re, pair_prod(c.y, h.y));
+        sum_add(im, pair_prod(c.x, h.y));
+        sum_add(im, pair_prod(-c.y, h.x));
+        sum_add(m, pair_prod(c.x, c.x));
+        sum_add(m, pair_prod(c.y, c.y));
       }
     }
-    if (G > 1 && pair_range(m.h) && fabsf(re.h) < 0x1p100f && fabsf(im.h) < 0x1p100f) {
-      v[0] += pair_value(re);
-      v[1] += pair_value(im);
-      v[2] += pair_value(m);
+    if (G > 1 && sum_range(m.h) && fabsf(re.h) < 0x1p100f && fabsf(im.h) < 0x1p100f) {
+      v[0] = sum_to(v[0], re, rest[0]);
+      v[1] = sum_to(v[1], im, rest[1]);
+      v[2] = sum_to(v[2], m, rest[2]);
     } else {
 #pragma unroll 1
       for (int y = y0; y < y0 + G && y < n; ++y) {
@@ -212,6 +230,8 @@ __global__ void __launch_bounds__(kDiagThreads) k_mu_2d_c64(int n, const float2*
       }
     }
   }
+#pragma unroll
+  for (int k = 0; k < 3; ++k) v[k] += (double)rest[k];
   diag_finish<3>(v, out);
 }
 

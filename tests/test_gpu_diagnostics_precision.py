@@ -108,3 +108,19 @@ def test_complex128_chemical_potential_of_a_uniform_density(gpu, power):  # noqa
         size = float(abs(cf[2] * r) + cf[3] + b) + 5.0 + 68 / 12
         errors += [float(Decimal(mu.real) - (b - lap)) / size, float(Decimal(mu.imag) - a) / size]
     assert math.sqrt(np.mean(np.square(errors))) <= 8 * EPS
+
+
+@pytest.mark.parametrize("n", [255, 256, 700])
+def test_norm_of_a_nearly_uniform_state(gpu, n):  # noqa: F811
+    """Nodes within 1e-3 of one amplitude, so that errors of equal sign add up: the last levels of the
+    sums, a dozen, round to a double's last place, 2^-53 / sqrt(3) rms each: at most four of it over
+    many amplitudes, and 8 of it is the bound."""
+    torch = gpu
+    from nls_gb300 import device
+    rng = np.random.default_rng(n)
+    errors = []
+    for amp in rng.uniform(0.5, 3, 24):
+        u = (amp * (1 + 1e-3 * rng.random((n, n))) * np.exp(0.3j)).astype(np.complex64)
+        want = math.fsum(np.float64(u.real).ravel() ** 2) + math.fsum(np.float64(u.imag).ravel() ** 2)
+        errors.append(device.norm(torch.tensor(u, device="cuda")) / want - 1)
+    assert math.sqrt(np.mean(np.square(errors))) <= 8 * EPS
