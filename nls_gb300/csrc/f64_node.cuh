@@ -17,8 +17,9 @@
 //     exact value than the FP64 chain it replaces (8 FP64 instructions a node at order 3, 16 at
 //     order 5).
 // Values the float pairs cannot hold (non-finite, huge, or a denominator outside 2^+-60) and steps
-// so long that the pairs' error would reach the state's last place (dt/2 |a| or dt/2 |b| above 2^-8)
-// take the plain FP64 expressions instead, decided per node.
+// so long that the pairs' error would reach the state's last place (dt/2 times c3 r, c4, c5 |u|^2 or
+// c6 r above 2^-8: the terms, since the error is a part of them, also where a or b vanishes because they
+// cancel) take the plain FP64 expressions instead, decided per node.
 #pragma once
 
 #include <stdint.h>
@@ -44,6 +45,7 @@ __device__ __forceinline__ float frcp(float x) {
   return y;
 }
 __device__ __forceinline__ float u2f(uint32_t x) { return __uint2float_rn(x); }
+__device__ __forceinline__ float fmax_abs(float a, float b) { return fmaxf(fabsf(a), fabsf(b)); }
 __device__ __forceinline__ int f2i(float x) { return __float2int_rn(x); }
 __device__ __forceinline__ uint32_t shf_l(uint32_t lo, uint32_t hi, int s) { return __funnelshift_l(lo, hi, s); }
 // hi:lo >> s, zero from 64 on
@@ -74,6 +76,11 @@ static inline float fadd(float a, float b) { return a + b; }
 static inline float fmul(float a, float b) { return a * b; }
 static inline float frcp(float x) { return 1.0f / x; }
 static inline float u2f(uint32_t x) { return (float)x; }
+static inline float fmax_abs(float a, float b) {
+  a = a < 0.f ? -a : a;
+  b = b < 0.f ? -b : b;
+  return a > b ? a : b;
+}
 static inline int f2i(float x) { return (int)lrintf(x); }
 static inline uint32_t shf_l(uint32_t lo, uint32_t hi, int s) { return (hi << s) | (lo >> (32 - s)); }
 static inline uint64_t shr64(uint32_t hi, uint32_t lo, uint32_t s) {
@@ -192,16 +199,16 @@ NLSG_HD inline bool f64_in_range(double v) { return (dhi(v) & 0x7fffffffu) < ((1
 
 // A = c3 r - c4 and B = c5 |u|^2 + c6 r, r = c12 P / (c13 + c14 |u|^2) (a and b of nls_common.cuh),
 // in pairs; false where they do not hold (the plain form then).  p: the pump split, p_ok: in range.
+// The limit is on the terms (c4's is the host's part): A and B vanish where their terms cancel.
 NLSG_HD inline bool f64_coeffs_pairs(double ux, double uy, F2 p, bool p_ok, const F64Consts& c, double& A, double& B) {
   const F2 s = f2_density(f2_square(f2_split(ux)), f2_square(f2_split(uy)));
   bool ok;
   const F2 r = f2_reservoir(p, s, c, ok);
-  const F2 a = f2_add(F2{-c.h[3], -c.l[3]}, f2_mul(F2{c.h[2], c.l[2]}, r));
-  const F2 b = f2_add(f2_mul(F2{c.h[4], c.l[4]}, s), f2_mul(F2{c.h[5], c.l[5]}, r));
-  const float aa = a.h < 0.f ? -a.h : a.h, ab = b.h < 0.f ? -b.h : b.h;
-  A = f2_join(a);
-  B = f2_join(b);
-  return ok && c.fast != 0 && p_ok && f64_in_range(ux) && f64_in_range(uy) && aa < c.lim && ab < c.lim;
+  const F2 t3 = f2_mul(F2{c.h[2], c.l[2]}, r), t5 = f2_mul(F2{c.h[4], c.l[4]}, s), t6 = f2_mul(F2{c.h[5], c.l[5]}, r);
+  A = f2_join(f2_add(F2{-c.h[3], -c.l[3]}, t3));
+  B = f2_join(f2_add(t5, t6));
+  return ok && c.fast != 0 && p_ok && f64_in_range(ux) && f64_in_range(uy) &&
+         fmax_abs(fmax_abs(t5.h, t6.h), t3.h) < c.lim;
 }
 NLSG_HD inline void f64_coeffs_plain(double ux, double uy, double P, const F64Consts& c, double& A, double& B) {
   const double s = dfma(ux, ux, dmul(uy, uy));
@@ -371,10 +378,9 @@ __device__ __forceinline__ bool f64_coeffs_lanes(double mine, F2 p, bool p_ok, c
   const F2 s = l.part ? f2_density(o, x) : f2_density(x, o);
   bool ok;
   const F2 r = f2_reservoir(p, s, c, ok);
-  const F2 v = f2_add(f2_mul(l.alpha, l.part ? s : F2{1.f, 0.f}), f2_mul(l.beta, r));
-  const float av = v.h < 0.f ? -v.h : v.h;
-  ok = ok && c.fast != 0 && p_ok && f64_in_range(mine) && av < c.lim;
-  const double val = f2_join(v), his = f64_other(val);
+  const F2 ts = f2_mul(l.alpha, l.part ? s : F2{1.f, 0.f}), tr = f2_mul(l.beta, r);
+  ok = ok && c.fast != 0 && p_ok && f64_in_range(mine) && fmax_abs(ts.h, tr.h) < c.lim;
+  const double val = f2_join(f2_add(ts, tr)), his = f64_other(val);
   A = l.part ? his : val;
   B = l.part ? val : his;
   // every lane takes part in the exchange, whatever its own answer
@@ -421,10 +427,9 @@ __device__ __forceinline__ double f64_slope_1d_lanes(double2 v, const double (&o
   const F2 r = f2_reservoir(p, q, c, ok);
   if (K > 2) tap(2);
   tap(K + 1);
-  const F2 w = f2_add(f2_mul(l.alpha, l.part ? q : F2{1.f, 0.f}), f2_mul(l.beta, r));
-  const float aw = w.h < 0.f ? -w.h : w.h;
-  ok = ok && c.fast != 0 && p_ok && f64_in_range(mine) && aw < c.lim;
-  const double val = f2_join(w), hval = f64_other(val);
+  const F2 t = f2_mul(l.alpha, l.part ? q : F2{1.f, 0.f}), tr = f2_mul(l.beta, r);
+  ok = ok && c.fast != 0 && p_ok && f64_in_range(mine) && fmax_abs(t.h, tr.h) < c.lim;
+  const double val = f2_join(f2_add(t, tr)), hval = f64_other(val);
   const int other_ok = __shfl_xor_sync(0xffffffffu, (int)ok, 1);
 #pragma unroll
   for (int d = K + 2; d <= 2 * K; ++d) tap(d);

@@ -43,7 +43,7 @@ struct F64Consts {
   double centre, unit;
   uint64_t unit_m;
   int unit_e;
-  float lim;          // |A|, |B| below which the pairs' error is below the state's last place
+  float lim;          // size of a term of A or B below which the pairs' error is below the state's last place
   int fast;           // every constant is zero or well inside the range of single precision
   int pad;
 };
@@ -119,6 +119,7 @@ inline F64Consts make_f64(const PhysD& ph, double dt, double centre = 0.0, doubl
   // the pairs are good to 2^-44 or better of A and B, which enter the state as dt/2 A u and dt/2 B u
   const double lim = 0x1p-8 / std::fabs(c.half_dt);
   c.lim = lim < 0x1p60 ? (float)lim : 0x1p60f;
+  if (!(std::fabs(ph.c4) < c.lim)) c.fast = 0;
   c.centre = centre;
   // unit = unit_m / 2^63 * 2^(unit_e - 1023); 0 outside the normal range (the plain products then)
   uint64_t bits;
