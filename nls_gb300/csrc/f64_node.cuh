@@ -7,9 +7,8 @@
 // double and float about 100, while FP32 and integer instructions issue every cycle.  So whatever
 // keeps its accuracy in other arithmetic leaves the FP64 pipe:
 //   * the reservoir and the coefficients a and b of the right-hand side (nls/nls.f90:570-650) are
-//     evaluated in pairs of floats: 3e-15 rms, 2^-45 at most, where one Newton step from an FP32
-//     seed left 5e-15 rms and 2^-44.4 (over pumps and densities of the benchmark's ranges).  About
-//     150 FP32 and integer instructions in place of 9 FP64 ones and two conversions;
+//     evaluated in pairs of floats, 2^-45 of their terms at most.  About 150 FP32 and integer
+//     instructions in place of 9 FP64 ones and two conversions;
 //   * doubles are split into such pairs and put together again by integer operations;
 //   * the neighbour part of the 2-D cross stencil (whose weights are whole numbers in units of
 //     1/h^2 or 1/(12 h^2)) is one 64-bit fixed-point sum aligned to the largest neighbour, times
@@ -20,6 +19,23 @@
 // so long that the pairs' error would reach the state's last place (dt/2 times c3 r, c4, c5 |u|^2 or
 // c6 r above 2^-8: the terms, since the error is a part of them, also where a or b vanishes because they
 // cancel) take the plain FP64 expressions instead, decided per node.
+//
+// Where the pairs are coarser than FP64 with a one-Newton-step quotient, which they replaced (rms errors,
+// measured on the GPU over the benchmark's coefficients, |u| <= 1): a is off by 2.8e-15 of its terms against
+// 1.8e-15 with pumps up to 8, b by 3.2e-15 against 2.0e-15; without a pump, where FP64 has no quotient to
+// form, a by 5.8e-16 against 0 and b by 2.3e-15 against 5e-17.  A slope also has the stencil in it, whose
+// fixed-point sum is closer than the FP64 chain it replaced, so the whole slope is off by 0.69 to 0.97
+// times as much at grid steps of 0.04 and with pumps up to 0.1 at 0.1 and 0.16, by 1.0 to 1.4 times at 0.1 and
+// 0.16 with pumps up to 8, and by 1.5 to 8 times at a grid step of 1, where the stencil is small: there the
+// limit above keeps it below the state's last place.  Final states against long double, geometric means of
+// the error over that of the FP64 form: with a pump 0.67 (radial, 300 to 2501 nodes) and 0.76 (square, 40 to
+// 100 a side) over 56 runs of 400 to 1000 steps at grid steps of 0.04 to 0.16; without one 0.91 to 1.05 by
+// order and grid step, 0.04 to 1, over 96 runs.
+// FP64 for everything but the quotient kept the coefficients at the former error and took 1.37 times
+// as long at 900^2 order 3 (107.8 against 78.7 us a step), 1.25 times on radial grids.
+//
+// The pair operations are the published ones: f2_sum is Knuth's two-sum, f2_quick Dekker's fast
+// two-sum, the products Dekker's with a fused multiply-add for the error.
 #pragma once
 
 #include <stdint.h>
@@ -44,7 +60,7 @@ __device__ __forceinline__ float frcp(float x) {
   asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
 }
-__device__ __forceinline__ float u2f(uint32_t x) { return __uint2float_rn(x); }
+__device__ __forceinline__ float i2f(int x) { return __int2float_rn(x); }
 __device__ __forceinline__ float fmax_abs(float a, float b) { return fmaxf(fabsf(a), fabsf(b)); }
 __device__ __forceinline__ int f2i(float x) { return __float2int_rn(x); }
 __device__ __forceinline__ uint32_t shf_l(uint32_t lo, uint32_t hi, int s) { return __funnelshift_l(lo, hi, s); }
@@ -75,7 +91,7 @@ static inline float ffma(float a, float b, float c) { return __builtin_fmaf(a, b
 static inline float fadd(float a, float b) { return a + b; }
 static inline float fmul(float a, float b) { return a * b; }
 static inline float frcp(float x) { return 1.0f / x; }
-static inline float u2f(uint32_t x) { return (float)x; }
+static inline float i2f(int x) { return (float)x; }
 static inline float fmax_abs(float a, float b) {
   a = a < 0.f ? -a : a;
   b = b < 0.f ? -b : b;
@@ -118,8 +134,8 @@ NLSG_HD inline F2 f2_quick(float a, float b) {  // a + b renormalised, |a| >= |b
   return r;
 }
 
-// A double rounded to 48 bits or more as hi + lo, split by integer operations; values below 2^-96
-// become zero.  |v| must be below 2^60.
+// A double as hi + lo, split by integer operations, hi the nearest float and lo its remainder to 24 bits,
+// so to 2^-49 of it; values below 2^-96 become zero.  |v| must be below 2^60.
 NLSG_HD inline F2 f2_split(double v) {
   const uint32_t hi = dhi(v), lo = dlo(v);
   const uint32_t mag = hi & 0x7fffffffu;
@@ -127,9 +143,9 @@ NLSG_HD inline F2 f2_split(double v) {
   const uint32_t t = mag - (896u << 20);
   const uint32_t f = shf_l(lo, t, 3) | (hi & 0x80000000u);  // sign, exponent - 896, 23 mantissa bits
   const uint32_t base = (f & 0xff800000u) - (23u << 23);    // the value of f's last place
-  // the 29 bits below f's last place, rounded to 24
-  const float rest = tiny ? 0.f : fmul(fmul(u2f(lo & 0x1fffffffu), 0x1p-29f), fbits(base));
-  return f2_quick(tiny ? 0.f : fbits(f), rest);
+  // the 29 bits below f's last place as a signed number: from half a place on, f is one place more
+  const float rest = fmul(fmul(i2f((int)(lo << 3) >> 3), 0x1p-29f), fbits(base));
+  return F2{tiny ? 0.f : fbits(f + ((lo >> 28) & 1u)), tiny ? 0.f : rest};
 }
 
 // hi + lo as a double, by integer operations.  |hi| in [2^-70, 2^60] keeps all of lo; smaller
@@ -181,18 +197,22 @@ NLSG_HD inline F2 f2_density(F2 x, F2 y) {
   const F2 s = f2_sum(x.h, y.h);
   return f2_quick(s.h, fadd(s.l, fadd(x.l, y.l)));
 }
+// p / d: a quotient whose remainder is exact in single precision, corrected twice; what is lost is below
+// the last place of the low part.
+NLSG_HD inline F2 f2_quotient(F2 p, F2 d) {
+  const float yr = frcp(d.h);
+  const float y0 = ffma(yr, ffma(-d.h, yr, 1.f), yr);
+  const float q0 = fmul(p.h, y0);
+  const float rem = ffma(-q0, d.h, p.h), low = ffma(-q0, d.l, p.l);
+  const float q1 = fmul(rem, y0);
+  return f2_quick(q0, ffma(fadd(ffma(-q1, d.h, rem), ffma(-q1, d.l, low)), y0, q1));
+}
 // p / (c13 + c14 s); ok: the denominator is in range.
 NLSG_HD inline F2 f2_reservoir(F2 p, F2 s, const F64Consts& c, bool& ok) {
   const F2 d = f2_add(F2{c.h[0], c.l[0]}, f2_mul(F2{c.h[1], c.l[1]}, s));
   const float ad = d.h < 0.f ? -d.h : d.h;
   ok = ad > 0x1p-60f && ad < 0x1p60f;
-  // two corrections of a quotient whose remainder is exact in single precision
-  const float yr = frcp(d.h);
-  const float y0 = ffma(yr, ffma(-d.h, yr, 1.f), yr);
-  const float q0 = fmul(p.h, y0);
-  const float rem = fadd(ffma(-q0, d.h, p.h), ffma(-q0, d.l, p.l));
-  const float q1 = fmul(rem, y0);
-  return f2_quick(q0, ffma(ffma(-q1, d.h, rem), y0, q1));
+  return f2_quotient(p, d);
 }
 // In range for the pairs: finite and below 2^40.
 NLSG_HD inline bool f64_in_range(double v) { return (dhi(v) & 0x7fffffffu) < ((1023u + 40u) << 20); }

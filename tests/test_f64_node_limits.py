@@ -90,9 +90,9 @@ def test_cancelling_terms_at_steps_of_all_lengths(node, what, dt):
 
 @pytest.mark.parametrize("power", [0.0, 0.1, 8.0])
 def test_errors_over_the_benchmark_ranges(node, power):
-    """With and without a pump: A and B hold their terms to 2^-45."""
+    """With and without a pump: a value is split to 2^-49 of it, A and B hold their terms to 2^-45."""
     rng = np.random.default_rng(9)
     rows = [_coeffs(rng) + list(rng.uniform(-1, 1, 2)) + [power * rng.random(), 1e-4] for _ in range(4000)]
     for v in node(rows):
-        assert v["pairs"]
+        assert v["pairs"] and abs(v["split"]) <= Fraction(1, 2 ** 49)
         assert all(abs(a) <= s * Fraction(1, 2 ** 45) for a, s in zip(v["err"], v["size"]))
