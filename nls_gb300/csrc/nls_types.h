@@ -141,8 +141,10 @@ inline Params<T> make_params(const PhysD& ph, double dt, double wc, double w1, d
   p.c12 = (T)ph.c12; p.c13 = (T)ph.c13; p.c14 = (T)ph.c14;
   p.half_dt = (T)(dt * 0.5); p.dt = (T)dt; p.dt6 = (T)(dt / 6.0);
   p.wc = (T)wc; p.w1 = (T)w1; p.w2 = (T)w2;
-  const double w = w2 != 0.0 ? -w2 : w1;
-  const double iw = w != 0.0 ? 1.0 / w : 0.0;
+  // (a weight below 2^-60 moves no state's last place, whatever the time step up to 2^30, and stands as
+  // 2^-60, so that the quotients stay within single precision)
+  const double least = 0x1p-60, weight = w2 != 0.0 ? -w2 : w1, w = weight > least ? weight : least;
+  const double iw = 1.0 / w;
   p.u3 = (T)(ph.c3 * iw); p.u4 = (T)(ph.c4 * iw); p.u5 = (T)(ph.c5 * iw); p.u6 = (T)(ph.c6 * iw);
   p.hw = (T)(0.5 * dt * w); p.dtw = (T)(dt * w); p.dw6 = (T)(dt * w / 6.0);
   return p;
