@@ -395,12 +395,11 @@ def run_serve(args):
     return 0
 
 
-# Algorithmic FP64 work of one node-step of the plain complex128 path (one RK4 step = four
-# right-hand sides + the RK4 combinations), counted per node and stage: the operator row (1-D
-# order 5: five complex-by-real multiply-adds, 20 flop; 2-D order 3: four neighbour sums and two
-# weights per component, 12 flop), |u|^2 (3), the reservoir (multiply, add, divide: 3), a and b
-# (4), the right-hand side (8) and the stage update plus accumulation (8).
-FP64_FLOP_PER_NODE_STEP = {(1, 5): 4 * (20 + 3 + 3 + 4 + 8 + 8), (2, 3): 4 * (12 + 3 + 3 + 4 + 8 + 8)}
+# FP64 operations of one node-step of the plain complex128 path as its kernels execute them (an FMA
+# counts two).  A stage: the centre's addition to b (1), the right-hand side (8) and the stage update (4),
+# in 1-D order 5 also the operator's row (four of its five weights, 14); the step's sum of slopes: 10.  The
+# reservoir, a and b are formed in pairs of floats and the 2-D neighbour sum in 64-bit integers: no FP64.
+FP64_FLOP_PER_NODE_STEP = {(1, 5): 4 * (14 + 1 + 8 + 4) + 10, (2, 3): 4 * (1 + 8 + 4) + 10}
 
 
 def measured_fp64_peak(dev):
