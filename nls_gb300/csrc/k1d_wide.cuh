@@ -13,11 +13,11 @@
 // What bounds it: complex64, the latency of four dependent stages (about 350 cycles each at order 5)
 // and the exchange, 540-950 cycles over S steps; complex128, the chain of a stage and the FP64
 // instructions of one warp per sub-partition (f64_node.cuh) -- so there two lanes share a node, one
-// for the real and one for the imaginary part, which halves them: 227 warp instructions and 1250
-// cycles a stage at order 5, the FP64 pipe 43 % busy.
+// for the real and one for the imaginary part, which halves them: 218 warp instructions and 1250
+// cycles a stage at order 5, the FP64 pipe 50 % busy.
 //
 // Measured, us a step, one CTA or cluster before and this kernel: complex64 order 5, 4096 nodes 4.64
-// and 0.70; complex128 order 5, 1000 nodes 5.3 and 2.5; order 7, 2501 nodes 8.5 and 3.0.
+// and 0.67; complex128 order 5, 1000 nodes 5.3 and 2.5; order 7, 2501 nodes 8.5 and 3.0.
 #pragma once
 
 namespace nlsg {

@@ -20,7 +20,7 @@ static constexpr size_t kWideSmem = 227 * 1024;
 // up to about 300 nodes a CTA, one beyond, and above 1800 nodes a CTA the stage kernels, whose
 // launches amortise there (600^2: 40.2 us a step against 41.1 here; 512^2: 30.3 against 27.8).  The
 // stages above are those of warps that fetched their own halo; with fetching warps 40^2 takes 5.2 us a
-// step, 128^2 5.7, 256^2 9.8 (stage kernels 8.5, 9.1 and 13.6).
+// step, 128^2 5.7, 256^2 9.6 (stage kernels 8.5, 9.2 and 13.7).
 Wide2DPlan wide_2d_plan(int K, int n, int sms) {
   Wide2DPlan best;
   double best_cost = 1e300;
@@ -98,7 +98,9 @@ static bool wide_reg_shape(int K, int shape, F&& f) {
 // order 3; 96 as 16 of 6 takes 5.7).  us a step, order 3, by rows of the region (16 / 24 / 32): 64^2
 // 1.99 / 2.09 / 2.32, 128^2 2.07 / 2.28 / 2.58; 512^2 3.14 with 48 rows, 3.78 with 64; streaming 8.7 to
 // 9.3.  Beyond one tile an SM (840 a side at order 3, 720 at order 5) the streaming and tile kernels;
-// the largest here against those: 840^2 5.5 and 11.1, order 5 700^2 7.5 and 9.5.
+// the largest here against those: 840^2 5.5 and 11.1, order 5 700^2 7.5 and 9.5.  Sixteen warps leave 128
+// registers a thread, and the largest regions spill a little (bytes a thread: 6 rows a warp 68 at order 3 and
+// 124 at order 5, 5 rows 24 and 4 rows 16 at order 5); the times are with the spills.
 WideReg2DPlan wide_reg_2d_plan(int K, int n, int sms) {
   WideReg2DPlan best;
   bool more = true;

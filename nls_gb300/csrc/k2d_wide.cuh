@@ -10,8 +10,8 @@
 // neighbours' values, the next own the tile's edge nodes -- they evaluate what their nodes need alone
 // (the reservoir and the coefficients) meanwhile, then the rest, and publish -- and the other warps
 // evaluate the nodes that need no neighbour's value.  One CTA barrier a stage.
-// Measured, order 3, us a step, stage kernels and this one: 40^2 8.5 and 5.2, 128^2 9.1 and 5.7, 256^2
-// 13.6 and 9.8 (602 warp instructions a stage and warp, FP64 pipe 41 % busy, integer pipe 44 %).
+// Measured, order 3, us a step, stage kernels and this one: 40^2 8.5 and 4.9-5.2, 128^2 9.2 and 5.7, 256^2
+// 13.7 and 9.6 (530 warp instructions a stage and warp, FP64 pipe 40 % busy, integer pipe 46 %).
 // LANES: two adjacent lanes share a node, one for each part, which shortens the chain of a node but
 // repeats the reservoir's quotient and the loop around it; for tiles of few warps, where the chain
 // bounds the stage.

@@ -11,7 +11,7 @@
 //
 // The arithmetic is reg_stage's, which agrees bit for bit with the streaming kernel's.  What bounds it:
 // the stages' arithmetic over the region (latency at 2-4 warps a scheduler), then one exchange
-// (540-950 cycles one way) a step.  Measured, order 3: 128^2 2.1 us a step, 777^2 6.0 (1442 warp
+// (540-950 cycles one way) a step.  Measured, order 3: 128^2 2.1 us a step, 777^2 6.0 (1361 warp
 // instructions a step, issue slots 44 % busy).
 #pragma once
 
