@@ -14,8 +14,8 @@
 // All CTAs of the launch are resident together (cooperative launch), so every wait ends; each is
 // bounded all the same, by two to three seconds.  CTAs do not wait for one another to start: beside
 // a kernel of another stream that held 24 SMs for longer than that bound, grids that need those SMs
-// started when it had ended (144 and 150 CTAs; a grid that fits beside it ran at once), and of two
-// contexts' cooperative grids the second starts after the first.
+// started when it had ended (144 and 150 CTAs; a grid that fits beside it ran at once), and no wait of
+// two contexts' grids that need most SMs, solved at the same time, has expired.
 // A wait that expires sets the context's status word; waits that see it set, or that belong to a
 // thread that has given up, end at once.  The values a thread gave up on are NaN from then on, and
 // NaN spreads with the stencil as the values would have, so a node of the final state is either
